@@ -224,6 +224,12 @@ void qb200_plan_destroy(qb200_plan* plan);
  * (input validation of execute_many, cuda.rs:1190-1220, 1699-1721). */
 qb200_status qb200_plan_bind(qb200_plan* plan, const char* name, const void* host, size_t nbytes);
 
+/* The same for n inputs in one call: slot i < QB200_Q_OUTPUT_COUNT - 1 is parameter i in declaration order, the
+ * data inputs follow in theirs.  The host buffers may be reused when the call returns; the uploads are queued, not
+ * waited for (pinned staging inside the library).  Nothing is uploaded when a slot or a size is wrong. */
+qb200_status qb200_plan_bind_many(qb200_plan* plan, const int32_t* slots, const void* const* hosts,
+                                  const size_t* nbytes, int32_t n);
+
 /* execute_retaining_without_output (cuda.rs:1233-1240): forward, residual,
  * reverse pass; leaves [loss, gradients...] on the device (all-reduced when a
  * communicator is attached). */
@@ -233,10 +239,25 @@ qb200_status qb200_plan_execute(qb200_plan* plan);
  * the gradients in parameter order (cuda.rs:1190-1220, 2961-2971). */
 qb200_status qb200_plan_read_output(qb200_plan* plan, int32_t index, void* host, size_t nbytes);
 
+/* All outputs in one transfer: the loss, then the gradients flat in parameter order, every leaf starting on a
+ * 4-element boundary behind the loss; 1 + QB200_Q_PARAMETER_COUNT elements. */
+qb200_status qb200_plan_read_outputs(qb200_plan* plan, void* host, size_t nbytes);
+
+/* Parameters and both Adam moments (null: not wanted) in that flat layout, with one wait; nbytes is the size of
+ * each.  Moments that no optimizer step has created read as zeros. */
+qb200_status qb200_plan_read_state(qb200_plan* plan, void* params, void* m, void* v, size_t nbytes);
+
 /* optimizer_step (cuda_optimizer.rs:207-398) with the element rule of
  * device_optimizer.rs:241-285, bias corrections formed in double on the host
  * and rounded once to the plan dtype (cuda_optimizer.rs:340-359). */
 qb200_status qb200_plan_optimizer_step(qb200_plan* plan, const qb200_opt_config* config);
+
+/* qb200_plan_execute and qb200_plan_optimizer_step in one call: a training step. */
+qb200_status qb200_plan_train_step(qb200_plan* plan, const qb200_opt_config* config);
+
+/* Page-locked host memory for read-back buffers. */
+qb200_status qb200_host_alloc(size_t nbytes, void** out);
+void qb200_host_free(void* host);
 
 /* execute_primary_retaining (cuda.rs:1245-1314): loss at the current
  * parameters, forward only; host_scalar receives one element of the plan dtype. */

@@ -83,7 +83,13 @@ SIGNATURES = {
     "qb200_plan_create": (_I32, [_P, _I32, C.POINTER(_P)]),
     "qb200_plan_destroy": (None, [_P]),
     "qb200_plan_bind": (_I32, [_P, C.c_char_p, _P, C.c_size_t]),
+    "qb200_plan_bind_many": (_I32, [_P, _P, _P, _P, _I32]),
     "qb200_plan_execute": (_I32, [_P]),
+    "qb200_plan_read_outputs": (_I32, [_P, _P, C.c_size_t]),
+    "qb200_plan_read_state": (_I32, [_P, _P, _P, _P, C.c_size_t]),
+    "qb200_plan_train_step": (_I32, [_P, C.POINTER(OptConfig)]),
+    "qb200_host_alloc": (_I32, [C.c_size_t, C.POINTER(_P)]),
+    "qb200_host_free": (None, [_P]),
     "qb200_plan_read_output": (_I32, [_P, _I32, _P, C.c_size_t]),
     "qb200_plan_optimizer_step": (_I32, [_P, C.POINTER(OptConfig)]),
     "qb200_plan_loss": (_I32, [_P, _P]),

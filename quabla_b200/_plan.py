@@ -14,7 +14,7 @@ from dataclasses import dataclass, field
 
 import numpy as np
 
-from . import _lib
+from . import _host, _lib
 from ._symbolic import Program
 
 COTANGENT_NAME = "__quabla_loss_cotangent"
@@ -141,6 +141,24 @@ class Plan:
             self._lib.qb200_desc_destroy(desc)
         self._handle = handle
 
+    def _layout(self) -> list[tuple[tuple[int, ...], int]]:
+        """(shape, first element) of every parameter in the flat parameter order: leaves start on 4-element
+        boundaries."""
+        found = getattr(self, "_flat_layout", None)
+        if found is None:
+            found, offset = [], 0
+            for index in range(len(self.spec.parameters)):
+                shape = self.spec.parameter_shape(index)
+                found.append((shape, offset))
+                offset += (int(np.prod(shape, dtype=np.int64)) + 3) // 4 * 4
+            self._flat_layout, self._flat_size = found, offset
+        return found
+
+    def _leaves(self, flat: np.ndarray, base: int = 0) -> list[np.ndarray]:
+        """Views of a flat buffer, one per parameter."""
+        item = self.dtype.itemsize
+        return [np.ndarray(shape, self.dtype, flat, (base + first) * item) for shape, first in self._layout()]
+
     def close(self) -> None:
         if getattr(self, "_handle", None) and self._owned:
             self._lib.qb200_plan_destroy(self._handle)
@@ -163,6 +181,23 @@ class Plan:
         """Bind from a host address (for example a pinned staging buffer)."""
         _lib.check(self._lib.qb200_plan_bind(self._handle, name.encode(), C.c_void_p(address), nbytes))
 
+    def slot(self, name: str) -> int:
+        """Number of a parameter or data input in `bind_many`."""
+        slots = getattr(self, "_slots", None)
+        if slots is None:
+            names = [n for n, _, _ in self.spec.parameters] + [n for n, _, _, _ in self.spec.inputs]
+            slots = self._slots = {n: i for i, n in enumerate(names)}
+        return slots[name]
+
+    def bind_many(self, slots: list[int], values: list) -> None:
+        """Several inputs in one call: arrays of the plan dtype (anything else is converted), by slot."""
+        n = len(slots)
+        arrays = [v if v.dtype == self.dtype and v.flags.c_contiguous else self._host(v) for v in values]
+        _lib.check(self._lib.qb200_plan_bind_many(
+            self._handle, (C.c_int32 * n)(*slots),
+            (C.c_void_p * n)(*[a.__array_interface__["data"][0] for a in arrays]),
+            (C.c_size_t * n)(*[a.nbytes for a in arrays]), n))
+
     def execute(self) -> None:
         _lib.check(self._lib.qb200_plan_execute(self._handle))
 
@@ -173,7 +208,23 @@ class Plan:
         return out
 
     def outputs(self) -> list[np.ndarray]:
-        return [self.read_output(i) for i in range(1 + len(self.spec.parameters))]
+        """The loss and every gradient, read in one transfer."""
+        self._layout()
+        flat = _host.empty(1 + self._flat_size, self.dtype)
+        _lib.check(self._lib.qb200_plan_read_outputs(self._handle, flat.__array_interface__["data"][0], flat.nbytes))
+        return [np.array(flat[0])] + self._leaves(flat, 1)  # the loss on its own: it is often kept for long
+
+    def read_state(self, moments: bool) -> list[list[np.ndarray]]:
+        """[parameters] or [parameters, first moments, second moments], each in parameter order; one wait."""
+        self._layout()
+        flats = [_host.empty(self._flat_size, self.dtype) for _ in range(3 if moments else 1)]
+        at = [f.__array_interface__["data"][0] for f in flats] + [None, None]
+        _lib.check(self._lib.qb200_plan_read_state(self._handle, at[0], at[1], at[2], flats[0].nbytes))
+        return [self._leaves(f) for f in flats]
+
+    def train_step(self, config: _lib.OptConfig) -> None:
+        """execute and optimizer_step in one call."""
+        _lib.check(self._lib.qb200_plan_train_step(self._handle, C.byref(config)))
 
     def optimizer_step(self, config: _lib.OptConfig) -> None:
         _lib.check(self._lib.qb200_plan_optimizer_step(self._handle, C.byref(config)))

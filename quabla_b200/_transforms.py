@@ -61,6 +61,65 @@ def _normalize_argnums(argnums, count: int) -> tuple[int, ...]:
     return tuple(out)
 
 
+# Shape of an argument as last seen, for calls that repeat it: ("dict", keys, children), ("list" | "tuple", children),
+# ("array", shape, dtype), ("none",) or ("static", value).
+def _template(node):
+    if isinstance(node, dict):
+        keys = sorted(node)
+        return ("dict", tuple(keys), tuple(_template(node[k]) for k in keys)) if type(node) is dict else None
+    if isinstance(node, (list, tuple)) and not hasattr(node, "_fields"):
+        kind = {list: "list", tuple: "tuple"}.get(type(node))
+        return (kind, tuple(_template(child) for child in node)) if kind else None
+    if node is None:
+        return ("none",)
+    if _is_array(node):
+        return ("array", np.shape(node), np.asarray(node).dtype)
+    return ("static", node)
+
+
+def _match(template, node, leaves: list) -> bool:
+    """Appends the array leaves of `node` in flattening order; False when it is not of the template's shape."""
+    if template is None:
+        return False
+    kind = template[0]
+    if kind == "array":
+        if type(node) is not np.ndarray or node.shape != template[1] or node.dtype != template[2]:
+            return False
+        leaves.append(node)
+        return True
+    if kind == "dict":
+        if type(node) is not dict or len(node) != len(template[1]):
+            return False
+        for key, child in zip(template[1], template[2]):
+            if key not in node or not _match(child, node[key], leaves):
+                return False
+        return True
+    if kind == "list" or kind == "tuple":
+        if type(node) is not (list if kind == "list" else tuple) or len(node) != len(template[1]):
+            return False
+        for child, value in zip(template[1], node):
+            if not _match(child, value, leaves):
+                return False
+        return True
+    if kind == "none":
+        return node is None
+    return type(node) is type(template[1]) and node == template[1]
+
+
+def _rebuild(template, values):
+    """The tree of a template with its array leaves taken from the iterator and None in place of static values."""
+    kind = template[0]
+    if kind == "array":
+        return next(values)
+    if kind == "dict":
+        return {key: _rebuild(child, values) for key, child in zip(template[1], template[2])}
+    if kind == "list":
+        return [_rebuild(child, values) for child in template[1]]
+    if kind == "tuple":
+        return tuple([_rebuild(child, values) for child in template[1]])
+    return None
+
+
 class CompiledLoss:
     """A loss traced for given argument signatures and compiled to a device plan.
 
@@ -124,6 +183,19 @@ class CompiledLoss:
         # needs no device).
         self.plan = Plan(self.spec, device_ordinal) if build_plan else None
         self._active = {name: i for i, (name, _, _) in enumerate(self.spec.parameters)}
+        self._templates = [_template(arg) for arg in args]
+        # For repeated calls: position among all array leaves and slot of every leaf the plan binds.
+        self._bound: list[tuple[int, int]] = []
+        if self.plan is not None:
+            at, params, data = 0, iter(self.param_names), iter(self.data_names)
+            for index, arg in enumerate(args):
+                for leaf in tr.flatten(arg)[0]:
+                    if not _is_array(leaf):
+                        continue
+                    name = next(params) if index in argnums else next(data)
+                    if index not in argnums or name in self._active:
+                        self._bound.append((at, self.plan.slot(name)))
+                    at += 1
 
     # -- running --------------------------------------------------------------
     def named_inputs(self, args: tuple) -> dict:
@@ -143,11 +215,20 @@ class CompiledLoss:
 
     def bind(self, args: tuple, skip_retained_bound: bool = False) -> None:
         params, data = self.leaves_of(args)
-        for name, value in zip(self.param_names, params):
-            if name in self._active:
-                self.plan.bind(name, value)
-        for name, value in zip(self.data_names, data):
-            self.plan.bind(name, value)
+        active = [(name, value) for name, value in zip(self.param_names, params) if name in self._active]
+        pairs = active + list(zip(self.data_names, data))
+        self.plan.bind_many([self.plan.slot(name) for name, _ in pairs], [value for _, value in pairs])
+
+    def bind_if_same(self, args: tuple) -> bool:
+        """Binds `args` if they have the structure, shapes and dtypes this loss was traced for."""
+        if len(args) != len(self._templates):
+            return False
+        leaves: list = []
+        for template, arg in zip(self._templates, args):
+            if not _match(template, arg, leaves):
+                return False
+        self.plan.bind_many([slot for _, slot in self._bound], [leaves[at] for at, _ in self._bound])
+        return True
 
     def gradients(self, args: tuple):
         """(value, grads) with grads shaped like the differentiated arguments."""
@@ -164,6 +245,9 @@ class CompiledLoss:
         it = iter(flat)
         trees = []
         for index in self.argnums:
+            if self._templates[index] is not None:
+                trees.append(_rebuild(self._templates[index], it))
+                continue
             leaves, rebuild = tr.flatten(args[index])
             trees.append(rebuild([next(it) if _is_array(leaf) else None for leaf in leaves]))
         return value, trees
@@ -185,6 +269,20 @@ class _Transform:
             raise TypeError("a transform requires a callable")
         self._fun = fun
         self._cache: OrderedDict = OrderedDict()
+        self._latest = None  # (device ordinal, cache key, compiled loss) of the last call
+
+    def _bound(self, args: tuple, argnums_of, device_ordinal: int):
+        """The compiled loss for these arguments, with them bound.  A call shaped like the last one skips the
+        signature."""
+        latest = self._latest
+        if latest is not None and latest[0] == device_ordinal and latest[1] in self._cache and latest[2].bind_if_same(args):
+            return latest[2]
+        argnums = argnums_of(len(args))
+        key = _signature(args, argnums, device_ordinal)
+        compiled = self._lookup(key, lambda: CompiledLoss(self._fun, args, argnums, device_ordinal))
+        compiled.bind(args)
+        self._latest = (device_ordinal, key, compiled)
+        return compiled
 
     def _lookup(self, key, build):
         found = self._cache.get(key)
@@ -215,10 +313,7 @@ class _ValueAndGrad(_Transform):
         return self._run(args, 0)
 
     def _run(self, args: tuple, device_ordinal: int):
-        argnums = _normalize_argnums(self._argnums, len(args))
-        key = _signature(args, argnums, device_ordinal)
-        compiled = self._lookup(key, lambda: CompiledLoss(self._fun, args, argnums, device_ordinal))
-        compiled.bind(args)
+        compiled = self._bound(args, lambda count: _normalize_argnums(self._argnums, count), device_ordinal)
         compiled.plan.execute()
         value, trees = compiled.gradients(args)
         grads = trees[0] if isinstance(self._argnums, int) else tuple(trees)
@@ -229,10 +324,7 @@ class _LossOnly(_Transform):
     """jit(loss): forward evaluation of the loss on the device."""
 
     def _run(self, args: tuple, device_ordinal: int):
-        key = _signature(args, (0,), device_ordinal)
-        compiled = self._lookup(key, lambda: CompiledLoss(self._fun, args, (0,), device_ordinal))
-        compiled.bind(args)
-        return compiled.plan.loss()
+        return self._bound(args, lambda count: (0,), device_ordinal).plan.loss()
 
     def __call__(self, *args):
         if _any_traced(args):

@@ -369,6 +369,14 @@ qb200_status qb200_plan_bind(qb200_plan* plan, const char* name, const void* hos
     return plan->bind(name, host, nbytes);
 }
 
+qb200_status qb200_plan_bind_many(qb200_plan* plan, const int32_t* slots, const void* const* hosts,
+                                  const size_t* nbytes, int32_t n) {
+    QB_PLAN(plan);
+    if (n < 0 || (n > 0 && (slots == nullptr || hosts == nullptr || nbytes == nullptr)))
+        return fail(QB200_INVALID, "bind_many needs slots, host buffers and sizes");
+    return plan->bind_many(slots, hosts, nbytes, n);
+}
+
 qb200_status qb200_plan_execute(qb200_plan* plan) {
     QB_PLAN(plan);
     QB_TRY(plan->execute_local());
@@ -381,9 +389,39 @@ qb200_status qb200_plan_read_output(qb200_plan* plan, int32_t index, void* host,
     return plan->read_output(index, host, nbytes);
 }
 
+qb200_status qb200_plan_read_outputs(qb200_plan* plan, void* host, size_t nbytes) {
+    QB_PLAN(plan);
+    if (host == nullptr) return fail(QB200_INVALID, "read_outputs needs a host buffer");
+    return plan->read_outputs(host, nbytes);
+}
+
+qb200_status qb200_plan_read_state(qb200_plan* plan, void* params, void* m, void* v, size_t nbytes) {
+    QB_PLAN(plan);
+    return plan->read_state(params, m, v, nbytes);
+}
+
 qb200_status qb200_plan_optimizer_step(qb200_plan* plan, const qb200_opt_config* config) {
     QB_PLAN(plan);
     return plan->optimizer_step(config);
+}
+
+qb200_status qb200_plan_train_step(qb200_plan* plan, const qb200_opt_config* config) {
+    QB_PLAN(plan);
+    QB_TRY(qb::validate_opt_config(config));  // before any device work, as optimizer_step
+    QB_TRY(plan->execute_local());
+    QB_TRY(plan->all_reduce());
+    return plan->optimizer_step(config);
+}
+
+qb200_status qb200_host_alloc(size_t nbytes, void** out) {
+    if (out == nullptr || nbytes == 0) return fail(QB200_INVALID, "host_alloc needs a size and an output");
+    *out = nullptr;
+    QB_CUDA(cudaHostAlloc(out, nbytes, cudaHostAllocPortable));
+    return QB200_OK;
+}
+
+void qb200_host_free(void* host) {
+    if (host != nullptr) cudaFreeHost(host);
 }
 
 qb200_status qb200_plan_loss(qb200_plan* plan, void* host_scalar) {

@@ -1,0 +1,91 @@
+// Pool of pinned staging blocks (see host_staging.h).
+#include "host_staging.h"
+
+#include <deque>
+#include <memory>
+#include <mutex>
+#include <vector>
+
+namespace qb {
+
+namespace {
+
+struct Pool {
+    int users = 0;
+    std::vector<std::unique_ptr<StagingBlock>> blocks;
+    std::deque<StagingBlock*> idle;  // oldest transfer first
+    void clear() {
+        for (auto& b : blocks) {
+            if (b->queued) cudaEventSynchronize(b->done);
+            cudaEventDestroy(b->done);
+            cudaFreeHost(b->host);
+        }
+        blocks.clear();
+        idle.clear();
+    }
+};
+
+std::mutex g_mutex;
+
+Pool& pool(int device) {
+    static std::vector<std::unique_ptr<Pool>>* pools = new std::vector<std::unique_ptr<Pool>>();  // never destroyed:
+    while ((int)pools->size() <= device) pools->emplace_back(new Pool());  // plans may outlive static destructors
+    return *(*pools)[device];
+}
+
+}  // namespace
+
+void staging_attach(int device) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    ++pool(device).users;
+}
+
+void staging_detach(int device) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    Pool& p = pool(device);
+    // Blocks handed out are back by now: a plan returns every block before its call ends.
+    if (--p.users == 0) p.clear();
+}
+
+cudaError_t staging_acquire(int device, StagingBlock** out) {
+    StagingBlock* block = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        Pool& p = pool(device);
+        const bool oldest_done = !p.idle.empty() && (!p.idle.front()->queued || cudaEventQuery(p.idle.front()->done) == cudaSuccess);
+        if (!oldest_done && (int)p.blocks.size() < STAGING_BLOCKS) {
+            std::unique_ptr<StagingBlock> fresh(new StagingBlock());
+            void* raw = nullptr;
+            cudaError_t e = cudaHostAlloc(&raw, STAGING_BLOCK_BYTES, cudaHostAllocPortable);
+            if (e != cudaSuccess) return e;
+            e = cudaEventCreateWithFlags(&fresh->done, cudaEventDisableTiming);
+            if (e != cudaSuccess) {
+                cudaFreeHost(raw);
+                return e;
+            }
+            fresh->host = static_cast<unsigned char*>(raw);
+            *out = fresh.get();
+            p.blocks.push_back(std::move(fresh));
+            return cudaSuccess;
+        }
+        if (!p.idle.empty()) {
+            block = p.idle.front();
+            p.idle.pop_front();
+        }
+    }
+    *out = block;
+    if (block == nullptr) return cudaSuccess;  // every block is in some other caller's hands at this instant
+    const cudaError_t e = block->queued ? cudaEventSynchronize(block->done) : cudaSuccess;
+    block->queued = false;
+    return e;
+}
+
+cudaError_t staging_release(int device, StagingBlock* block, cudaStream_t stream) {
+    const cudaError_t e = cudaEventRecord(block->done, stream);
+    block->queued = e == cudaSuccess;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    pool(device).idle.push_back(block);
+    return e;
+}
+
+}  // namespace qb

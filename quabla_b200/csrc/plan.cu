@@ -11,6 +11,7 @@
 #include "fused_kernel.cuh"
 #include "jet_kernels.cuh"
 #include "dmma_gemm.cuh"
+#include "host_staging.h"
 #include "layer_kernels.cuh"
 #include "point_kernels.cuh"
 #include "tc_gemm.h"
@@ -143,8 +144,11 @@ class Plan final : public qb200_plan {
     qb200_status init();
 
     qb200_status bind(const char* name, const void* host, size_t nbytes) override;
+    qb200_status bind_many(const int32_t* slots, const void* const* hosts, const size_t* nbytes, int n) override;
     qb200_status execute_local() override;
     qb200_status all_reduce() override;
+    qb200_status read_outputs(void* host, size_t nbytes) override;
+    qb200_status read_state(void* params, void* m, void* v, size_t nbytes) override;
     qb200_status read_output(int index, void* host, size_t nbytes) override;
     qb200_status optimizer_step(const qb200_opt_config* config) override;
     qb200_status loss(void* host_scalar) override;
@@ -163,7 +167,10 @@ class Plan final : public qb200_plan {
     // [loss, gradients..., flag]: the last element carries the device error flag through the all-reduce.
     size_t flat_count() const override { return 2 + n_params_; }
     cudaStream_t stream() const override { return stream_; }
-    void set_dp_scale(double inv_world) override { dp_scale_ = inv_world; }
+    void set_dp_scale(double inv_world) override {
+        if (inv_world != dp_scale_) drop_graphs();  // the factor is an argument of the captured kernels
+        dp_scale_ = inv_world;
+    }
     int device() const override { return device_; }
     int dtype() const override { return DTypeOf<T>::value; }
     int64_t input_shard_bytes(const char* name) const override;
@@ -181,7 +188,9 @@ class Plan final : public qb200_plan {
         bool bound = false;
     };
     struct InputState {
-        T* dev = nullptr;
+        T* dev = nullptr;      // inside the arena
+        size_t offset = 0;     // elements from the start of the arena
+        size_t count = 0;
         bool bound = false;
     };
     struct SetState {
@@ -214,7 +223,20 @@ class Plan final : public qb200_plan {
     }
     qb200_status check_bound() const;
     qb200_status refresh_tables();
+    // The kernel sequence of a step (or of a loss evaluation) as a CUDA graph: see run().
+    struct StepGraph {
+        int uses = 0;
+        cudaGraphExec_t exec = nullptr;
+        int64_t launches = 0;
+    };
+    void drop_graphs() {
+        for (auto& g : graphs_)
+            if (g.second.exec != nullptr) cudaGraphExecDestroy(g.second.exec);
+        graphs_.clear();
+    }
     qb200_status run(bool forward_only);
+    qb200_status enqueue(bool forward_only);
+    qb200_status upload(size_t offset, const void* host, size_t nbytes, cudaStream_t stream);
     qb200_status run_chunk(int si, long long point0, int C, int partial_slot, bool forward_only);
     qb200_status run_fused(int si, bool forward_only);
     qb200_status prepare_weight_images();
@@ -279,13 +301,24 @@ class Plan final : public qb200_plan {
     std::vector<int> w_leaf_, b_leaf_;
     std::vector<InputState> inputs_;
     std::vector<SetState> sets_;
-    T* d_params_ = nullptr;
+    // One device array for everything the host binds, parameters first, then the data inputs (each on a 256-byte
+    // boundary), so that binding several of them is one transfer.
+    T* d_arena_ = nullptr;
+    T* d_params_ = nullptr;    // start of the arena
     T* d_flat_ = nullptr;      // [loss, gradients...]
     double* d_acc_ = nullptr;  // gradient accumulators
     T* d_m_ = nullptr;
     T* d_v_ = nullptr;
     T* d_ct_ = nullptr;
-    T* d_loss_only_ = nullptr;
+    T* h_loss_ = nullptr;      // mapped host word that a loss evaluation writes
+    T* d_loss_only_ = nullptr; // the same as the device sees it
+    std::map<uint32_t, StepGraph> graphs_;
+    // Large batches are uploaded on a stream of their own, under the previous step's kernels (which read the point
+    // tables, not the inputs); ev_inputs_ is the last point of the main stream that touched the inputs.
+    cudaStream_t copy_stream_ = nullptr;
+    cudaEvent_t ev_inputs_ = nullptr, ev_copied_ = nullptr;
+    bool staging_attached_ = false;
+    bool inputs_touched_ = true;  // the main stream touched the inputs after ev_inputs_ was recorded
     double* d_partials_ = nullptr;
     double* d_clip_ = nullptr;
     int total_partials_ = 0;
@@ -357,6 +390,11 @@ class Plan final : public qb200_plan {
     cudaEvent_t ev_begin_ = nullptr, ev_end_ = nullptr;  // around the kernels of point set 0
     cudaEvent_t ev_ar0_ = nullptr, ev_ar1_ = nullptr;    // around the gradient all-reduce
     bool ev_valid_ = false, ev_ar_valid_ = false;
+    bool capturing_ = false;
+    // A timing mark on the main stream; inside a captured sequence it becomes a node of the graph.
+    cudaError_t mark(cudaEvent_t e) {
+        return cudaEventRecordWithFlags(e, stream_, capturing_ ? cudaEventRecordExternal : cudaEventRecordDefault);
+    }
     int64_t launches_ = 0;
     int64_t steps_ = 0;
     bool executed_ = false;
@@ -393,8 +431,20 @@ void Plan<T>::release() {
     if (stream_ != nullptr) cudaStreamSynchronize(stream_);
     for (void* p : buffers_) cudaFree(p);
     buffers_.clear();
+    drop_graphs();
     if (h_status_ != nullptr) cudaFreeHost(h_status_);
     h_status_ = d_status_ = nullptr;
+    h_loss_ = d_loss_only_ = nullptr;  // in the same allocation
+    if (copy_stream_ != nullptr) {
+        cudaStreamSynchronize(copy_stream_);
+        cudaStreamDestroy(copy_stream_);
+    }
+    copy_stream_ = nullptr;
+    if (ev_inputs_ != nullptr) cudaEventDestroy(ev_inputs_);
+    if (ev_copied_ != nullptr) cudaEventDestroy(ev_copied_);
+    ev_inputs_ = ev_copied_ = nullptr;
+    if (staging_attached_) staging_detach(device_);
+    staging_attached_ = false;
     for (cudaEvent_t e : timer_events_) cudaEventDestroy(e);
     timer_events_.clear();
     if (ev_begin_ != nullptr) cudaEventDestroy(ev_begin_);
@@ -453,32 +503,43 @@ qb200_status Plan<T>::init() {
         (p.kind == QB200_WEIGHT ? w_leaf_ : b_leaf_)[p.layer] = (int)i;
     }
     n_params_ = offset;
-    QB_TRY(dev_alloc(&d_params_, n_params_));
+    QB_CUDA(cudaEventCreateWithFlags(&ev_inputs_, cudaEventDisableTiming));
+    QB_CUDA(cudaEventCreateWithFlags(&ev_copied_, cudaEventDisableTiming));
+    staging_attach(device_);
+    staging_attached_ = true;
+    constexpr size_t ALIGN = 256 / sizeof(T);
+    size_t arena = (n_params_ + ALIGN - 1) / ALIGN * ALIGN;
+    inputs_.resize(desc_.inputs.size());
+    for (size_t i = 0; i < desc_.inputs.size(); ++i) {
+        inputs_[i].offset = arena;
+        inputs_[i].count = (size_t)(desc_.inputs[i].rows * desc_.inputs[i].cols);
+        arena += (inputs_[i].count + ALIGN - 1) / ALIGN * ALIGN;
+    }
+    QB_TRY(dev_alloc(&d_arena_, arena));
+    d_params_ = d_arena_;
+    for (auto& in : inputs_) in.dev = d_arena_ + in.offset;
     QB_TRY(dev_alloc(&d_flat_, 2 + n_params_));
     QB_TRY(dev_alloc(&d_ct_, 1));
-    QB_TRY(dev_alloc(&d_loss_only_, 1));
     QB_TRY(dev_alloc(&d_clip_, 3));
     QB_TRY(dev_alloc(&d_error_, 1));
     QB_CUDA(cudaMemsetAsync(d_error_, 0, sizeof(int), stream_));
     QB_CUDA(cudaMemsetAsync(d_flat_, 0, (2 + n_params_) * sizeof(T), stream_));
     {
         void* raw = nullptr;
-        QB_CUDA(cudaHostAlloc(&raw, 2 * sizeof(int), cudaHostAllocMapped));
+        QB_CUDA(cudaHostAlloc(&raw, 2 * sizeof(int) + sizeof(T), cudaHostAllocMapped));
         h_status_ = static_cast<int*>(raw);
         h_status_[0] = h_status_[1] = 0;
         void* mapped = nullptr;
         QB_CUDA(cudaHostGetDevicePointer(&mapped, raw, 0));
         d_status_ = static_cast<int*>(mapped);
+        h_loss_ = reinterpret_cast<T*>(h_status_ + 2);
+        d_loss_only_ = reinterpret_cast<T*>(d_status_ + 2);
     }
     QB_CUDA(cudaMemsetAsync(d_params_, 0, n_params_ * sizeof(T), stream_));
     QB_CUDA(cudaMemsetAsync(d_clip_, 0, 3 * sizeof(double), stream_));
     const T one = T(1);
     QB_CUDA(cudaMemcpyAsync(d_ct_, &one, sizeof(T), cudaMemcpyHostToDevice, stream_));
     QB_CUDA(cudaStreamSynchronize(stream_));
-
-    inputs_.resize(desc_.inputs.size());
-    for (size_t i = 0; i < desc_.inputs.size(); ++i)
-        QB_TRY(dev_alloc(&inputs_[i].dev, (size_t)(desc_.inputs[i].rows * desc_.inputs[i].cols)));
 
     fused_ = choose_fused();
     // Saved-jet scratch: sized per set from a byte budget, then the maximum over sets.
@@ -684,38 +745,130 @@ int64_t Plan<T>::input_shard_bytes(const char* name) const {
 template <typename T>
 qb200_status Plan<T>::bind(const char* name, const void* host, size_t nbytes) {
     if (name == nullptr || host == nullptr) return fail(QB200_INVALID, "bind needs a name and a host buffer");
-    std::lock_guard<std::recursive_mutex> lock(mutex_);
-    QB_TRY(use_device());
     const std::string key(name);
     if (key == kCotangentName) {
+        std::lock_guard<std::recursive_mutex> lock(mutex_);
+        QB_TRY(use_device());
         if (nbytes != sizeof(T)) return fail(QB200_INVALID, "input '%s' is one scalar of %zu bytes, got %zu", name, sizeof(T), nbytes);
         QB_CUDA(cudaMemcpyAsync(d_ct_, host, nbytes, cudaMemcpyHostToDevice, stream_));
         QB_CUDA(cudaStreamSynchronize(stream_));
         return QB200_OK;
     }
-    for (size_t i = 0; i < desc_.params.size(); ++i) {
-        if (desc_.params[i].name != key) continue;
-        const size_t want = leaves_[i].count * sizeof(T);
-        if (nbytes != want) return fail(QB200_INVALID, "parameter '%s' needs %zu bytes, got %zu", name, want, nbytes);
-        QB_CUDA(cudaMemcpyAsync(d_params_ + leaves_[i].offset, host, nbytes, cudaMemcpyHostToDevice, stream_));
-        QB_CUDA(cudaStreamSynchronize(stream_));
-        leaves_[i].bound = true;
-        return QB200_OK;
+    int32_t slot = 0;
+    for (const auto& p : desc_.params) {
+        if (p.name == key) return bind_many(&slot, &host, &nbytes, 1);
+        ++slot;
     }
-    for (size_t i = 0; i < desc_.inputs.size(); ++i) {
-        if (desc_.inputs[i].name != key) continue;
-        const size_t want = (size_t)(desc_.inputs[i].rows * desc_.inputs[i].cols) * sizeof(T);
-        if (nbytes != want) return fail(QB200_INVALID, "input '%s' needs %zu bytes, got %zu", name, want, nbytes);
-        QB_CUDA(cudaMemcpyAsync(inputs_[i].dev, host, nbytes, cudaMemcpyHostToDevice, stream_));
-        // The host buffer may be pageable and reused by the caller right away.
-        QB_CUDA(cudaStreamSynchronize(stream_));
-        inputs_[i].bound = true;
-        for (size_t si = 0; si < desc_.sets.size(); ++si)
-            for (const auto& c : desc_.sets[si].cols)
-                if (c.first == (int)i) sets_[si].table_dirty = true;
-        return QB200_OK;
+    for (const auto& in : desc_.inputs) {
+        if (in.name == key) return bind_many(&slot, &host, &nbytes, 1);
+        ++slot;
     }
     return fail(QB200_INVALID, "the plan has no input named '%s'", name);
+}
+
+// Host array into the arena through pinned blocks: the caller's buffer is free when this returns, the transfers
+// are queued on `stream`.
+template <typename T>
+qb200_status Plan<T>::upload(size_t offset, const void* host, size_t nbytes, cudaStream_t stream) {
+    const unsigned char* src = static_cast<const unsigned char*>(host);
+    unsigned char* dst = reinterpret_cast<unsigned char*>(d_arena_ + offset);
+    for (size_t at = 0; at < nbytes; at += STAGING_BLOCK_BYTES) {
+        const size_t piece = std::min(STAGING_BLOCK_BYTES, nbytes - at);
+        StagingBlock* block = nullptr;
+        QB_CUDA(staging_acquire(device_, &block));
+        if (block == nullptr) {
+            QB_CUDA(cudaMemcpyAsync(dst + at, src + at, piece, cudaMemcpyHostToDevice, stream));
+            QB_CUDA(cudaStreamSynchronize(stream));
+            continue;
+        }
+        memcpy(block->host, src + at, piece);
+        const cudaError_t e = cudaMemcpyAsync(dst + at, block->host, piece, cudaMemcpyHostToDevice, stream);
+        QB_CUDA(staging_release(device_, block, stream));
+        QB_CUDA(e);
+    }
+    return QB200_OK;
+}
+
+// Uploads of at least this size go on the copy stream; below it the two event waits cost more than the transfer.
+constexpr size_t COPY_STREAM_BYTES = (size_t)128 << 10;
+
+template <typename T>
+qb200_status Plan<T>::bind_many(const int32_t* slots, const void* const* hosts, const size_t* nbytes, int n) {
+    const int np = (int)desc_.params.size(), ni = (int)desc_.inputs.size();
+    auto offset_of = [&](int slot) { return slot < np ? leaves_[slot].offset : inputs_[slot - np].offset; };
+    auto count_of = [&](int slot) { return slot < np ? leaves_[slot].count : inputs_[slot - np].count; };
+    size_t total = 0;
+    bool params = false, data = false;
+    for (int i = 0; i < n; ++i) {
+        if (slots[i] < 0 || slots[i] >= np + ni) return fail(QB200_INVALID, "slot %d of %d", slots[i], np + ni);
+        const bool is_param = slots[i] < np;
+        const char* name = is_param ? desc_.params[slots[i]].name.c_str() : desc_.inputs[slots[i] - np].name.c_str();
+        if (hosts[i] == nullptr) return fail(QB200_INVALID, "bind needs a host buffer for '%s'", name);
+        const size_t want = count_of(slots[i]) * sizeof(T);
+        if (nbytes[i] != want)
+            return fail(QB200_INVALID, "%s '%s' needs %zu bytes, got %zu", is_param ? "parameter" : "input", name, want, nbytes[i]);
+        total += want;
+        params = params || is_param;
+        data = data || !is_param;
+    }
+    std::lock_guard<std::recursive_mutex> lock(mutex_);
+    QB_TRY(use_device());
+    cudaStream_t stream = stream_;
+    if (!params && total >= COPY_STREAM_BYTES) {
+        if (copy_stream_ == nullptr) QB_CUDA(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
+        if (inputs_touched_) {
+            QB_CUDA(cudaEventRecord(ev_inputs_, stream_));
+            inputs_touched_ = false;
+        }
+        stream = copy_stream_;
+        QB_CUDA(cudaStreamWaitEvent(stream, ev_inputs_, 0));
+    }
+    for (int i = 0; i < n;) {
+        // A run of slots that follow one another in the arena and fit one block together: one transfer (the
+        // padding between them, which stays zero, included).
+        const size_t first = offset_of(slots[i]);
+        size_t end = first + count_of(slots[i]);
+        int j = i + 1;
+        while (j < n && offset_of(slots[j]) >= end && offset_of(slots[j]) - end < 256 / sizeof(T) &&
+               (offset_of(slots[j]) + count_of(slots[j]) - first) * sizeof(T) <= STAGING_BLOCK_BYTES) {
+            end = offset_of(slots[j]) + count_of(slots[j]);
+            ++j;
+        }
+        StagingBlock* block = nullptr;
+        if (j > i + 1) QB_CUDA(staging_acquire(device_, &block));
+        if (block == nullptr) {
+            for (; i < j; ++i) QB_TRY(upload(offset_of(slots[i]), hosts[i], nbytes[i], stream));
+            continue;
+        }
+        size_t at = first;
+        for (; i < j; ++i) {
+            const size_t off = offset_of(slots[i]);
+            memset(block->host + (at - first) * sizeof(T), 0, (off - at) * sizeof(T));
+            memcpy(block->host + (off - first) * sizeof(T), hosts[i], nbytes[i]);
+            at = off + count_of(slots[i]);
+        }
+        const cudaError_t e = cudaMemcpyAsync(d_arena_ + first, block->host, (end - first) * sizeof(T), cudaMemcpyHostToDevice, stream);
+        QB_CUDA(staging_release(device_, block, stream));
+        QB_CUDA(e);
+    }
+    if (stream != stream_) {
+        QB_CUDA(cudaEventRecord(ev_copied_, stream));
+        QB_CUDA(cudaStreamWaitEvent(stream_, ev_copied_, 0));
+    } else if (data) {
+        inputs_touched_ = true;
+    }
+    for (int i = 0; i < n; ++i) {
+        if (slots[i] < np) {
+            leaves_[slots[i]].bound = true;
+            continue;
+        }
+        const int input = slots[i] - np;
+        inputs_[input].bound = true;
+        for (size_t si = 0; si < desc_.sets.size(); ++si)
+            for (const auto& c : desc_.sets[si].cols)
+                if (c.first == input) sets_[si].table_dirty = true;
+    }
+    return QB200_OK;
 }
 
 template <typename T>
@@ -753,6 +906,7 @@ qb200_status Plan<T>::sample_uniform(const char* name, int column, uint64_t key,
                                                                         (unsigned long long)key, minval, width, low, high);
         QB_TRY(launched("sample_uniform_kernel"));
         inputs_[i].bound = true;
+        inputs_touched_ = true;
         for (size_t si = 0; si < desc_.sets.size(); ++si)
             for (const auto& c : desc_.sets[si].cols)
                 if (c.first == (int)i) sets_[si].table_dirty = true;
@@ -787,6 +941,12 @@ qb200_status Plan<T>::refresh_tables() {
         gather_table_kernel<T><<<grid_for(n * st.ncols, 256), 256, 0, stream_>>>(a, st.table, n);
         QB_TRY(launched("gather_table_kernel"));
         st.table_dirty = false;
+        inputs_touched_ = true;
+    }
+    if (inputs_touched_ && copy_stream_ != nullptr) {
+        // The tables now hold what the kernels of this step read: the next upload may overwrite the inputs from here.
+        QB_CUDA(cudaEventRecord(ev_inputs_, stream_));
+        inputs_touched_ = false;
     }
     return QB200_OK;
 }
@@ -1277,11 +1437,50 @@ qb200_status Plan<T>::run_chunk(int si, long long point0, int C, int partial_slo
     return QB200_OK;
 }
 
+// The kernel sequence of a step depends on the plan and on nothing a call passes, so from its second use on it is
+// launched as one CUDA graph (a step of a small network is a dozen launches of a few microseconds each).
+// Left as single launches: sequences too long for launch gaps to matter, and plans whose launches are timed one by one.
+constexpr int64_t GRAPH_MAX_LAUNCHES = 256;
+
 template <typename T>
 qb200_status Plan<T>::run(bool forward_only) {
     QB_TRY(use_device());
     QB_TRY(check_bound());
     QB_TRY(refresh_tables());
+    StepGraph& g = graphs_[forward_only ? 1 : 0];
+    if (timers_ || g.uses == 0 || g.launches > GRAPH_MAX_LAUNCHES) {
+        const int64_t before = launches_;
+        QB_TRY(enqueue(forward_only));
+        ++g.uses;
+        g.launches = launches_ - before;
+        return QB200_OK;
+    }
+    if (g.exec == nullptr) {
+        const int64_t before = launches_;
+        QB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+        capturing_ = true;
+        const qb200_status st = enqueue(forward_only);
+        capturing_ = false;
+        cudaGraph_t graph = nullptr;
+        const cudaError_t e = cudaStreamEndCapture(stream_, &graph);
+        launches_ = before;
+        if (st != QB200_OK) {
+            if (graph != nullptr) cudaGraphDestroy(graph);
+            return st;
+        }
+        QB_CUDA(e);
+        const cudaError_t made = cudaGraphInstantiate(&g.exec, graph, 0);
+        cudaGraphDestroy(graph);
+        if (made != cudaSuccess) g.exec = nullptr;
+        QB_CUDA(made);
+    }
+    QB_CUDA(cudaGraphLaunch(g.exec, stream_));
+    launches_ += g.launches;
+    return QB200_OK;
+}
+
+template <typename T>
+qb200_status Plan<T>::enqueue(bool forward_only) {
     if (!forward_only) {
         timer_used_ = 0;
         timer_flops_ = 0.0;
@@ -1309,11 +1508,11 @@ qb200_status Plan<T>::run(bool forward_only) {
         SetState& st = sets_[si];
         const long long n = desc_.sets[si].n;
         int slot = st.partial_offset;
-        if (si == 0 && !forward_only) QB_CUDA(cudaEventRecord(ev_begin_, stream_));
+        if (si == 0 && !forward_only) QB_CUDA(mark(ev_begin_));
         if (fused_) {
             QB_TRY(run_fused((int)si, forward_only));
             if (si == 0 && !forward_only) {
-                QB_CUDA(cudaEventRecord(ev_end_, stream_));
+                QB_CUDA(mark(ev_end_));
                 ev_valid_ = true;
             }
             la.offset[si] = st.partial_offset;
@@ -1330,7 +1529,7 @@ qb200_status Plan<T>::run(bool forward_only) {
         }
         select_lane(0);
         if (si == 0 && !forward_only) {
-            QB_CUDA(cudaEventRecord(ev_end_, stream_));
+            QB_CUDA(mark(ev_end_));
             ev_valid_ = true;
         }
         la.offset[si] = st.partial_offset;
@@ -1390,7 +1589,7 @@ qb200_status Plan<T>::all_reduce() {
         // (crates/quabla-core/src/tensor_ir/cuda.rs:132-145, 699-716).
         api->CommAbort(comm_);
         comm_ = nullptr;
-        dp_scale_ = 1.0;
+        set_dp_scale(1.0);
         return fail(QB200_NCCL_ERROR, "ncclAllReduce failed: %s; the communicator was aborted, attach a new one", api->GetErrorString(r));
     }
     return QB200_OK;
@@ -1461,8 +1660,8 @@ qb200_status Plan<T>::loss(void* host_scalar) {
     if (host_scalar == nullptr) return fail(QB200_INVALID, "loss needs a host scalar");
     std::lock_guard<std::recursive_mutex> lock(mutex_);
     QB_TRY(run(true));
-    QB_CUDA(cudaMemcpyAsync(host_scalar, d_loss_only_, sizeof(T), cudaMemcpyDeviceToHost, stream_));
-    QB_CUDA(cudaStreamSynchronize(stream_));
+    QB_CUDA(cudaStreamSynchronize(stream_));  // the last kernel wrote the loss into mapped host memory
+    memcpy(host_scalar, h_loss_, sizeof(T));
     return check_device_error();
 }
 
@@ -1493,6 +1692,38 @@ qb200_status Plan<T>::read_input(const char* name, void* host, size_t nbytes) {
     if (src == nullptr) return fail(QB200_INVALID, "the plan has no input named '%s'", name);
     if (nbytes != count * sizeof(T)) return fail(QB200_INVALID, "input '%s' has %zu bytes, got a buffer of %zu", name, count * sizeof(T), nbytes);
     QB_CUDA(cudaMemcpyAsync(host, src, nbytes, cudaMemcpyDeviceToHost, stream_));
+    QB_CUDA(cudaStreamSynchronize(stream_));
+    return check_device_error();
+}
+
+template <typename T>
+qb200_status Plan<T>::read_outputs(void* host, size_t nbytes) {
+    std::lock_guard<std::recursive_mutex> lock(mutex_);
+    QB_TRY(use_device());
+    if (!executed_) return fail(QB200_INVALID, "read_outputs before execute");
+    if (nbytes != (1 + n_params_) * sizeof(T))
+        return fail(QB200_INVALID, "the outputs are %zu bytes, got a buffer of %zu", (1 + n_params_) * sizeof(T), nbytes);
+    QB_CUDA(cudaMemcpyAsync(host, d_flat_, nbytes, cudaMemcpyDeviceToHost, stream_));
+    QB_CUDA(cudaStreamSynchronize(stream_));
+    return check_device_error();
+}
+
+template <typename T>
+qb200_status Plan<T>::read_state(void* params, void* m, void* v, size_t nbytes) {
+    std::lock_guard<std::recursive_mutex> lock(mutex_);
+    QB_TRY(use_device());
+    if (nbytes != n_params_ * sizeof(T)) return fail(QB200_INVALID, "the state is %zu bytes per array, got buffers of %zu", n_params_ * sizeof(T), nbytes);
+    if (params != nullptr)
+        for (size_t i = 0; i < desc_.params.size(); ++i)
+            if (!leaves_[i].bound) return fail(QB200_NOT_BOUND, "parameter '%s' was never bound", desc_.params[i].name.c_str());
+    if (params != nullptr) QB_CUDA(cudaMemcpyAsync(params, d_params_, nbytes, cudaMemcpyDeviceToHost, stream_));
+    if (moments_ready_) {
+        if (m != nullptr) QB_CUDA(cudaMemcpyAsync(m, d_m_, nbytes, cudaMemcpyDeviceToHost, stream_));
+        if (v != nullptr) QB_CUDA(cudaMemcpyAsync(v, d_v_, nbytes, cudaMemcpyDeviceToHost, stream_));
+    } else {
+        if (m != nullptr) memset(m, 0, nbytes);
+        if (v != nullptr) memset(v, 0, nbytes);
+    }
     QB_CUDA(cudaStreamSynchronize(stream_));
     return check_device_error();
 }
@@ -1608,7 +1839,10 @@ qb200_status Plan<T>::set_option(int key, int64_t value) {
     std::lock_guard<std::recursive_mutex> lock(mutex_);
     switch (key) {
         case QB200_OPT_KERNEL_TIMERS: timers_ = value != 0; return QB200_OK;
-        case QB200_OPT_SINGLE_LANE: single_lane_ = value != 0; return QB200_OK;
+        case QB200_OPT_SINGLE_LANE:
+            single_lane_ = value != 0;
+            drop_graphs();
+            return QB200_OK;
         default: return fail(QB200_INVALID, "unknown option key %d", key);
     }
 }
@@ -1640,7 +1874,7 @@ qb200_status Plan<T>::attach_comm(const void* id, int rank, int world, int reduc
         return fail(QB200_NCCL_ERROR, "ncclCommInitRank failed: %s", api->GetErrorString(r));
     }
     world_ = world;
-    dp_scale_ = reduction == QB200_REDUCE_MEAN ? 1.0 / world : 1.0;
+    set_dp_scale(reduction == QB200_REDUCE_MEAN ? 1.0 / world : 1.0);
     return QB200_OK;
 }
 
@@ -1657,7 +1891,7 @@ qb200_status Plan<T>::detach_comm() {
     }
     comm_ = nullptr;
     world_ = 1;
-    dp_scale_ = 1.0;
+    set_dp_scale(1.0);
     return QB200_OK;
 }
 

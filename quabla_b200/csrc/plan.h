@@ -12,9 +12,13 @@
 struct qb200_plan {
     virtual ~qb200_plan() {}
     virtual qb200_status bind(const char* name, const void* host, size_t nbytes) = 0;
+    // Several inputs at once; slots number the parameters in declaration order, then the data inputs.
+    virtual qb200_status bind_many(const int32_t* slots, const void* const* hosts, const size_t* nbytes, int n) = 0;
     virtual qb200_status execute_local() = 0;   // forward + reverse, no collective
     virtual qb200_status all_reduce() = 0;       // the plan's own communicator, if attached
     virtual qb200_status read_output(int index, void* host, size_t nbytes) = 0;
+    virtual qb200_status read_outputs(void* host, size_t nbytes) = 0;  // the flat [loss, gradients...] buffer
+    virtual qb200_status read_state(void* params, void* m, void* v, size_t nbytes) = 0;
     virtual qb200_status optimizer_step(const qb200_opt_config* config) = 0;
     virtual qb200_status loss(void* host_scalar) = 0;
     virtual qb200_status read_input(const char* name, void* host, size_t nbytes) = 0;

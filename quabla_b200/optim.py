@@ -204,6 +204,7 @@ class CudaTrainerExecutor:
         self._dtype = compiled.dtype
         self._shapes = dict(zip(compiled.param_names, compiled.param_shapes))
         self._active = active
+        self._trained = [name for name, _, _ in compiled.spec.parameters]  # in the plan's flat order
 
     @property
     def learning_rate(self) -> float:
@@ -217,22 +218,27 @@ class CudaTrainerExecutor:
         self._learning_rate = value
 
     def _config(self):
-        return opt_config(learning_rate=self._learning_rate, **self._rule)
+        config = getattr(self, "_last_config", None)
+        if config is None:
+            config = self._last_config = opt_config(learning_rate=self._learning_rate, **self._rule)
+        config.learning_rate = self._learning_rate
+        return config
+
+    def _bind(self, inputs: dict | None) -> None:
+        if inputs:
+            self._plan.bind_many([self._plan.slot(name) for name in inputs], list(inputs.values()))
 
     def step(self, inputs: dict | None = None) -> None:
         config = self._config()
-        for name, value in (inputs or {}).items():
-            self._plan.bind(name, value)
-        self._plan.execute()
-        self._plan.optimizer_step(config)
+        self._bind(inputs)
+        self._plan.train_step(config)
         if self._frozen and self._rule["rule"] == "adam" and self._rule["weight_decay"] != 0.0:
             for name in self._frozen:
                 self._frozen[name] = decay_frozen_parameter(self._frozen[name], self._rule["weight_decay"],
                                                             self._learning_rate)
 
     def loss(self, inputs: dict | None = None) -> np.ndarray:
-        for name, value in (inputs or {}).items():
-            self._plan.bind(name, value)
+        self._bind(inputs)
         return self._plan.loss()
 
     def last_value(self) -> np.ndarray:
@@ -240,13 +246,15 @@ class CudaTrainerExecutor:
         return self._plan.read_output(0)
 
     def parameters(self) -> dict:
-        out = {}
-        for name in self._parameter_names:
-            if name in self._active:
-                out[name] = self._plan.read_input(name, self._shapes[name])
-            else:
-                out[name] = self._frozen[name].copy()
-        return out
+        return self._named_parameters(self._plan.read_state(moments=False)[0])
+
+    def _by_name(self, values: list) -> dict:
+        return {name: value.reshape(self._shapes[name]) for name, value in zip(self._trained, values)}
+
+    def _named_parameters(self, trained: list) -> dict:
+        values = self._by_name(trained)
+        return {name: values[name] if name in self._active else self._frozen[name].copy()
+                for name in self._parameter_names}
 
     def _moment_layout(self):
         """(name, shape, first element, element count) of every active parameter, in the plan's flat order."""
@@ -260,16 +268,19 @@ class CudaTrainerExecutor:
 
     def export_state(self) -> dict:
         """Optimizer state as host arrays: `{"step": n}` plus, for Adam, `"m"` and `"v"` (name -> array in the
-        plan dtype).  One device-to-host read per moment buffer (qb200_plan_read_moments)."""
+        plan dtype)."""
+        return self.export_all()[1]
+
+    def export_all(self) -> tuple[dict, dict]:
+        """(parameters by name, optimizer state), read together."""
         from . import _lib
 
+        adam = self._rule["rule"] == "adam"
+        params, *moments = self._plan.read_state(moments=adam)
         state: dict = {"step": int(self._plan.query(_lib.Q_STEP_COUNT))}
-        if self._rule["rule"] == "adam":
-            for key, which in (("m", 0), ("v", 1)):
-                flat = self._plan.read_moments(which)
-                state[key] = {name: flat[first:first + count].reshape(shape).copy()
-                              for name, shape, first, count in self._moment_layout()}
-        return state
+        for key, values in zip(("m", "v"), moments):
+            state[key] = self._by_name(values)
+        return self._named_parameters(params), state
 
     def _checked_moments(self, state: dict):
         """The flat moment vectors (or None for SGD) and the step count of a state; raises on any mismatch."""
@@ -406,7 +417,9 @@ class Trainer:
 
     @property
     def params(self) -> Any:
-        values = self._executor.parameters()
+        return self._params_tree(self._executor.parameters())
+
+    def _params_tree(self, values: dict) -> Any:
         return self._rebuild_params([values[name] for name in self._parameter_names])
 
     def step(self, *batch: Any) -> None:
@@ -433,7 +446,8 @@ class Trainer:
         The reference's Trainer keeps this state inside its native executor and exposes only
         `params` (python/quabla/optim.py:351-550); checkpointing a device run needs the moments too.
         """
-        return {"step": self._device_steps, "params": self.params, "optimizer": self._executor.export_state()}
+        params, optimizer = self._executor.export_all()
+        return {"step": self._device_steps, "params": self._params_tree(params), "optimizer": optimizer}
 
     def import_state(self, state: dict) -> None:
         """Resume from `export_state()` (of a trainer built with the same loss, parameter shapes and

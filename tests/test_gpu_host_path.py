@@ -1,0 +1,94 @@
+"""Uploads through the pinned staging blocks, captured step sequences and flat read-backs against the per-name calls
+and single launches they stand for: the same bits."""
+
+import numpy as np
+import pytest
+
+import quabla_b200 as qb
+from quabla_b200 import _host, _lib
+from quabla_b200._plan import Plan, opt_config
+
+from _util import traced
+
+pytestmark = pytest.mark.gpu
+
+
+# Point sets below and above the size that goes on the copy stream, and ragged around one staging block (1 MiB:
+# 131,072 points of two float32 columns, 65,536 of heat's four).
+@pytest.mark.parametrize("name,points", [("poisson1d", 64), ("poisson2d", 131072), ("poisson2d", 131075), ("heat3d", 65537)])
+def test_staged_uploads_and_captured_steps_equal_single_calls(cuda_device, name, points):
+    w, compiled, inputs = traced(name, points)
+    plan, single = Plan(compiled.spec, 0), Plan(compiled.spec, 0)
+    names = [n for n, _, _ in compiled.spec.parameters] + [n for n, _, _, _ in compiled.spec.inputs]
+    plan.bind_many([plan.slot(n) for n in names], [inputs[n] for n in names])
+    for n in names:
+        np.testing.assert_array_equal(plan.read_input(n, np.shape(inputs[n])), inputs[n])
+        single.bind(n, inputs[n])
+    single.set_option(_lib.OPT_KERNEL_TIMERS, 1)  # never captured
+    config = opt_config("adam", 1e-3)
+    data = [n for n, _, _, _ in compiled.spec.inputs]
+    for step in range(4):  # the second step captures the sequence, the later ones replay it on new batches
+        batch = [np.roll(inputs[n], step, axis=0) for n in data]
+        plan.bind_many([plan.slot(n) for n in data], batch)
+        for n, value in zip(data, batch):
+            single.bind(n, value)
+        plan.train_step(config)
+        single.execute()
+        single.optimizer_step(config)
+    for got, expected in zip(plan.outputs(), [single.read_output(i) for i in range(1 + len(compiled.spec.parameters))]):
+        assert got.tobytes() == expected.tobytes()
+    params, m, v = plan.read_state(moments=True)
+    for i in range(len(compiled.spec.parameters)):
+        assert params[i].tobytes() == single.read_parameter(i).tobytes()
+    flat = np.concatenate([np.pad(a.reshape(-1), (0, -a.size % 4)) for a in v])
+    assert flat.tobytes() == single.read_moments(1).tobytes()
+    assert plan.loss() == single.loss()
+
+
+def test_wrong_slots_and_sizes_upload_nothing(cuda_device):
+    w, compiled, inputs = traced("poisson1d", 64)
+    plan = Plan(compiled.spec, 0)
+    names = [n for n, _, _ in compiled.spec.parameters]
+    for slots, values in [([0, 99], [inputs[names[0]], inputs[names[1]]]), ([0, 1], [inputs[names[0]], np.zeros(999)])]:
+        with pytest.raises(_lib.BackendError):
+            plan.bind_many(slots, values)
+    with pytest.raises(_lib.BackendError) as caught:
+        plan.read_input(names[0], np.shape(inputs[names[0]]))
+    assert caught.value.status == _lib.NOT_BOUND
+
+
+def test_read_back_buffers_are_recycled_and_bounded(cuda_device):
+    first = _host.empty(1000, np.dtype(np.float32))
+    address = first.__array_interface__["data"][0]
+    view = first[10:20]
+    del first
+    second = _host.empty(1000, np.dtype(np.float32))  # the view keeps the first block out of the pool
+    assert second.__array_interface__["data"][0] != address
+    del view
+    assert _host.empty(1000, np.dtype(np.float32)).__array_interface__["data"][0] == address
+    held = [_host.empty(_host.LIMIT // 16, np.dtype(np.float64)) for _ in range(4)]  # more than the limit in all
+    assert all(a.flags.writeable for a in held)
+    assert _host._total <= _host.LIMIT
+    del held
+    assert _host._idle_bytes <= _host.IDLE_LIMIT
+
+
+def test_repeated_calls_follow_changed_arguments(cuda_device):
+    # Same structure: bound without a new signature; another shape, another static value: traced anew.
+    def loss(params, p, scale):
+        u = qb.vmap(lambda x: (qb.tanh(x.reshape(1, -1) @ params["w"] + params["b"]) @ params["v"]).reshape(()))(p)
+        return qb.mean((scale * u - 1.0) ** 2)
+
+    rng = np.random.default_rng(3)
+    params = {"w": rng.normal(size=(2, 16)), "b": np.zeros(16), "v": rng.normal(size=(16, 1))}
+    step = qb.jit(qb.value_and_grad(loss), device="cuda:0")
+    points = rng.normal(size=(40, 2))
+
+    def value_of(p, scale):
+        u = np.tanh(p @ params["w"] + params["b"]) @ params["v"]
+        return np.mean((scale * u[:, 0] - 1.0) ** 2)
+
+    for p, scale in [(points, 1.0), (points[::-1], 1.0), (points[:7], 1.0), (points, 2.0), (points, 1.0)]:
+        value, grads = step(params, p, scale)
+        assert abs(value - value_of(p, scale)) <= 1e-12
+        assert sorted(grads) == ["b", "v", "w"] and grads["v"].shape == (16, 1)
