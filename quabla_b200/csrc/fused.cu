@@ -22,90 +22,53 @@ FusedEntry<T> make_entry() {
     e.smem_bytes = G::SMEM_BASE_BYTES;
     e.scratch_per_layer = G::SCRATCH_PER_CTA;
     e.tensor_core = false;
+    e.dw_bytes = 0;
+    e.width = W;
     e.threads = FUSED_THREADS;
     e.ctas_per_sm = 1;
     return e;
 }
 
-template <int CODE, int PG, int ACT>
-FusedEntry<float> make_mma_entry() {
-    typedef MmaGeom<CODE, PG> G;
-    FusedEntry<float> e;
-    e.kernel = fused_mma_kernel<CODE, PG, ACT>;
-    e.streams = G::S;
-    e.tile_points = G::TP;
-    e.smem_bytes = G::SMEM_BASE_BYTES;
-    e.scratch_per_layer = G::SCRATCH_PER_CTA;
-    e.tensor_core = true;
-    e.threads = G::THREADS;
-    e.ctas_per_sm = 3 - PG;
-    return e;
-}
-
-// QB200_FUSED=simt keeps the FP32-pipe variant for float32 width-64 networks
-// (for comparisons); the default is the tensor-core (3xTF32) variant.
+// QB200_FUSED=simt keeps the FP32-pipe variant for float32 width-64 networks (for comparisons); the default is the
+// tensor-core variant.
 bool want_simt() {
     const char* env = getenv("QB200_FUSED");
     return env != nullptr && strcmp(env, "simt") == 0;
 }
 
-// QB200_FUSED_TILE=32 selects the one-CTA-per-SM variant (32 points per tile, 256 threads); the
-// default is two CTAs per SM with 16 points per tile each.
-bool want_wide_tile() {
-    const char* env = getenv("QB200_FUSED_TILE");
-    return env != nullptr && strcmp(env, "32") == 0;
-}
-
 }  // namespace
-
-// tanh networks have every variant; sin networks the default ones (tensor-core kernel with two CTAs per SM at
-// width 64, the FP32/FP64-pipe kernel at widths 16 and 32) and otherwise fall to the layer-wise engine.
-#define QB_MMA_CASE(CODE)                                                                                        \
-    if (width == 64 && code == CODE && !want_simt()) {                                                            \
-        if (act == ACT_TANH) {                                                                                    \
-            *out = want_wide_tile() ? make_mma_entry<CODE, 2, ACT_TANH>() : make_mma_entry<CODE, 1, ACT_TANH>(); \
-            return true;                                                                                          \
-        }                                                                                                         \
-        if (!want_wide_tile()) {                                                                                  \
-            *out = make_mma_entry<CODE, 1, ACT_SIN>();                                                            \
-            return true;                                                                                          \
-        }                                                                                                         \
-        return false;                                                                                             \
-    }
 
 // Signature codes: 0 = value only; 1 = {1}; 2 = {2}; 3 = {3}; 4 = {4}; 6 = {1,1};
 // 7 = {2,1}; 11 = {1,2}; 12 = {2,2}; SIG_MERGED + 6 / 31 = {1,1} / {1,1,1} plus the merged
 // second-order stream (2-D / 3-D Laplacian).
-#define QB_CASE(T, W, CODE)                                     \
-    if (width == W && code == CODE) {                           \
-        if (act == ACT_TANH) {                                  \
-            *out = make_entry<T, W, CODE, ACT_TANH>();          \
-            return true;                                        \
-        }                                                       \
-        if (W < 64) {                                           \
-            *out = make_entry<T, (W < 64 ? W : 16), CODE, ACT_SIN>(); \
-            return true;                                        \
-        }                                                       \
-        return false;                                           \
+#define QB_CASE(T, W, CODE)                                                                            \
+    if (width == W && code == CODE) {                                                                  \
+        if (act == ACT_SIN && sizeof(T) == 4) return false; /* the comparison variant carries tanh only */ \
+        *out = act == ACT_TANH ? make_entry<T, W, CODE, ACT_TANH>()                                    \
+                               : make_entry<T, W, CODE, sizeof(T) == 4 ? ACT_TANH : ACT_SIN>();        \
+        return true;                                                                                   \
     }
 
 template <>
-bool fused_lookup<float>(int width, int code, int act, FusedEntry<float>* out) {
+bool fused_lookup<float>(int width, bool uniform, int layers, int code, int act, FusedEntry<float>* out) {
     if (act != ACT_TANH && act != ACT_SIN) return false;
-    QB_MMA_CASE(0) QB_MMA_CASE(1) QB_MMA_CASE(2) QB_MMA_CASE(4) QB_MMA_CASE(7) QB_MMA_CASE(12)
-    QB_MMA_CASE(SIG_MERGED + 6) QB_MMA_CASE(SIG_MERGED + 31)
-    QB_CASE(float, 64, 0) QB_CASE(float, 64, 1) QB_CASE(float, 64, 2) QB_CASE(float, 64, 4)
-    QB_CASE(float, 64, 7) QB_CASE(float, 64, 12) QB_CASE(float, 64, SIG_MERGED + 6)
-    QB_CASE(float, 32, 0) QB_CASE(float, 32, 1) QB_CASE(float, 32, 2) QB_CASE(float, 32, 12)
-    QB_CASE(float, 32, SIG_MERGED + 6)
-    QB_CASE(float, 16, 0) QB_CASE(float, 16, 1) QB_CASE(float, 16, 2) QB_CASE(float, 16, 12)
-    QB_CASE(float, 16, SIG_MERGED + 6)
+    if (want_simt()) {
+        if (!uniform) return false;
+        QB_CASE(float, 64, 0) QB_CASE(float, 64, 1) QB_CASE(float, 64, 2) QB_CASE(float, 64, 4)
+        QB_CASE(float, 64, 7) QB_CASE(float, 64, 12) QB_CASE(float, 64, SIG_MERGED + 6)
+        return false;
+    }
+    if (width <= 16) return fused_mma_lookup<16>(layers, code, act, out);
+    if (width <= 32) return fused_mma_lookup<32>(layers, code, act, out);
+    if (width <= 48) return fused_mma_lookup<48>(layers, code, act, out);
+    if (width <= 64) return fused_mma_lookup<64>(layers, code, act, out);
     return false;
 }
 
 template <>
-bool fused_lookup<double>(int width, int code, int act, FusedEntry<double>* out) {
-    if (act != ACT_TANH && act != ACT_SIN) return false;
+bool fused_lookup<double>(int width, bool uniform, int layers, int code, int act, FusedEntry<double>* out) {
+    (void)layers;
+    if (!uniform || (act != ACT_TANH && act != ACT_SIN)) return false;
     QB_CASE(double, 16, 0) QB_CASE(double, 16, 1) QB_CASE(double, 16, 2) QB_CASE(double, 16, 7)
     QB_CASE(double, 16, 12) QB_CASE(double, 16, SIG_MERGED + 6)
     QB_CASE(double, 32, 0) QB_CASE(double, 32, 1) QB_CASE(double, 32, 2)
@@ -113,8 +76,7 @@ bool fused_lookup<double>(int width, int code, int act, FusedEntry<double>* out)
 }
 
 template <typename T>
-cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, cudaStream_t stream, const FusedArgs<T>& args) {
-    const size_t smem = fused_smem_bytes(entry, args.prog.n_instr);
+cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, size_t smem, cudaStream_t stream, const FusedArgs<T>& args) {
     cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(entry.kernel),
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -128,17 +90,21 @@ cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, cudaStream_t stre
     return cudaGetLastError();
 }
 
-size_t fused_weight_image_bytes(int hidden_to_hidden) {
-    return (size_t)std::max(hidden_to_hidden, 1) * 4 * WIMG_PLANE * sizeof(uint32_t);
+size_t fused_weight_image_bytes(int hidden_to_hidden, int width) {
+    return (size_t)std::max(hidden_to_hidden, 1) * 4 * width * (width + 8);
 }
 
-cudaError_t fused_prep_launch(const float* params, const int* w_off, int hidden_to_hidden, void* images,
-                              cudaStream_t stream) {
+cudaError_t fused_prep_launch(const float* params, const int* w_off, const int* rows, const int* cols, int hidden_to_hidden,
+                              int width, void* images, float* scales, cudaStream_t stream) {
     if (hidden_to_hidden < 1) return cudaSuccess;
     PrepArgs p;
     p.layers = hidden_to_hidden;
-    for (int i = 0; i <= FUSED_MAX_LAYERS; ++i) p.w_off[i] = i < hidden_to_hidden ? w_off[i] : 0;
-    prep_weights_kernel<<<dim3(4, hidden_to_hidden), 256, 0, stream>>>(params, p, static_cast<uint32_t*>(images));
+    for (int i = 0; i <= FUSED_MAX_LAYERS; ++i) {
+        p.w_off[i] = i < hidden_to_hidden ? w_off[i] : 0;
+        p.rows[i] = i < hidden_to_hidden ? rows[i] : 0;
+        p.cols[i] = i < hidden_to_hidden ? cols[i] : 0;
+    }
+    prep_weights_kernel<<<hidden_to_hidden, 1024, 0, stream>>>(params, p, width, static_cast<uint32_t*>(images), scales);
     return cudaGetLastError();
 }
 
@@ -159,7 +125,7 @@ cudaError_t unarmed_wait_launch(int* error, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template cudaError_t fused_launch<float>(const FusedEntry<float>&, int, cudaStream_t, const FusedArgs<float>&);
-template cudaError_t fused_launch<double>(const FusedEntry<double>&, int, cudaStream_t, const FusedArgs<double>&);
+template cudaError_t fused_launch<float>(const FusedEntry<float>&, int, size_t, cudaStream_t, const FusedArgs<float>&);
+template cudaError_t fused_launch<double>(const FusedEntry<double>&, int, size_t, cudaStream_t, const FusedArgs<double>&);
 
 }  // namespace qb

@@ -14,13 +14,18 @@ struct FusedEntry {
     int streams;                  // S
     int tile_points;              // TP
     size_t smem_bytes;            // dynamic shared memory per CTA, without the residual program
+    size_t dw_bytes;              // tensor-core variant: running weight-gradient sums of one layer, in shared memory
+                                  // behind the program when they fit, else in global memory
     size_t scratch_per_layer;     // saved-jet elements per CTA per hidden layer (each of Z and H)
-    bool tensor_core;             // 3xTF32 variant: needs the pre-split weight images
+    bool tensor_core;             // split-operand variant: needs the pre-split weight images
+    int width;                    // hidden width the kernel is built for (networks up to it run padded)
     int threads;                  // threads per CTA
     int ctas_per_sm;              // CTAs the kernel is sized to co-reside on one SM
 };
 
 constexpr size_t FUSED_MAX_SMEM = 227 * 1024;
+constexpr size_t FUSED_SM_SMEM = 228 * 1024;      // of an SM; a resident CTA takes FUSED_CTA_SMEM of it besides its own
+constexpr size_t FUSED_CTA_SMEM = 1024;
 
 // Dynamic shared memory of a launch: the regions plus the staged residual program.
 template <typename T>
@@ -28,20 +33,26 @@ inline size_t fused_smem_bytes(const FusedEntry<T>& entry, int n_instr) {
     return entry.smem_bytes + (size_t)n_instr * 16 + 16;
 }
 
-// True when a kernel exists for this dtype, hidden width, derivative signature code (sum over
-// directions j of order_j * 5^j) and activation (ACT_TANH or ACT_SIN).
+// True when a kernel exists for this dtype, largest hidden width, number of hidden layers, derivative signature code
+// (sum over directions j of order_j * 5^j) and activation (ACT_TANH or ACT_SIN).  `uniform`: every hidden layer has
+// that width (the FP32/FP64-pipe kernels have no padding).
 template <typename T>
-bool fused_lookup(int width, int code, int act, FusedEntry<T>* out);
+bool fused_lookup(int width, bool uniform, int layers, int code, int act, FusedEntry<T>* out);
 
-// Launches entry.kernel; sets the shared-memory attribute on first use.
+// Split-operand kernels of one padded width (fused_mma_w*.cu).
+template <int W>
+bool fused_mma_lookup(int layers, int code, int act, FusedEntry<float>* out);
+
+// Launches entry.kernel with `smem` bytes of dynamic shared memory.
 template <typename T>
-cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, cudaStream_t stream, const FusedArgs<T>& args);
+cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, size_t smem, cudaStream_t stream, const FusedArgs<T>& args);
 
-// Bytes of the pre-split weight images of `hidden_to_hidden` layers of width 64.
-size_t fused_weight_image_bytes(int hidden_to_hidden);
-// Writes the images from the flat float32 parameters; w_off[i] is the offset of network layer 1 + i.
-cudaError_t fused_prep_launch(const float* params, const int* w_off, int hidden_to_hidden, void* images,
-                              cudaStream_t stream);
+// Bytes of the pre-split weight images of `hidden_to_hidden` layers padded to `width`.
+size_t fused_weight_image_bytes(int hidden_to_hidden, int width);
+// Writes the images and their scales from the flat float32 parameters; image i is network layer 1 + i, of
+// rows[i] x cols[i] at offset w_off[i].
+cudaError_t fused_prep_launch(const float* params, const int* w_off, const int* rows, const int* cols, int hidden_to_hidden,
+                              int width, void* images, float* scales, cudaStream_t stream);
 // One thread's bounded wait on a barrier that is never completed: raises *error when it gives up.
 cudaError_t unarmed_wait_launch(int* error, cudaStream_t stream);
 

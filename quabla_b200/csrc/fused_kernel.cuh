@@ -76,6 +76,7 @@ struct FusedArgs {
     const T* params;
     int w_off[FUSED_MAX_LAYERS + 1];  // layer l = 0..L (L is the head)
     int b_off[FUSED_MAX_LAYERS + 1];  // -1: no bias
+    int width[FUSED_MAX_LAYERS + 1];  // hidden widths (the tensor-core variant pads them)
     const T* table;
     int ncols;
     long long n_points;
@@ -87,10 +88,12 @@ struct FusedArgs {
     T extra;
     T* scratch_z;       // per CTA [L][S][TP][W]
     T* scratch_h;       // per CTA [L][S][TP][W]
-    T* grad_cta;        // [gridDim.x][P]
+    T* grad_cta;        // [gridDim.x][P]; entries of no parameter are zero and stay so
     double* loss_cta;   // [gridDim.x]
     int forward_only;
     const void* weight_images;  // tensor-core variant: pre-split weight images (prep_weights_kernel)
+    const float* image_scales;  // and their scales
+    float* dw_scratch;          // tensor-core variant: running weight-gradient sums, or null: in shared memory
     int* error;                 // set to 1 when a bounded wait inside the kernel gave up
 };
 
@@ -183,7 +186,7 @@ __device__ __forceinline__ void tile_gemm(const T* __restrict__ A, const T* __re
 }
 
 // Derivatives of the fused engines' activations (ACT_TANH or ACT_SIN, a compile-time choice: a run-time switch
-// cost the tensor-core kernel 8 % on the tanh path) at z; *value receives the activation itself.
+// cost 8 % on the tanh path) at z; *value receives the activation itself.
 template <typename T, int ACT>
 __device__ __forceinline__ TanhD<T> fused_activation(T z, T* value) {
     if (ACT == ACT_SIN) return TanhD<T>(z, ACT_SIN, value);

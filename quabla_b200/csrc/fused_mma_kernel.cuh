@@ -1,24 +1,32 @@
-// Fused engine, float32, hidden width 64, weight contractions on the tensor
-// cores with the 3xTF32 split: every float32 operand x is written as
-// hi + lo with hi = tf32(x), lo = tf32(x - hi), and a product A.B is
-// accumulated in float32 as A_lo.B_hi + A_hi.B_lo + A_hi.B_hi, which keeps
-// float32 accuracy (the dropped A_lo.B_lo term is ~2^-22 relative).
+// Fused engine, float32, hidden widths up to 64, weight contractions on the tensor cores with operands split into
+// two float16 parts.
 //
-// Same structure as fused_step_kernel (fused_kernel.cuh): one persistent CTA
-// per SM walks tiles of 32 points, runs forward / residual / reverse sweep per
-// tile, keeps the saved jets in an L2-resident per-CTA scratch and accumulates
-// weight gradients per CTA.  What changes is who owns what:
+// Split.  A block of 16 x 16 elements (16 points x 16 units of one stream) is scaled by a power of two so that its
+// largest element lies in [2^13, 2^14), and every scaled element y is written as hi + lo with hi = f16(y) and
+// lo = f16(y - hi).  The pair carries y to 2^-23 of itself down to 2^-16 of the block's largest element and to
+// 2^-39 of that largest element below (hi and lo are then subnormal).  A product A.B is lo.hi + hi.lo + hi.hi,
+// three m16n8k16 instructions per 16 contraction elements: half the tensor-pipe time and half the instructions of three
+// tf32 products, which left 2e-7 per product against 1e-7 here (the dropped lo.lo is of random sign).  One
+// contraction step of 16 reads exactly one block of either operand, so the blocks' scales multiply the step's
+// partial sum on its way into the running sum: a multiply-add where a plain addition was needed anyway.
 //
-//   warp w: point group pg = w & 1 (16 points), column group cg = w >> 1 (16 units);
-//   for every stream s the warp owns the 16 x 16 tile (points x units) as two
-//   m16n8k8 accumulator fragments, so thread (g = lane / 4, t = lane % 4) holds
-//   points {g, g + 8} x units {2t, 2t + 1} of both fragments for ALL streams,
-//   and the tanh-jet composition stays register-only.
+// Same structure as fused_step_kernel (fused_kernel.cuh): persistent CTAs walk tiles of 16 points, run forward /
+// residual / reverse sweep per tile, keep the saved jets in an L2-resident per-CTA scratch and accumulate weight
+// gradients per CTA.  Warp w owns units 16 w .. 16 w + 15 (W / 16 warps): for every stream the 16 x 16 tile
+// (points x units) as two m16n8 accumulator fragments, so thread (g = lane / 4, t = lane % 4) holds points
+// {g, g + 8} x units {2t, 2t + 1} of both fragments for ALL streams, and the jet composition stays register-only.
+// Networks narrower than W (or of unequal widths) run padded with zero weights: a padded unit's activation meets
+// only zero weights and its cotangent is zero.
 //
-// Replaces, like the SIMT variant, the reference's per-node plan execution
-// (crates/quabla-core/src/tensor_ir/cuda.rs:1792-2972) and its cuBLAS
-// strided-batched GEMV-shaped calls (cuda.rs:4936-5035).
+// Bound: issue slots and latencies of the epilogues between the contractions (the tensor pipe is not the limit), which
+// is why a CTA is one point group with as few registers as its stream count allows: as many CTAs as fit
+// overlap one another's phases (three per SM at width 64 and up to four streams).
+//
+// Replaces the reference's per-node plan execution (crates/quabla-core/src/tensor_ir/cuda.rs:1792-2972) and its
+// cuBLAS strided-batched GEMV-shaped calls (cuda.rs:4936-5035).
 #pragma once
+#include <cuda_fp16.h>
+
 #include <cstdint>
 #include <cstdio>
 
@@ -26,42 +34,61 @@
 
 namespace qb {
 
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return r;
+// Four 8x8 matrices of 16-bit elements; thread (g, t) receives elements 2t, 2t + 1 of row g of each (TRANS: of
+// column g), the m16n8k16 fragment layouts.
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const __half* row_ptr) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(row_ptr);
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(at));
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(at));
 }
 
-// hi = x with the 13 low mantissa bits cleared (a valid tf32; the remainder x - hi is exact),
-// lo = that remainder ROUNDED to tf32.  Rounding matters: truncating lo leaves a one-sided
-// error of up to 2^-21 |x| that accumulates linearly over the contraction.  The tensor core
-// ignores the 13 low bits of an operand, so adding half a tf32 ulp (bit 12) to the remainder's
-// bit pattern rounds it to nearest with one integer add instead of a cvt.rna.tf32.
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-    hi = __float_as_uint(x) & 0xffffe000u;
-#ifdef QB_SPLIT_CVT
-    lo = to_tf32(x - __uint_as_float(hi));
-#else
-    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
-#endif
-}
-
-// Four 8x8 matrices of 16-bit pairs = four 8x4 tiles of 32-bit words: thread (g, t) of the
-// warp receives word t of row g of each tile, which is exactly the m16n8k8 tf32 fragment
-// layout when rows are contiguous in the fragment's k index.
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* row_ptr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"((uint32_t)__cvta_generic_to_shared(row_ptr)));
-}
-
-// d += a (16x8, row) * b (8x8, col), tf32 operands, float32 accumulate.
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    // Not volatile: the accumulator operands carry the dependencies, the compiler may interleave
-    // independent chains.
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+// d += a (16x16, row) * b (16x8, col), float16 operands, float32 accumulate.  Not volatile: the accumulator operands
+// carry the dependencies, the compiler may interleave independent chains.
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// acc += f * (A_lo.B_hi + A_hi.B_lo + A_hi.B_hi) of one 16 x 16 by 16 x 16 step.  The tensor core adds into its
+// accumulator with truncation, so every step chains its three products from zero and the partial is added to the
+// running sum with a round-to-nearest multiply-add.
+__device__ __forceinline__ void mma_step(float (&acc)[2][4], const uint32_t (&ahi)[4], const uint32_t (&alo)[4],
+                                         const uint32_t (&bhi)[4], const uint32_t (&blo)[4], float f) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma_f16(part, alo, bhi[2 * j], bhi[2 * j + 1]);
+        mma_f16(part, ahi, blo[2 * j], blo[2 * j + 1]);
+        mma_f16(part, ahi, bhi[2 * j], bhi[2 * j + 1]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(part[c], f, acc[j][c]);
+    }
+}
+
+// Power-of-two scale of a block whose largest magnitude has the bit pattern `largest`: *inverse maps it into
+// [2^13, 2^14), the returned factor maps back.  Blocks below 2^-113 (and empty ones) share the scale of that size.
+__device__ __forceinline__ float block_scale(uint32_t largest, float* inverse) {
+    const uint32_t e = max(largest >> 23, 14u);
+    *inverse = __uint_as_float((267u - e) << 23);
+    return __uint_as_float((e - 13u) << 23);
+}
+
+// Two scaled elements as packed float16 hi and lo pairs.
+__device__ __forceinline__ void split_f16(float x0, float x1, float inverse, uint32_t& hi, uint32_t& lo) {
+    const float y0 = x0 * inverse, y1 = x1 * inverse;
+    const __half2 h = __floats2half2_rn(y0, y1);
+    const float2 back = __half22float2(h);
+    const __half2 l = __floats2half2_rn(y0 - back.x, y1 - back.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
 // ---- asynchronous staging: bulk copies (TMA engine, no multicast) and cp.async ----
@@ -103,129 +130,81 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// Weight images written by prep_weights_kernel, one per hidden-to-hidden layer:
-// [4][64][WIMG_LDH] tf32 words = {forward hi, forward lo, transposed hi, transposed lo}.
-// An image is the B operand stored [n][k] (k contiguous, rows padded), exactly as it sits
-// in shared memory: forward B(k, n) = W[k][n], transposed B(k, n) = W[n][k].
-constexpr int WIMG_LDH = 68;
-constexpr int WIMG_PLANE = 64 * WIMG_LDH;            // words per plane
-constexpr int WIMG_PAIR_BYTES = 2 * WIMG_PLANE * 4;  // hi + lo of one orientation
 
+// Weight images written by prep_weights_kernel, one per hidden-to-hidden layer: {hi, lo} planes [W][W + 8] halves of
+// the row-major [in][out] matrix, zero-padded to W x W, scaled as one block; its factor goes to scales[layer].  The
+// forward contraction reads it transposed (ldmatrix .trans), the data gradient as it is.
 struct PrepArgs {
     int layers;                       // hidden-to-hidden layers
     int w_off[FUSED_MAX_LAYERS + 1];  // parameter offset of network layer 1 + i
+    int rows[FUSED_MAX_LAYERS + 1];   // its true input and output widths
+    int cols[FUSED_MAX_LAYERS + 1];
 };
 
-static __global__ void prep_weights_kernel(const float* __restrict__ params, PrepArgs p, uint32_t* __restrict__ images) {
-    const int layer = blockIdx.y;  // hidden-to-hidden layer index 0..layers-1 (network layer index - 1)
-    if (layer >= p.layers) return;
+static __global__ void __launch_bounds__(1024) prep_weights_kernel(const float* __restrict__ params, PrepArgs p, int W,
+                                                                   uint32_t* __restrict__ images, float* __restrict__ scales) {
+    __shared__ uint32_t warp_max[32];
+    const int layer = blockIdx.x, rows = p.rows[layer], cols = p.cols[layer];
     const float* w = params + p.w_off[layer];
-    uint32_t* img = images + (size_t)layer * 4 * WIMG_PLANE;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 64 * 64; e += gridDim.x * blockDim.x) {
-        const int k = e >> 6, n = e & 63;
+    uint32_t largest = 0;
+    for (int e = threadIdx.x; e < rows * cols; e += blockDim.x) largest = max(largest, __float_as_uint(w[e]) & 0x7fffffffu);
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = largest;
+    __syncthreads();
+    largest = __reduce_max_sync(0xffffffffu, (threadIdx.x & 31) < (blockDim.x >> 5) ? warp_max[threadIdx.x & 31] : 0u);
+    float inverse;
+    const float scale = block_scale(largest, &inverse);
+    if (threadIdx.x == 0) scales[layer] = scale;
+    const int pairs = W / 2, stride = (W + 8) / 2, plane = W * stride;  // in 32-bit words
+    uint32_t* img = images + (size_t)layer * 2 * plane;
+    for (int e = threadIdx.x; e < W * pairs; e += blockDim.x) {
+        const int r = e / pairs, c = 2 * (e % pairs);
+        const float x0 = (r < rows && c < cols) ? w[r * cols + c] : 0.0f;
+        const float x1 = (r < rows && c + 1 < cols) ? w[r * cols + c + 1] : 0.0f;
         uint32_t hi, lo;
-        split_tf32(w[e], hi, lo);
-        img[0 * WIMG_PLANE + n * WIMG_LDH + k] = hi;
-        img[1 * WIMG_PLANE + n * WIMG_LDH + k] = lo;
-        img[2 * WIMG_PLANE + k * WIMG_LDH + n] = hi;
-        img[3 * WIMG_PLANE + k * WIMG_LDH + n] = lo;
+        split_f16(x0, x1, inverse, hi, lo);
+        img[r * stride + c / 2] = hi;
+        img[plane + r * stride + c / 2] = lo;
     }
 }
 
-// PG = point groups of 16 per tile.  PG = 2: 256 threads, 32 points, two weight buffers, one CTA per
-// SM.  PG = 1: 128 threads, 16 points, one weight buffer; half the shared memory, so two CTAs share
-// an SM and one's GEMM phases overlap the other's epilogues and residual program.
-template <int CODE, int PG>
+template <int CODE, int W_>
 struct MmaGeom {
     typedef Sig<CODE> sig;
-    static constexpr int W = 64;
+    static constexpr int W = W_;
     static constexpr int S = sig::S;
-    static constexpr int THREADS = 128 * PG;
-    static constexpr int NBUF = PG;  // weight-image buffers
-    static constexpr int TP = 16 * PG;
+    static constexpr int NW = W / 16;            // warps = column blocks
+    static constexpr int THREADS = 32 * NW;
+    static constexpr int TP = 16;
     static constexpr int ROWS = S * TP;
-    // Every operand row is 16-byte aligned and its stride is 4 (mod 32) words, so the eight
-    // row addresses of an ldmatrix tile fall into distinct bank groups.
-    static constexpr int LDA = 68;        // activations / cotangents, row-major [row][unit]
-    static constexpr int LDT = ROWS + 4;  // transposed operands of the weight gradient, [unit][row]
-    static constexpr int OFF_ACT = 0;                       // [ROWS][LDA]
-    static constexpr int LDH = 72;        // previous layer's jets [row][unit], read k-major: stride 8 (mod 32)
-    static constexpr int OFF_HT = OFF_ACT + ROWS * LDA;     // [ROWS][LDH] previous layer's jets
-    static constexpr int OFF_ZT = OFF_HT + ROWS * LDH;      // [64][LDT] pre-activation cotangents, transposed
-    static constexpr int OFF_WB = OFF_ZT + W * LDT;         // NBUF buffers x {hi, lo} x [64][WIMG_LDH]
-    static constexpr int OFF_RED = OFF_WB + NBUF * 2 * WIMG_PLANE;  // [5][PG][64] column reductions / [4][S][TP] head partials
-    static constexpr int RED = (5 * PG * W > 4 * ROWS) ? 5 * PG * W : 4 * ROWS;
-    static constexpr int OFF_U = OFF_RED + RED;             // [S][TP]
-    static constexpr int OFF_UH = OFF_U + ROWS;             // [S][TP]
-    static constexpr int OFF_BAR = OFF_UH + ROWS;           // NBUF mbarriers (4 words reserved)
-    static constexpr int TOTAL = OFF_BAR + 4;
-    static constexpr size_t SMEM_BASE_BYTES = ((size_t)TOTAL * sizeof(float) + 15) / 16 * 16;
-    // Saved jets keep the row stride of the shared-memory operand (LDA), so that one bulk copy saves a layer.
-    static constexpr size_t SCRATCH_PER_CTA = (size_t)S * TP * LDA;
+    // Rows of W + 8 halves: 16-byte aligned, and the eight row addresses of an ldmatrix tile fall into distinct
+    // bank groups for every W used (stride 4 (mod 8) words).
+    static constexpr int LD = W + 8;
+    static constexpr int PLANE = ROWS * LD;      // halves per operand plane
+    static constexpr int WPLANE = W * LD;        // halves per weight plane
+    static constexpr int ACT_BYTES = 4 * PLANE;  // hi and lo
+    static constexpr int WIMG_BYTES = 4 * WPLANE;
+    static constexpr int OFF_ACT = 0;                      // activations / cotangents, [hi, lo][ROWS][LD]
+    static constexpr int OFF_HT = OFF_ACT + ACT_BYTES;     // previous layer's jets (weight-gradient operand), same layout
+    static constexpr int OFF_WB = OFF_HT + ACT_BYTES;      // weight image of the contraction at hand
+    static constexpr int OFF_RED = OFF_WB + WIMG_BYTES;    // [NW][S][TP] output-layer partials
+    static constexpr int OFF_U = OFF_RED + 4 * NW * ROWS;  // [S][TP]
+    static constexpr int OFF_UH = OFF_U + 4 * ROWS;        // [S][TP]
+    static constexpr int OFF_BAR = OFF_UH + 4 * ROWS;      // two mbarriers
+    static constexpr int OFF_VAR = OFF_BAR + 16;           // regions that depend on the depth:
+    // block scales [L + 1][S][NW], weight scales [L], parameters {biases [L][W], first layer [4][W], output layer
+    // [W]}, gradient sums of the same, of the output bias
+    static __host__ __device__ constexpr size_t var_bytes(int L) {
+        return 4 * ((size_t)(L + 1) * S * NW + L + 2 * (size_t)(L + 5) * W + 4);
+    }
+    static __host__ __device__ constexpr size_t base_bytes(int L) { return ((size_t)OFF_VAR + var_bytes(L) + 15) / 16 * 16; }
+    static constexpr size_t DW_BYTES = 4 * (size_t)W * W;  // running weight-gradient sums of one layer
+    // Registers decide how many CTAs share an SM: 168 per thread hold up to four streams, 224 to 255 more.
+    static constexpr int MIN_CTAS = (S <= 4 ? 12 : 8) / NW;
+    // Saved jets: the operand planes as they sit in shared memory, one bulk copy per layer.  Saved pre-activations:
+    // read back by the thread that wrote them, so laid out per thread.
+    static constexpr size_t SCRATCH_PER_CTA = (size_t)ROWS * LD;
 };
-
-// acc[s][j] += A[rows of stream s][64] * B[64][16 columns of this warp], 3xTF32.
-// A: activations [ROWS][LDA] float32 (split here); B: pre-split weight image [n][k].
-template <int S, int TP, int LDA>
-__device__ __forceinline__ void warp_gemm_3xtf32(const float* __restrict__ A, const uint32_t* __restrict__ Bhi,
-                                                 const uint32_t* __restrict__ Blo, int row0, int col0, int lane,
-                                                 float (&acc)[S][2][4]) {
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[s][j][c] = 0.0f;
-    const int mi = lane >> 3, rr = lane & 7;
-    // A tiles: (rows 0-7, k 0-3), (rows 8-15, k 0-3), (rows 0-7, k 4-7), (rows 8-15, k 4-7).
-    const float* a_lane = A + (row0 + rr + (mi & 1) * 8) * LDA + (mi >> 1) * 4;
-    // B tiles: (n 0-7, k 0-3), (n 0-7, k 4-7), (n 8-15, k 0-3), (n 8-15, k 4-7).
-    const int b_lane = (col0 + (mi >> 1) * 8 + rr) * WIMG_LDH + (mi & 1) * 4;
-#pragma unroll 2
-    for (int kb = 0; kb < 8; ++kb) {
-        uint32_t bhi[4], blo[4];
-        ldmatrix_x4(bhi, Bhi + b_lane + kb * 8);
-        ldmatrix_x4(blo, Blo + b_lane + kb * 8);
-        // The tensor core adds into its accumulator with truncation, which biases a long chain
-        // (measured: 5e-6 relative on the gradients against 1e-6 with this scheme).  So the three
-        // products of one k-block chain from zero, and the block's partial is added to the running
-        // sum with a round-to-nearest float add.
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-            uint32_t raw[4], ahi[4], alo[4];
-            ldmatrix_x4(raw, a_lane + s * TP * LDA + kb * 8);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) split_tf32(__uint_as_float(raw[q]), ahi[q], alo[q]);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                mma_tf32(part, alo, bhi[2 * j], bhi[2 * j + 1]);
-                mma_tf32(part, ahi, blo[2 * j], blo[2 * j + 1]);
-                mma_tf32(part, ahi, bhi[2 * j], bhi[2 * j + 1]);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[s][j][c] += part[c];
-            }
-        }
-    }
-}
-
-// Sum v[4] (this thread's 4 units, already summed over its points) over the 8
-// point rows of the warp; lanes with g == 0 store the warp's totals.
-__device__ __forceinline__ void reduce_units_over_points(float (&v)[4], float* dst, int lane, int col0, int t) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        v[c] += __shfl_xor_sync(0xffffffffu, v[c], 4);
-        v[c] += __shfl_xor_sync(0xffffffffu, v[c], 8);
-        v[c] += __shfl_xor_sync(0xffffffffu, v[c], 16);
-    }
-    if (lane < 4) {
-        dst[col0 + 2 * t] = v[0];
-        dst[col0 + 2 * t + 1] = v[1];
-        dst[col0 + 8 + 2 * t] = v[2];
-        dst[col0 + 8 + 2 * t + 1] = v[3];
-    }
-}
-
 
 // Optional per-phase cycle counters of CTA 0 (compile with -DQB_PHASE_TIMING), printed once per launch.
 #ifdef QB_PHASE_TIMING
@@ -241,86 +220,185 @@ __device__ __forceinline__ void reduce_units_over_points(float (&v)[4], float* d
 #define QB_PHASE(i)
 #endif
 
-template <int CODE, int PG, int ACT>
-__global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<float> a) {
-    typedef MmaGeom<CODE, PG> G;
-    constexpr int THREADS = G::THREADS, NBUF = G::NBUF;
-    typedef Sig<CODE> SG;
-    constexpr int S = G::S, TP = G::TP, W = G::W, LDA = G::LDA, LDT = G::LDT, LDH = G::LDH, ROWS = G::ROWS;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float* smem = reinterpret_cast<float*>(smem_raw);
-    float* act = smem + G::OFF_ACT;
-    float* ht = smem + G::OFF_HT;
-    float* zt = smem + G::OFF_ZT;
-    uint32_t* wbuf = reinterpret_cast<uint32_t*>(smem + G::OFF_WB);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G::OFF_BAR);
-    float* red = smem + G::OFF_RED;
-    float* us = smem + G::OFF_U;
-    float* uh = smem + G::OFF_UH;
-    int4* code = reinterpret_cast<int4*>(smem_raw + G::SMEM_BASE_BYTES);
+// The warp's 16 x 16 block of every stream as scaled float16 pairs into the operand planes; scales [S][NW].
+template <int S, int NW, int LD, int PLANE>
+__device__ __forceinline__ void store_blocks(const float (&acc)[S][2][4], __half* planes, float* scales, int warp, int g, int t) {
+    uint32_t largest[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) m = max(m, __float_as_uint(acc[s][j][c]) & 0x7fffffffu);
+        largest[s] = __reduce_max_sync(0xffffffffu, m);
+    }
+    uint32_t* words = reinterpret_cast<uint32_t*>(planes) + (g * LD + 16 * warp + 2 * t) / 2;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        float inverse;
+        const float scale = block_scale(largest[s], &inverse);
+        if (g == 0 && t == 0) scales[s * NW + warp] = scale;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                uint32_t hi, lo;
+                split_f16(acc[s][j][2 * i], acc[s][j][2 * i + 1], inverse, hi, lo);
+                uint32_t* at = words + ((s * 16 + 8 * i) * LD + 8 * j) / 2;
+                at[0] = hi;
+                at[PLANE / 2] = lo;
+            }
+    }
+}
 
+// acc[s] = A[rows of stream s][W] * B[W][16 columns of this warp].  FORWARD: B(k, n) = W[k][n]; else B(k, n) = W[n][k].
+template <int S, int NW, int LD, int PLANE, int WPLANE, bool FORWARD>
+__device__ __forceinline__ void warp_contract(const __half* __restrict__ A, const __half* __restrict__ Wimg,
+                                              const float* __restrict__ scales, float wscale, int warp, int lane,
+                                              float (&acc)[S][2][4]) {
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[s][j][c] = 0.0f;
+    const int mi = lane >> 3, rr = lane & 7;
+    const __half* a_lane = A + (rr + (mi & 1) * 8) * LD + (mi >> 1) * 8;
+    const __half* b_lane = FORWARD ? Wimg + ((mi & 1) * 8 + rr) * LD + 16 * warp + (mi >> 1) * 8
+                                   : Wimg + (16 * warp + (mi >> 1) * 8 + rr) * LD + (mi & 1) * 8;
+#pragma unroll
+    for (int kb = 0; kb < NW; ++kb) {
+        uint32_t bhi[4], blo[4];
+        const __half* b = b_lane + (FORWARD ? kb * 16 * LD : kb * 16);
+        ldmatrix_x4<FORWARD>(bhi, b);
+        ldmatrix_x4<FORWARD>(blo, b + WPLANE);
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            uint32_t ahi[4], alo[4];
+            ldmatrix_x4<false>(ahi, a_lane + s * 16 * LD + kb * 16);
+            ldmatrix_x4<false>(alo, a_lane + s * 16 * LD + kb * 16 + PLANE);
+            mma_step(acc[s], ahi, alo, bhi, blo, scales[s * NW + kb] * wscale);
+        }
+    }
+}
+
+// Column sums over the 16 points of the warp's block (v: this thread's four units, its two points already added);
+// lanes with g == 0 add them to dst, which only this warp touches.
+__device__ __forceinline__ void add_column_sums(float (&v)[4], float* dst, int lane, int col0, int t) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        v[c] += __shfl_xor_sync(0xffffffffu, v[c], 4);
+        v[c] += __shfl_xor_sync(0xffffffffu, v[c], 8);
+        v[c] += __shfl_xor_sync(0xffffffffu, v[c], 16);
+    }
+    if (lane < 4) {
+        dst[col0 + 2 * t] += v[0];
+        dst[col0 + 2 * t + 1] += v[1];
+        dst[col0 + 8 + 2 * t] += v[2];
+        dst[col0 + 8 + 2 * t + 1] += v[3];
+    }
+}
+
+template <int CODE, int W, int ACT>
+__global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::MIN_CTAS) fused_mma_kernel(FusedArgs<float> a) {
+    typedef MmaGeom<CODE, W> G;
+    typedef Sig<CODE> SG;
+    constexpr int THREADS = G::THREADS, NW = G::NW, S = G::S, TP = G::TP, LD = G::LD, PLANE = G::PLANE, WPLANE = G::WPLANE;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __half* act = reinterpret_cast<__half*>(smem_raw + G::OFF_ACT);
+    __half* ht = reinterpret_cast<__half*>(smem_raw + G::OFF_HT);
+    __half* wbuf = reinterpret_cast<__half*>(smem_raw + G::OFF_WB);
+    float* red = reinterpret_cast<float*>(smem_raw + G::OFF_RED);
+    float* us = reinterpret_cast<float*>(smem_raw + G::OFF_U);
+    float* uh = reinterpret_cast<float*>(smem_raw + G::OFF_UH);
+    uint64_t* wbar = reinterpret_cast<uint64_t*>(smem_raw + G::OFF_BAR);  // weight image landed
+    uint64_t* hbar = wbar + 1;                                            // saved jets landed
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int col0 = warp * 16;  // first unit of the warp
+    const int L = a.L, d0 = a.d0, HL = L - 1;
+    const bool backward = a.forward_only == 0;
+    float* scl = reinterpret_cast<float*>(smem_raw + G::OFF_VAR);  // [L][S][NW] activations, then one row for the cotangents
+    float* scl_z = scl + L * S * NW;
+    float* wscl = scl_z + S * NW;        // [L], by hidden-to-hidden layer
+    float* pbias = wscl + L;             // [L][W]
+    float* pfirst = pbias + L * W;       // [4][W]
+    float* phead = pfirst + 4 * W;       // [W]
+    float* gbias = phead + W;            // gradient sums in the same order
+    float* gfirst = gbias + L * W;
+    float* ghead = gfirst + 4 * W;
+    int4* code = reinterpret_cast<int4*>(smem_raw + G::base_bytes(L));
+    float* sz = a.scratch_z + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
+    float* sh = a.scratch_h + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
+    // Running weight-gradient sums [HL][2 NW][THREADS] float4, every thread its own fragments: in shared memory when
+    // the host found room beside the other CTAs, else in global memory (L2).
+    float4* dws = a.dw_scratch != nullptr ? reinterpret_cast<float4*>(a.dw_scratch) + (size_t)blockIdx.x * HL * 2 * NW * THREADS
+                                          : reinterpret_cast<float4*>(code + a.prog.n_instr);
 #ifdef QB_PHASE_TIMING
     long long phase_[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     long long last_ = clock64();
 #endif
-    const int g = lane >> 2, t = lane & 3;
-    const int pg = PG == 2 ? (warp & 1) : 0, cg = PG == 2 ? (warp >> 1) : warp;
-    const int row0 = pg * 16;   // first point of the warp inside the tile
-    const int col0 = cg * 16;   // first unit of the warp
-    const int L = a.L, d0 = a.d0;
-    const bool backward = a.forward_only == 0;
-    float* my_grad = a.grad_cta + (size_t)blockIdx.x * a.P;
-    float* sz = a.scratch_z + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
-    float* sh = a.scratch_h + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
 
     for (int i = tid; i < a.prog.n_instr; i += THREADS) code[i] = a.prog.code[i];
+    for (int i = tid; i < L * W; i += THREADS) {
+        const int l = i / W, n = i % W;
+        pbias[i] = (a.b_off[l] >= 0 && n < a.width[l]) ? a.params[a.b_off[l] + n] : 0.0f;
+        gbias[i] = 0.0f;
+    }
+    for (int i = tid; i < 4 * W; i += THREADS) {
+        const int k = i / W, n = i % W;
+        pfirst[i] = (k < d0 && n < a.width[0]) ? a.params[a.w_off[0] + k * a.width[0] + n] : 0.0f;
+        gfirst[i] = 0.0f;
+    }
+    for (int i = tid; i < W; i += THREADS) {
+        phead[i] = i < a.width[L - 1] ? a.params[a.w_off[L] + i] : 0.0f;
+        ghead[i] = 0.0f;
+    }
+    if (tid < HL) wscl[tid] = a.image_scales[tid];
     if (backward)
-        for (int i = tid; i < a.P; i += THREADS) my_grad[i] = 0.0f;
+        for (int i = tid; i < HL * 2 * NW * THREADS; i += THREADS) dws[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     double loss_sum = 0.0;
+    float head_bias_grad = 0.0f;  // thread 0
+    const float head_bias = a.b_off[L] >= 0 ? a.params[a.b_off[L]] : 0.0f;
     const float seed = a.cotangent[0] * a.weight * a.extra;
     if (tid == 0) {
-#pragma unroll
-        for (int b = 0; b < NBUF; ++b) mbar_init(bars + b, 1);
+        mbar_init(wbar, 1);
+        mbar_init(hbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
 
-    // Unit of accumulator element (j, c) and its point index (0: row g, 1: row g + 8).
+    // Unit of accumulator element (j, c); its point is g for c < 2 and g + 8 above.
     auto unit_of = [&](int j, int c) { return col0 + j * 8 + 2 * t + (c & 1); };
 
-    const long long n_tiles = (a.n_points + TP - 1) / TP;
-    // Weight pipeline: the split weight images are bulk-copied into NBUF shared buffers in
-    // the fixed order a tile uses them (forward layers 1..L-1, then the transposed images
-    // of layers L-1..1), NBUF uses ahead of the GEMM that consumes them.
-    const int HL = L - 1;
+    const int n_tiles = (int)((a.n_points + TP - 1) / TP);
+    // The weight image of the next contraction is bulk-copied into shared memory as soon as the last one has been
+    // read, in the order a tile uses them: forward layers 1..L-1, then L-1..1.
     const int uses_per_tile = backward ? 2 * HL : HL;
-    const long long my_tiles = blockIdx.x < n_tiles ? (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    const long long total_uses = my_tiles * uses_per_tile;
-    const uint32_t* images = static_cast<const uint32_t*>(a.weight_images);
-    long long use = 0;
-    auto issue = [&](long long q) {
-        if (tid == 0 && q < total_uses) {
-            const int idx = (int)(q % uses_per_tile);
-            const int layer = idx < HL ? idx : 2 * HL - 1 - idx;
-            const int plane = idx < HL ? 0 : 2;
-            uint64_t* bar = bars + (q % NBUF);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(bar, WIMG_PAIR_BYTES);
-            bulk_load(wbuf + (q % NBUF) * 2 * WIMG_PLANE, images + ((size_t)layer * 4 + plane) * WIMG_PLANE,
-                      WIMG_PAIR_BYTES, bar);
-        }
+    const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    long long loads_left = (long long)my_tiles * uses_per_tile;
+    int next_use = 0;              // position of the next load in the tile's order
+    uint32_t wphase = 0, hphase = 0;
+    const __half* images = static_cast<const __half*>(a.weight_images);
+    auto load_weights = [&]() {  // thread 0
+        if (loads_left-- <= 0) return;
+        const int layer = next_use < HL ? next_use : 2 * HL - 1 - next_use;
+        if (++next_use == uses_per_tile) next_use = 0;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect_tx(wbar, G::WIMG_BYTES);
+        bulk_load(wbuf, images + (size_t)layer * 2 * WPLANE, G::WIMG_BYTES, wbar);
     };
-#pragma unroll
-    for (int q = 0; q < NBUF; ++q) issue(q);
-    for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const long long p0 = tile * TP;
+    if (tid == 0) load_weights();
+
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const long long p0 = (long long)tile * TP;
         float acc[S][2][4];
         float x[2][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const long long p = min(p0 + row0 + g + 8 * i, a.n_points - 1);
+            const long long p = min(p0 + g + 8 * i, a.n_points - 1);
 #pragma unroll
             for (int k = 0; k < 4; ++k) x[i][k] = k < d0 ? a.table[p * a.ncols + k] : 0.0f;
         }
@@ -328,7 +406,6 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
         // ------------------------------ forward ------------------------------
         for (int l = 0; l < L; ++l) {
             if (l == 0) {
-                const float* w0 = a.params + a.w_off[0];
 #pragma unroll
                 for (int s = 0; s < S; ++s)
 #pragma unroll
@@ -342,7 +419,7 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
                         for (int j = 0; j < 2; ++j)
 #pragma unroll
                             for (int c = 0; c < 4; ++c) {
-                                const float w = w0[k * W + unit_of(j, c)];
+                                const float w = pfirst[k * W + unit_of(j, c)];
                                 acc[0][j][c] += x[c >> 1][k] * w;
 #pragma unroll
                                 for (int dj = 0; dj < SG::ndirs; ++dj) acc[SG::base(dj)][j][c] += a.dirs[dj * d0 + k] * w;
@@ -350,44 +427,38 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
                     }
                 }
             } else {
-                const uint32_t* whi = wbuf + (use % NBUF) * 2 * WIMG_PLANE;
-                mbar_wait(bars + (use % NBUF), (uint32_t)((use / NBUF) & 1), a.error);
+                mbar_wait(wbar, wphase, a.error);
+                wphase ^= 1;
                 __syncthreads();  // the previous epilogue's activations are in place
                 if (backward && tid == 0) {
-                    // Save layer l-1's jets for the reverse sweep: the operand tile as it sits in shared memory,
-                    // one bulk copy (TMA engine) instead of 8-byte stores from every thread.
+                    // Save layer l-1's jets for the reverse sweep: the operand planes as they sit in shared memory, one
+                    // bulk copy (TMA engine).
                     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
                                      sh + (size_t)(l - 1) * G::SCRATCH_PER_CTA),
-                                 "r"(smem_u32(act)), "r"((uint32_t)(ROWS * LDA * sizeof(float)))
+                                 "r"(smem_u32(act)), "r"((uint32_t)G::ACT_BYTES)
                                  : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
-                QB_PHASE(0);      // wait for the weight image
-                warp_gemm_3xtf32<S, TP, LDA>(act, whi, whi + WIMG_PLANE, row0, col0, lane, acc);
+                QB_PHASE(0);  // wait for the weight image
+                warp_contract<S, NW, LD, PLANE, WPLANE, true>(act, wbuf, scl + (l - 1) * S * NW, wscl[l - 1], warp, lane, acc);
                 // The epilogue overwrites the operand: the bulk copy must have read it.
                 if (backward && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 __syncthreads();
-                issue(use + NBUF);
-                ++use;
-                QB_PHASE(1);  // forward GEMM
+                if (tid == 0) load_weights();
+                QB_PHASE(1);  // forward contraction
             }
-            if (a.b_off[l] >= 0) {
-                const float* bl = a.params + a.b_off[l];
 #pragma unroll
-                for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[0][j][c] += bl[unit_of(j, c)];
-            }
-            float* zl = sz + (size_t)l * G::SCRATCH_PER_CTA;
+                for (int c = 0; c < 4; ++c) acc[0][j][c] += pbias[l * W + unit_of(j, c)];
+            // The reverse sweep needs the pre-activation streams; of the primal one only tanh itself (z_0 for sin).
+            float4* zl = reinterpret_cast<float4*>(sz + (size_t)l * G::SCRATCH_PER_CTA) + tid;
             if (backward) {
 #pragma unroll
-                for (int s = 0; s < S; ++s)
+                for (int s = ACT == ACT_TANH ? 1 : 0; s < S; ++s)
 #pragma unroll
                     for (int j = 0; j < 2; ++j)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            st2(zl + ((size_t)s * TP + row0 + g + 8 * i) * W + col0 + j * 8 + 2 * t, acc[s][j][2 * i],
-                                acc[s][j][2 * i + 1]);
+                        zl[(2 * s + j) * THREADS] = make_float4(acc[s][j][0], acc[s][j][1], acc[s][j][2], acc[s][j][3]);
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j)
@@ -400,37 +471,34 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
 #pragma unroll
                     for (int s = 0; s < S; ++s) acc[s][j][c] = v[s];
                 }
+            if (backward && ACT == ACT_TANH) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) zl[j * THREADS] = make_float4(acc[0][j][0], acc[0][j][1], acc[0][j][2], acc[0][j][3]);
+            }
             if (l + 1 < L) {
-#pragma unroll
-                for (int s = 0; s < S; ++s)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            st2(act + (s * TP + row0 + g + 8 * i) * LDA + col0 + j * 8 + 2 * t, acc[s][j][2 * i],
-                                acc[s][j][2 * i + 1]);
-                // The next iteration saves this tile with a bulk copy: make the writes visible to that proxy.
+                store_blocks<S, NW, LD, PLANE>(acc, act, scl + l * S * NW, warp, g, t);
+                // The next iteration saves these planes with a bulk copy: make the writes visible to that proxy.
                 if (backward) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
         }
 
-        QB_PHASE(2);  // forward epilogues (bias, saves, tanh jets, staging of the next operand)
+        QB_PHASE(2);  // forward epilogues (bias, saves, jets, staging of the next operand)
         // ------------------------- head and residual -------------------------
-        float wh[2][4];
+        float wh[2][2];
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) wh[j][c] = a.params[a.w_off[L] + unit_of(j, c)];
+            for (int c = 0; c < 2; ++c) wh[j][c] = phead[unit_of(j, c)];
 #pragma unroll
         for (int s = 0; s < S; ++s)
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 float dot = 0.0f;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) dot += acc[s][j][2 * i] * wh[j][2 * i] + acc[s][j][2 * i + 1] * wh[j][2 * i + 1];
+                for (int j = 0; j < 2; ++j) dot += acc[s][j][2 * i] * wh[j][0] + acc[s][j][2 * i + 1] * wh[j][1];
                 dot += __shfl_xor_sync(0xffffffffu, dot, 1);
                 dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-                if (t == 0) red[(cg * S + s) * TP + row0 + g + 8 * i] = dot;
+                if (t == 0) red[(warp * S + s) * TP + g + 8 * i] = dot;
             }
         __syncthreads();
         if (tid < TP) {
@@ -439,11 +507,10 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
             const long long pc = valid ? p : a.n_points - 1;
 #pragma unroll
             for (int s = 0; s < S; ++s) {
-                float u = red[(0 * S + s) * TP + tid];
+                float u = red[s * TP + tid];
 #pragma unroll
-                for (int q = 1; q < 4; ++q) u += red[(q * S + s) * TP + tid];
-                if (s == 0 && a.b_off[L] >= 0) u += a.params[a.b_off[L]];
-                us[s * TP + tid] = u;
+                for (int q = 1; q < NW; ++q) u += red[(q * S + s) * TP + tid];
+                us[s * TP + tid] = s == 0 ? u + head_bias : u;
             }
             float r[MAX_REGS];
             run_program<float>(code, a.prog.n_instr, static_cast<const float*>(a.prog.consts), a.table + pc * a.ncols,
@@ -458,71 +525,66 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
         __syncthreads();
         QB_PHASE(3);  // head and residual program
         if (!backward) continue;
-        // The saved jets are read back below (cp.async): the bulk stores must have completed.  The
-        // barriers of the head phase separate this wait from the first prefetch.
-        if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 
         // ------------------------------ backward ------------------------------
+        auto load_jets = [&](int layer) {  // thread 0: saved jets of `layer` into ht
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_expect_tx(hbar, G::ACT_BYTES);
+            bulk_load(ht, sh + (size_t)layer * G::SCRATCH_PER_CTA, G::ACT_BYTES, hbar);
+        };
+        if (tid == 0 && HL > 0) {
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // the saves of the forward pass are complete
+            load_jets(HL - 1);
+        }
         {
             // Head: dW = sum h * uhat, db = sum uhat(primal), G = uhat (x) w.
-            float ug[S][2];
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                ug[s][0] = uh[s * TP + row0 + g];
-                ug[s][1] = uh[s * TP + row0 + g + 8];
-            }
             float pw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int s = 0; s < S; ++s)
+            for (int s = 0; s < S; ++s) {
+                const float u0 = uh[s * TP + g], u1 = uh[s * TP + g + 8];
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        pw[2 * j + (c & 1)] += acc[s][j][c] * ug[s][c >> 1];
-                        acc[s][j][c] = ug[s][c >> 1] * wh[j][c];
+                        const float u = c < 2 ? u0 : u1;
+                        pw[2 * j + (c & 1)] += acc[s][j][c] * u;
+                        acc[s][j][c] = u * wh[j][c & 1];
                     }
-            reduce_units_over_points(pw, red + pg * W, lane, col0, t);
-            __syncthreads();
-            if (tid < W) my_grad[a.w_off[L] + tid] += PG == 2 ? red[tid] + red[W + tid] : red[tid];
-            if (tid == 0 && a.b_off[L] >= 0) {
-                float total = 0.0f;
-                for (int p = 0; p < TP; ++p) total += uh[p];
-                my_grad[a.b_off[L]] += total;
             }
-            __syncthreads();
+            add_column_sums(pw, ghead, lane, col0, t);
+            if (tid == 0) {
+                float total = 0.0f;
+#pragma unroll
+                for (int p = 0; p < TP; ++p) total += uh[p];
+                head_bias_grad += total;
+            }
         }
         for (int l = L - 1; l >= 0; --l) {
-            const float* zl = sz + (size_t)l * G::SCRATCH_PER_CTA;
-            if (l > 0) {
-                // Prefetch the previous layer's saved jets (weight-gradient operand) while the
-                // transposed jets are computed.
-                const float* hp = sh + (size_t)(l - 1) * G::SCRATCH_PER_CTA;
-                for (int e = tid; e < ROWS * 16; e += THREADS)
-                    cp_async16(ht + (e >> 4) * LDH + 4 * (e & 15), hp + (size_t)(e >> 4) * LDA + 4 * (e & 15));
-                cp_async_commit();
-            }
+            const float4* zl = reinterpret_cast<const float4*>(sz + (size_t)l * G::SCRATCH_PER_CTA) + tid;
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < 2; ++j) {
+                float z[S][4];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    float z0[S], z1[S];
-#pragma unroll
-                    for (int s = 0; s < S; ++s)
-                        ld2(zl + ((size_t)s * TP + row0 + g + 8 * i) * W + col0 + j * 8 + 2 * t, z0[s], z1[s]);
-                    float g0[S], g1[S];
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        g0[s] = acc[s][j][2 * i];
-                        g1[s] = acc[s][j][2 * i + 1];
-                    }
-                    jet_apply_transposed<float, SG, ACT>(z0, g0, a.merge_w);
-                    jet_apply_transposed<float, SG, ACT>(z1, g1, a.merge_w);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) {
-                        acc[s][j][2 * i] = g0[s];
-                        acc[s][j][2 * i + 1] = g1[s];
-                    }
+                for (int s = 0; s < S; ++s) {
+                    const float4 q = zl[(2 * s + j) * THREADS];
+                    z[s][0] = q.x; z[s][1] = q.y; z[s][2] = q.z; z[s][3] = q.w;
                 }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float zc[S], gc[S];
+#pragma unroll
+                    for (int s = 0; s < S; ++s) {
+                        zc[s] = z[s][c];
+                        gc[s] = acc[s][j][c];
+                    }
+                    if (ACT == ACT_TANH)
+                        jet_apply_transposed_with<float, SG>(TanhD<float>(zc[0]), zc, gc, a.merge_w);
+                    else
+                        jet_apply_transposed<float, SG, ACT>(zc, gc, a.merge_w);
+#pragma unroll
+                    for (int s = 0; s < S; ++s) acc[s][j][c] = gc[s];
+                }
+            }
             {
                 float pb[4];
 #pragma unroll
@@ -530,7 +592,7 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
                     pb[2 * j] = acc[0][j][0] + acc[0][j][2];
                     pb[2 * j + 1] = acc[0][j][1] + acc[0][j][3];
                 }
-                reduce_units_over_points(pb, red + pg * W, lane, col0, t);
+                add_column_sums(pb, gbias + l * W, lane, col0, t);
             }
             if (l == 0) {
 #pragma unroll
@@ -546,119 +608,110 @@ __global__ void __launch_bounds__(128 * PG, 3 - PG) fused_mma_kernel(FusedArgs<f
                                 for (int dj = 0; dj < SG::ndirs; ++dj) v += a.dirs[dj * d0 + k] * acc[SG::base(dj)][j][c];
                                 pw[2 * j + (c & 1)] += v;
                             }
-                        reduce_units_over_points(pw, red + ((1 + k) * PG + pg) * W, lane, col0, t);
+                        add_column_sums(pw, gfirst + k * W, lane, col0, t);
                     }
                 }
-                __syncthreads();
-                for (int e = tid; e < (1 + d0) * W; e += THREADS) {
-                    const int which = e / W, n = e % W;
-                    const float total = PG == 2 ? red[(which * 2) * W + n] + red[(which * 2 + 1) * W + n] : red[which * W + n];
-                    if (which == 0) {
-                        if (a.b_off[0] >= 0) my_grad[a.b_off[0] + n] += total;
-                    } else {
-                        my_grad[a.w_off[0] + (which - 1) * W + n] += total;
-                    }
-                }
-                __syncthreads();
                 break;
             }
-            QB_PHASE(4);  // transposed jets (reload of z, tanh, bias partials)
-            // Stage: cotangents as the dgrad A operand / wgrad B operand, the previous layer's
-            // jets for the weight gradient, the transposed split weights for dgrad.
-#pragma unroll
-            for (int s = 0; s < S; ++s)
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        st2(act + (s * TP + row0 + g + 8 * i) * LDA + col0 + j * 8 + 2 * t, acc[s][j][2 * i],
-                            acc[s][j][2 * i + 1]);
-#pragma unroll
-            for (int s = 0; s < S; ++s)
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) zt[unit_of(j, c) * LDT + s * TP + row0 + g + 8 * (c >> 1)] = acc[s][j][c];
-            cp_async_wait_all();
+            QB_PHASE(4);  // transposed jets, bias partials
+            // Cotangents of the pre-activations: operand of both contractions below.
+            store_blocks<S, NW, LD, PLANE>(acc, act, scl_z, warp, g, t);
+            mbar_wait(hbar, hphase, a.error);
+            hphase ^= 1;
             __syncthreads();
             QB_PHASE(5);  // backward staging
-            if (tid < W && a.b_off[l] >= 0) my_grad[a.b_off[l] + tid] += PG == 2 ? red[tid] + red[W + tid] : red[tid];
-            // Weight gradient: dW[k][n] += sum_rows H[row][k] * Zhat[row][n]; warp: 16 k x 64/PG n,
-            // the cotangents read from their transposed copy.
+            // Weight gradient: dW[k][n] += sum_rows H[row][k] * Zhat[row][n]; this warp: its 16 k x all n.
             {
-                constexpr int NJJ = 4 / PG;  // 16-column groups of this warp's (64 / PG) columns
-                const int k0 = (warp / PG) * 16, n0 = (warp % PG) * (W / PG);
-                float* gw = my_grad + a.w_off[l];
-                // Starts from the running per-CTA sums, loaded before the loop so that the latency of
-                // the read-modify-write hides behind the contraction.
-                float dw[2 * NJJ][4];
+                float4* gw = dws + (size_t)(l - 1) * 2 * NW * THREADS + tid;
+                // Starts from the running sums, loaded before the loop so that their latency hides behind the contraction.
+                float dw[NW][2][4];
 #pragma unroll
-                for (int j = 0; j < 2 * NJJ; ++j)
+                for (int nb = 0; nb < NW; ++nb)
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        ld2(gw + (k0 + g + 8 * i) * W + n0 + j * 8 + 2 * t, dw[j][2 * i], dw[j][2 * i + 1]);
+                    for (int j = 0; j < 2; ++j) {
+                        const float4 q = gw[(2 * nb + j) * THREADS];
+                        dw[nb][j][0] = q.x; dw[nb][j][1] = q.y; dw[nb][j][2] = q.z; dw[nb][j][3] = q.w;
+                    }
                 const int mi = lane >> 3, rr = lane & 7;
-                const float* b_lane = zt + (n0 + (mi >> 1) * 8 + rr) * LDT + (mi & 1) * 4;
-#pragma unroll 2
-                for (int kb = 0; kb < ROWS / 8; ++kb) {
-                    // A(m = unit, k = row) from the row-major jets: element (g, t) = H[kb*8 + t][k0 + g].
-                    const float* ha = ht + (kb * 8 + t) * LDH + k0 + g;
+                const __half* a_lane = ht + ((mi >> 1) * 8 + rr) * LD + col0 + (mi & 1) * 8;
+                const __half* b_lane = act + ((mi & 1) * 8 + rr) * LD + (mi >> 1) * 8;
+                const float* scl_h = scl + (l - 1) * S * NW;
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
                     uint32_t ahi[4], alo[4];
-                    split_tf32(ha[0], ahi[0], alo[0]);
-                    split_tf32(ha[8], ahi[1], alo[1]);
-                    split_tf32(ha[4 * LDH], ahi[2], alo[2]);
-                    split_tf32(ha[4 * LDH + 8], ahi[3], alo[3]);
+                    ldmatrix_x4<true>(ahi, a_lane + s * 16 * LD);
+                    ldmatrix_x4<true>(alo, a_lane + s * 16 * LD + PLANE);
+                    const float fh = scl_h[s * NW + warp];
 #pragma unroll
-                    for (int jj = 0; jj < NJJ; ++jj) {
-                        uint32_t braw[4], bhi[4], blo[4];
-                        ldmatrix_x4(braw, b_lane + jj * 16 * LDT + kb * 8);
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) split_tf32(__uint_as_float(braw[q]), bhi[q], blo[q]);
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                            mma_tf32(part, alo, bhi[2 * h], bhi[2 * h + 1]);
-                            mma_tf32(part, ahi, blo[2 * h], blo[2 * h + 1]);
-                            mma_tf32(part, ahi, bhi[2 * h], bhi[2 * h + 1]);
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) dw[2 * jj + h][c] += part[c];
-                        }
+                    for (int nb = 0; nb < NW; ++nb) {
+                        uint32_t bhi[4], blo[4];
+                        ldmatrix_x4<true>(bhi, b_lane + s * 16 * LD + nb * 16);
+                        ldmatrix_x4<true>(blo, b_lane + s * 16 * LD + nb * 16 + PLANE);
+                        mma_step(dw[nb], ahi, alo, bhi, blo, fh * scl_z[s * NW + nb]);
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < 2 * NJJ; ++j)
+                for (int nb = 0; nb < NW; ++nb)
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        st2(gw + (k0 + g + 8 * i) * W + n0 + j * 8 + 2 * t, dw[j][2 * i], dw[j][2 * i + 1]);
+                    for (int j = 0; j < 2; ++j)
+                        gw[(2 * nb + j) * THREADS] = make_float4(dw[nb][j][0], dw[nb][j][1], dw[nb][j][2], dw[nb][j][3]);
             }
             QB_PHASE(6);  // weight gradient
             // Cotangents of layer l-1's jets: G = Zhat W^T.
-            {
-                const uint32_t* whi = wbuf + (use % NBUF) * 2 * WIMG_PLANE;
-                mbar_wait(bars + (use % NBUF), (uint32_t)((use / NBUF) & 1), a.error);
-                warp_gemm_3xtf32<S, TP, LDA>(act, whi, whi + WIMG_PLANE, row0, col0, lane, acc);
-            }
+            mbar_wait(wbar, wphase, a.error);
+            wphase ^= 1;
+            warp_contract<S, NW, LD, PLANE, WPLANE, false>(act, wbuf, scl_z, wscl[l - 1], warp, lane, acc);
             __syncthreads();
-            issue(use + NBUF);
-            ++use;
-            QB_PHASE(7);  // dgrad
+            if (tid == 0) {
+                load_weights();
+                if (l > 1) load_jets(l - 2);
+            }
+            QB_PHASE(7);  // data gradient
         }
     }
 #ifdef QB_PHASE_TIMING
     if (tid == 0 && blockIdx.x == 0) {
-        printf("phases S=%d:", S);
-        for (int i = 0; i < 8; ++i) printf(" %lld", phase_[i]);
+        printf("phases S=%d W=%d tiles=%d:", S, W, my_tiles);
+        for (int i = 0; i < 8; ++i) printf(" %lld", phase_[i] / max(my_tiles, 1));
         printf("\n");
     }
 #endif
 
-    double* lred = reinterpret_cast<double*>(ht);
+    // Per-CTA gradients in parameter order, and the loss partial, in a fixed order.
     __syncthreads();
-    if (tid < TP) lred[tid] = loss_sum;
+    if (backward) {
+        float* my_grad = a.grad_cta + (size_t)blockIdx.x * a.P;
+        for (int i = tid; i < L * W; i += THREADS) {
+            const int l = i / W, n = i % W;
+            if (a.b_off[l] >= 0 && n < a.width[l]) my_grad[a.b_off[l] + n] = gbias[i];
+        }
+        for (int i = tid; i < d0 * W; i += THREADS) {
+            const int k = i / W, n = i % W;
+            if (n < a.width[0]) my_grad[a.w_off[0] + k * a.width[0] + n] = gfirst[i];
+        }
+        for (int i = tid; i < a.width[L - 1]; i += THREADS) my_grad[a.w_off[L] + i] = ghead[i];
+        if (tid == 0 && a.b_off[L] >= 0) my_grad[a.b_off[L]] = head_bias_grad;
+        for (int l = 1; l < L; ++l) {
+            const int rows = a.width[l - 1], cols = a.width[l];
+            float* out = my_grad + a.w_off[l];
+            for (int q = 0; q < 2 * NW; ++q) {
+                const float4 v = dws[((size_t)(l - 1) * 2 * NW + q) * THREADS + tid];
+                const int k = col0 + g, n = (q >> 1) * 16 + (q & 1) * 8 + 2 * t;
+                if (k < rows && n < cols) out[k * cols + n] = v.x;
+                if (k < rows && n + 1 < cols) out[k * cols + n + 1] = v.y;
+                if (k + 8 < rows && n < cols) out[(k + 8) * cols + n] = v.z;
+                if (k + 8 < rows && n + 1 < cols) out[(k + 8) * cols + n + 1] = v.w;
+            }
+        }
+    }
+    double* lred = reinterpret_cast<double*>(red);
+    static_assert(4 * NW * G::ROWS >= 8 * TP || S == 1, "loss partials fit the reduction area");
+    double* lsum = S == 1 ? reinterpret_cast<double*>(act) : lred;
+    if (tid < TP) lsum[tid] = loss_sum;
     __syncthreads();
     if (tid == 0) {
         double total = 0.0;
-        for (int p = 0; p < TP; ++p) total += lred[p];
+        for (int p = 0; p < TP; ++p) total += lsum[p];
         a.loss_cta[blockIdx.x] = total;
     }
 }

@@ -363,6 +363,10 @@ class Plan final : public qb200_plan {
     int fused_width_ = 0;
     std::vector<FusedEntry<T>> fused_entries_;  // per set
     std::vector<int> fused_grid_;               // per set
+    std::vector<size_t> fused_smem_;            // per set: dynamic shared memory of its launch
+    std::vector<size_t> fused_dw_, fused_dw0_;  // per set: elements of running weight-gradient sums kept in global memory
+    float* fused_dw_scratch_ = nullptr;
+    float* fused_scales_ = nullptr;             // of the weight images
     // Every set has its own saved-jet scratch and gradient rows, so that the small sets run beside
     // the first one on a second stream; rows of all sets are consecutive for the final reduction.
     std::vector<size_t> fused_jet0_, fused_row0_;  // per set: first scratch element, first gradient row
@@ -418,6 +422,7 @@ static int slice_rows(long long rows, int tiles, int granule) {
     chunk = std::max<long long>(256, (chunk + granule - 1) / granule * granule);
     return (int)std::min<long long>(chunk, K_CHUNK_ROWS);
 }
+constexpr long long PADDED_MIN_POINTS = 1024;  // see choose_fused()
 constexpr int BIAS_SLICES = 512;  // upper bound on the row slices of one bias-gradient column sum
 
 template <typename T>
@@ -676,6 +681,12 @@ qb200_status Plan<T>::init() {
             rows += (size_t)fused_grid_[si];
         }
         fused_rows_ = rows;
+        size_t dw = 0;
+        for (size_t count : fused_dw_) {
+            fused_dw0_.push_back(dw);
+            dw += count;
+        }
+        QB_TRY(dev_alloc(&fused_dw_scratch_, dw));
         if (sets_.size() > 1) {
             int least = 0, greatest = 0;
             QB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -686,12 +697,14 @@ qb200_status Plan<T>::init() {
         QB_TRY(dev_alloc(&fused_z_, jets));
         QB_TRY(dev_alloc(&fused_h_, jets));
         QB_TRY(dev_alloc(&fused_grad_, rows * n_params_));
+        QB_CUDA(cudaMemsetAsync(fused_grad_, 0, rows * n_params_ * sizeof(T), stream_));
         scratch_bytes_ = (2 * jets + rows * n_params_) * sizeof(T);
         for (const auto& e : fused_entries_) fused_tensor_core_ = fused_tensor_core_ || e.tensor_core;
         if (fused_tensor_core_) {
             unsigned char* raw = nullptr;
-            QB_TRY(dev_alloc(&raw, fused_weight_image_bytes(hidden - 1)));
+            QB_TRY(dev_alloc(&raw, fused_weight_image_bytes(hidden - 1, fused_entries_[0].width)));
             fused_images_ = raw;
+            QB_TRY(dev_alloc(&fused_scales_, (size_t)hidden));
         }
         return QB200_OK;
     }
@@ -959,13 +972,20 @@ bool Plan<T>::choose_fused() {
     if (desc_.activation != QB200_ACT_TANH && desc_.activation != QB200_ACT_SIN) return false;
     const int hidden = L_ - 1;
     if (hidden < 1 || hidden > FUSED_MAX_LAYERS || desc_.sizes[0] > 4) return false;
-    const int W = desc_.sizes[1];
-    for (int l = 1; l <= hidden; ++l)
-        if (desc_.sizes[l] != W) return false;
+    int width = 0;
+    bool uniform = true;
+    for (int l = 1; l <= hidden; ++l) {
+        width = std::max(width, desc_.sizes[l]);
+        uniform = uniform && desc_.sizes[l] == desc_.sizes[1];
+    }
+    long long points = 0;
+    for (const auto& s : desc_.sets) points += s.n;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_);
     fused_entries_.resize(desc_.sets.size());
     fused_grid_.resize(desc_.sets.size());
+    fused_smem_.resize(desc_.sets.size());
+    fused_dw_.assign(desc_.sets.size(), 0);
     for (size_t si = 0; si < desc_.sets.size(); ++si) {
         const auto& s = desc_.sets[si];
         int code = 0, scale = 1;
@@ -974,12 +994,28 @@ bool Plan<T>::choose_fused() {
             scale *= 5;
         }
         if (!s.merge_w.empty()) code += SIG_MERGED;
-        if (!fused_lookup<T>(W, code, desc_.activation, &fused_entries_[si])) return false;
-        if (fused_smem_bytes(fused_entries_[si], (int)s.code.size() / 4) > FUSED_MAX_SMEM) return false;
-        const long long tiles = (s.n + fused_entries_[si].tile_points - 1) / fused_entries_[si].tile_points;
-        fused_grid_[si] = (int)std::min<long long>(tiles, (long long)sms * fused_entries_[si].ctas_per_sm);
+        FusedEntry<T>& entry = fused_entries_[si];
+        if (!fused_lookup<T>(width, uniform, hidden, code, desc_.activation, &entry)) return false;
+        // Padded networks (widths other than 16, 32 and 64): from PADDED_MIN_POINTS points on, where the idle units
+        // cost less than the layer-wise engine's launches per layer and point set.
+        const bool padded = entry.tensor_core && (!uniform || (width != 16 && width != 32 && width != 64));
+        if (padded && points < PADDED_MIN_POINTS) return false;
+        size_t smem = fused_smem_bytes(entry, (int)s.code.size() / 4);
+        if (smem > FUSED_MAX_SMEM) return false;
+        const long long tiles = (s.n + entry.tile_points - 1) / entry.tile_points;
+        const long long fit = std::min<long long>(entry.ctas_per_sm, std::max<long long>(1, FUSED_SM_SMEM / (smem + FUSED_CTA_SMEM)));
+        fused_grid_[si] = (int)std::min<long long>(tiles, (long long)sms * fit);
+        if (entry.tensor_core) {
+            // The running weight-gradient sums stay in shared memory where that costs no co-resident CTA.
+            const size_t dw = (size_t)(hidden - 1) * entry.dw_bytes, per_sm = (size_t)(fused_grid_[si] + sms - 1) / sms;
+            if (smem + dw <= FUSED_MAX_SMEM && (smem + dw + FUSED_CTA_SMEM) * per_sm <= FUSED_SM_SMEM)
+                smem += dw;
+            else
+                fused_dw_[si] = dw / sizeof(float) * (size_t)fused_grid_[si];
+        }
+        fused_smem_[si] = smem;
     }
-    fused_width_ = W;
+    fused_width_ = width;
     return true;
 }
 
@@ -994,7 +1030,8 @@ qb200_status Plan<float>::prepare_weight_images() {
     if (hidden_to_hidden < 1) return QB200_OK;
     int w_off[FUSED_MAX_LAYERS + 1];
     for (int i = 0; i < hidden_to_hidden; ++i) w_off[i] = (int)leaves_[w_leaf_[1 + i]].offset;
-    cudaError_t e = fused_prep_launch(d_params_, w_off, hidden_to_hidden, fused_images_, stream_);
+    cudaError_t e = fused_prep_launch(d_params_, w_off, &desc_.sizes[1], &desc_.sizes[2], hidden_to_hidden, fused_entries_[0].width,
+                                      fused_images_, fused_scales_, stream_);
     ++launches_;
     if (e != cudaSuccess) return fail(QB200_CUDA_ERROR, "launch of prep_weights_kernel failed: %s", cudaGetErrorString(e));
     return QB200_OK;
@@ -1031,6 +1068,7 @@ qb200_status Plan<T>::run_fused(int si, bool forward_only) {
     for (int l = 0; l <= FUSED_MAX_LAYERS; ++l) {
         a.w_off[l] = l < L_ ? (int)leaves_[w_leaf_[l]].offset : 0;
         a.b_off[l] = (l < L_ && b_leaf_[l] >= 0) ? (int)leaves_[b_leaf_[l]].offset : -1;
+        a.width[l] = l < L_ ? desc_.sizes[l + 1] : 0;
     }
     a.table = st.table;
     a.ncols = st.ncols;
@@ -1049,10 +1087,12 @@ qb200_status Plan<T>::run_fused(int si, bool forward_only) {
     a.loss_cta = d_partials_ + st.partial_offset;
     a.forward_only = forward_only ? 1 : 0;
     a.weight_images = fused_images_;
+    a.image_scales = fused_scales_;
+    a.dw_scratch = fused_dw_[si] > 0 ? fused_dw_scratch_ + fused_dw0_[si] : nullptr;
     a.error = d_error_;
     // Sets after the first run on the side stream, between the fork and join events of run().
     cudaStream_t stream = (si > 0 && side_stream_ != nullptr) ? side_stream_ : stream_;
-    cudaError_t e = fused_launch<T>(fused_entries_[si], fused_grid_[si], stream, a);
+    cudaError_t e = fused_launch<T>(fused_entries_[si], fused_grid_[si], fused_smem_[si], stream, a);
     ++launches_;
     if (e != cudaSuccess) return fail(QB200_CUDA_ERROR, "launch of fused_step_kernel failed: %s", cudaGetErrorString(e));
     return QB200_OK;
@@ -1781,7 +1821,7 @@ qb200_status Plan<T>::query(int key, int64_t* out) {
         case QB200_Q_FLAT_DEVICE_PTR: *out = (int64_t)(intptr_t)d_flat_; return QB200_OK;
         case QB200_Q_SCRATCH_BYTES: *out = (int64_t)scratch_bytes_; return QB200_OK;
         case QB200_Q_STEP_COUNT: *out = steps_; return QB200_OK;
-        case QB200_Q_ENGINE: *out = fused_ ? (fused_tensor_core_ ? 2 : 1) : (tc_any_ ? 3 : 0); return QB200_OK;
+        case QB200_Q_ENGINE: *out = fused_ ? (fused_tensor_core_ && fused_width_ > 32 ? 2 : 1) : (tc_any_ ? 3 : 0); return QB200_OK;
         case QB200_Q_ALLREDUCE_NANOSECONDS: {
             if (!ev_ar_valid_) {
                 *out = 0;  // no communicator attached, or no execute yet

@@ -30,7 +30,7 @@
 
 #include <cstdint>
 
-#include "fused_mma_kernel.cuh"  // split_tf32, mbarrier helpers
+#include "fused_mma_kernel.cuh"  // mbarrier helpers
 #include "tc_gemm.cuh"           // tc_commit, tile constants
 
 namespace qb {

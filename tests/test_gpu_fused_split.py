@@ -1,0 +1,91 @@
+"""The split-operand fused kernels against the CPU oracle at the edges of what they take: every padded width, unequal
+widths, one to many hidden layers (running weight-gradient sums in shared and in global memory), ragged point counts,
+every derivative signature, and operands whose blocks differ by many orders of magnitude."""
+
+import math
+
+import numpy as np
+import pytest
+
+import quabla_b200 as qb
+from oracle import contracted
+from quabla_b200 import _lib, workloads
+from quabla_b200._plan import Plan
+from quabla_b200._transforms import CompiledLoss
+
+from _util import TOLERANCE, relative_error
+
+pytestmark = pytest.mark.gpu
+
+
+def _residual(kind):
+    def residual(f, q):
+        if kind == "value":
+            return f(q) - qb.sin(q[0])
+        g = qb.grad(f)
+        if kind == "first":
+            return g(q)[0] + f(q)
+        if kind == "second":
+            return qb.hessian(f)(q)[0, 0] - f(q)
+        if kind == "laplacian":
+            h = qb.hessian(f)(q)
+            total = h[0, 0]
+            for i in range(1, q.shape[0]):
+                total = total + (i + 1.0) * h[i, i]
+            return total + f(q) * g(q)[0]
+        if kind == "burgers":
+            return g(q)[1] + f(q) * g(q)[0] - 0.1 * qb.hessian(f)(q)[0, 0]
+        raise ValueError(kind)
+
+    return residual
+
+
+def _check(sizes, points, kind, activation="tanh", scale=1.0):
+    u = workloads.make_u(qb, activation)
+    params = workloads.init_mlp(qb.random.key(11), sizes, np.float32)
+    for i, layer in enumerate(params):
+        layer["b"] = qb.random.uniform(qb.random.key(50 + i), layer["b"].shape, np.float32, -0.5, 0.5)
+    if scale != 1.0:  # input directions on very different scales: streams of very different size
+        params[0]["w"] = params[0]["w"] * np.float32(scale)
+    p = np.stack([qb.random.uniform(qb.random.fold_in(qb.random.key(5), j), (points,), np.float32, -1.0, 1.0)
+                  for j in range(sizes[0])], axis=1)
+
+    def loss(params, p):
+        return qb.mean(qb.vmap(lambda q: _residual(kind)(lambda s: u(params, s), q))(p) ** 2)
+
+    args = (params, p)
+    compiled = CompiledLoss(loss, args, (0,), 0)
+    assert compiled.plan.query(_lib.Q_ENGINE) in (1, 2)
+    spec = compiled.spec.unmerged or compiled.spec
+    value, grads = contracted.value_and_grad(spec, compiled.named_inputs(args), threads=contracted.max_threads())
+    compiled.bind(args)
+    compiled.plan.execute()
+    got = compiled.plan.outputs()
+    tol = TOLERANCE[np.dtype(np.float32)]
+    assert relative_error(got[0], value) <= tol
+    for (name, _, _), g, expected in zip(compiled.spec.parameters, got[1:], grads):
+        assert relative_error(g.reshape(expected.shape), expected) <= tol, name
+
+
+@pytest.mark.parametrize("sizes,points", [
+    ([1, 16, 1], 1), ([2, 16, 16, 1], 17), ([2, 32, 32, 32, 1], 255), ([2, 64, 64, 1], 15),
+    ([2, 3, 5, 1], 1024), ([3, 17, 17, 17, 1], 1025), ([4, 48, 48, 48, 1], 1031), ([2, 33, 64, 20, 1], 1100),
+    ([2, 63, 50, 1], 1999), ([1] + [64] * 12 + [1], 1050), ([2] + [16] * 12 + [1], 5000), ([2, 64, 64, 64, 64, 1], 9001),
+], ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else str(v))
+def test_widths_depths_and_point_counts(cuda_device, sizes, points):
+    _check(sizes, points, "second")
+
+
+@pytest.mark.parametrize("activation", ["tanh", "sin"])
+@pytest.mark.parametrize("width,kind,inputs", [
+    (64, "value", 2), (64, "first", 2), (64, "burgers", 2), (64, "laplacian", 2), (64, "laplacian", 3), (64, "laplacian", 4),
+    (50, "laplacian", 4), (48, "burgers", 2), (32, "laplacian", 3), (16, "laplacian", 4)])
+def test_signatures(cuda_device, activation, width, kind, inputs):
+    _check([inputs, width, width, width, 1], 1037, kind, activation)
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -40, 2.0 ** -12, 16.0])
+def test_streams_of_very_different_size(cuda_device, scale):
+    # Derivative streams grow with the scale of the first weights, to the first and second power: block scales keep
+    # each stream's relative accuracy (a plain float16 operand would be subnormal or infinite here).
+    _check([2, 64, 64, 1], 1040, "burgers", "sin", scale=scale)
