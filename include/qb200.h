@@ -90,8 +90,8 @@ typedef enum qb200_query {
     QB200_Q_FLAT_DEVICE_PTR = 6,     /* device address of the flat [loss, gradients...] buffer */
     QB200_Q_SCRATCH_BYTES = 7,       /* bytes of saved-jet scratch the plan holds */
     QB200_Q_STEP_COUNT = 8,          /* optimizer updates applied so far */
-    QB200_Q_ENGINE = 9,              /* 0: layer-wise (FP pipe), 1: fused, widths up to 32 or on the FP32/FP64 pipe, 2: fused, tensor cores, widths
-                                        above 32, 3: layer-wise with tcgen05 GEMMs */
+    QB200_Q_ENGINE = 9,              /* 0: layer-wise (FP pipe), 1: fused, float64 or widths up to 32, 2: fused, float32, widths above 32,
+                                        3: layer-wise with tcgen05 GEMMs */
     QB200_Q_SET0_NANOSECONDS = 10,   /* device time of the last execute's kernels for point set 0 (events) */
     QB200_Q_ALLREDUCE_NANOSECONDS = 11, /* device time of the last execute's gradient all-reduce, waits for peers included */
     QB200_Q_GEMM_NANOSECONDS = 12,   /* with QB200_OPT_KERNEL_TIMERS: summed device time of the last execute's layer GEMM launches

@@ -16,7 +16,8 @@ CSRC = os.path.join(_HERE, "csrc")
 # QB200_LIBRARY points the binding at another build of the same sources (A/B comparisons on one GPU box).
 LIBRARY = os.environ.get("QB200_LIBRARY") or os.path.join(_HERE, "libqb200.so")
 SOURCES = ["api.cu", "plan.cu", "host_staging.cu", "static_scratch.cu", "fused.cu", "fused_mma_w16.cu",
-           "fused_mma_w32.cu", "fused_mma_w48.cu", "fused_mma_w64.cu", "tc_gemm.cu"]
+           "fused_mma_w32.cu", "fused_mma_w48.cu", "fused_mma_w64.cu", "fused_dmma_w16.cu", "fused_dmma_w32.cu",
+           "fused_dmma_w48.cu", "fused_dmma_w64.cu", "tc_gemm.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -6,6 +6,7 @@
 #include <cstring>
 
 #include "fused_kernel.cuh"
+#include "fused_dmma_kernel.cuh"
 #include "fused_mma_kernel.cuh"
 
 namespace qb {
@@ -41,38 +42,37 @@ bool want_simt() {
 // Signature codes: 0 = value only; 1 = {1}; 2 = {2}; 3 = {3}; 4 = {4}; 6 = {1,1};
 // 7 = {2,1}; 11 = {1,2}; 12 = {2,2}; SIG_MERGED + 6 / 31 = {1,1} / {1,1,1} plus the merged
 // second-order stream (2-D / 3-D Laplacian).
-#define QB_CASE(T, W, CODE)                                                                            \
-    if (width == W && code == CODE) {                                                                  \
-        if (act == ACT_SIN && sizeof(T) == 4) return false; /* the comparison variant carries tanh only */ \
-        *out = act == ACT_TANH ? make_entry<T, W, CODE, ACT_TANH>()                                    \
-                               : make_entry<T, W, CODE, sizeof(T) == 4 ? ACT_TANH : ACT_SIN>();        \
-        return true;                                                                                   \
+#define QB_CASE(T, W, CODE)                       \
+    if (width == W && code == CODE) {             \
+        *out = make_entry<T, W, CODE, ACT_TANH>(); \
+        return true;                              \
     }
+
+template <typename T>
+static bool padded_lookup(int width, int layers, int code, int act, FusedEntry<T>* out) {
+    if (width <= 16) return fused_mma_lookup<T, 16>(layers, code, act, out);
+    if (width <= 32) return fused_mma_lookup<T, 32>(layers, code, act, out);
+    if (width <= 48) return fused_mma_lookup<T, 48>(layers, code, act, out);
+    if (width <= 64) return fused_mma_lookup<T, 64>(layers, code, act, out);
+    return false;
+}
 
 template <>
 bool fused_lookup<float>(int width, bool uniform, int layers, int code, int act, FusedEntry<float>* out) {
     if (act != ACT_TANH && act != ACT_SIN) return false;
     if (want_simt()) {
-        if (!uniform) return false;
+        if (!uniform || act != ACT_TANH) return false;
         QB_CASE(float, 64, 0) QB_CASE(float, 64, 1) QB_CASE(float, 64, 2) QB_CASE(float, 64, 4)
         QB_CASE(float, 64, 7) QB_CASE(float, 64, 12) QB_CASE(float, 64, SIG_MERGED + 6)
         return false;
     }
-    if (width <= 16) return fused_mma_lookup<16>(layers, code, act, out);
-    if (width <= 32) return fused_mma_lookup<32>(layers, code, act, out);
-    if (width <= 48) return fused_mma_lookup<48>(layers, code, act, out);
-    if (width <= 64) return fused_mma_lookup<64>(layers, code, act, out);
-    return false;
+    return padded_lookup<float>(width, layers, code, act, out);
 }
 
 template <>
-bool fused_lookup<double>(int width, bool uniform, int layers, int code, int act, FusedEntry<double>* out) {
-    (void)layers;
-    if (!uniform || (act != ACT_TANH && act != ACT_SIN)) return false;
-    QB_CASE(double, 16, 0) QB_CASE(double, 16, 1) QB_CASE(double, 16, 2) QB_CASE(double, 16, 7)
-    QB_CASE(double, 16, 12) QB_CASE(double, 16, SIG_MERGED + 6)
-    QB_CASE(double, 32, 0) QB_CASE(double, 32, 1) QB_CASE(double, 32, 2)
-    return false;
+bool fused_lookup<double>(int width, bool, int layers, int code, int act, FusedEntry<double>* out) {
+    if (act != ACT_TANH && act != ACT_SIN) return false;
+    return padded_lookup<double>(width, layers, code, act, out);
 }
 
 template <typename T>
@@ -90,21 +90,40 @@ cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, size_t smem, cuda
     return cudaGetLastError();
 }
 
-size_t fused_weight_image_bytes(int hidden_to_hidden, int width) {
+template <>
+size_t fused_weight_image_bytes<float>(int hidden_to_hidden, int width) {
     return (size_t)std::max(hidden_to_hidden, 1) * 4 * width * (width + 8);
 }
+template <>
+size_t fused_weight_image_bytes<double>(int hidden_to_hidden, int width) {
+    return (size_t)std::max(hidden_to_hidden, 1) * 8 * width * (width + 4);
+}
 
-cudaError_t fused_prep_launch(const float* params, const int* w_off, const int* rows, const int* cols, int hidden_to_hidden,
-                              int width, void* images, float* scales, cudaStream_t stream) {
-    if (hidden_to_hidden < 1) return cudaSuccess;
+static PrepArgs prep_args(const int* w_off, const int* rows, const int* cols, int layers) {
     PrepArgs p;
-    p.layers = hidden_to_hidden;
+    p.layers = layers;
     for (int i = 0; i <= FUSED_MAX_LAYERS; ++i) {
-        p.w_off[i] = i < hidden_to_hidden ? w_off[i] : 0;
-        p.rows[i] = i < hidden_to_hidden ? rows[i] : 0;
-        p.cols[i] = i < hidden_to_hidden ? cols[i] : 0;
+        p.w_off[i] = i < layers ? w_off[i] : 0;
+        p.rows[i] = i < layers ? rows[i] : 0;
+        p.cols[i] = i < layers ? cols[i] : 0;
     }
-    prep_weights_kernel<<<hidden_to_hidden, 1024, 0, stream>>>(params, p, width, static_cast<uint32_t*>(images), scales);
+    return p;
+}
+
+template <>
+cudaError_t fused_prep_launch<float>(const float* params, const int* w_off, const int* rows, const int* cols,
+                                     int hidden_to_hidden, int width, void* images, float* scales, cudaStream_t stream) {
+    if (hidden_to_hidden < 1) return cudaSuccess;
+    prep_weights_kernel<<<hidden_to_hidden, 1024, 0, stream>>>(params, prep_args(w_off, rows, cols, hidden_to_hidden), width,
+                                                               static_cast<uint32_t*>(images), scales);
+    return cudaGetLastError();
+}
+template <>
+cudaError_t fused_prep_launch<double>(const double* params, const int* w_off, const int* rows, const int* cols,
+                                      int hidden_to_hidden, int width, void* images, float*, cudaStream_t stream) {
+    if (hidden_to_hidden < 1) return cudaSuccess;
+    prep_weights64_kernel<<<dim3(4, hidden_to_hidden), 256, 0, stream>>>(
+        params, prep_args(w_off, rows, cols, hidden_to_hidden), width, static_cast<double*>(images));
     return cudaGetLastError();
 }
 

@@ -10,7 +10,7 @@
 // 1792-2972: one kernel per IR node; op/vjp.rs:176-209: a materialised
 // [B, in, out] product per weight gradient).
 //
-// Shapes: every hidden layer has the same width W (16, 32 or 64), the input
+// Shapes: every hidden layer has the same width W, the input
 // width d0 <= 4, the output width 1.  A CTA of 256 threads owns a tile of TP
 // points; thread (tp, tn) holds, for 2 points x 4 units, ALL S streams in
 // registers, so the tanh-jet composition and its transpose are register-only.
@@ -93,7 +93,7 @@ struct FusedArgs {
     int forward_only;
     const void* weight_images;  // tensor-core variant: pre-split weight images (prep_weights_kernel)
     const float* image_scales;  // and their scales
-    float* dw_scratch;          // tensor-core variant: running weight-gradient sums, or null: in shared memory
+    T* dw_scratch;              // tensor-core variant: running weight-gradient sums, or null: in shared memory
     int* error;                 // set to 1 when a bounded wait inside the kernel gave up
 };
 

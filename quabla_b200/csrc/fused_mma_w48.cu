@@ -1,6 +1,6 @@
-// Split-operand fused kernels for hidden widths up to 48.
+// Float32 fused kernels for hidden widths up to 48.
 #include "fused_mma_entries.cuh"
 
 namespace qb {
-QB_MMA_LOOKUP(48)
+QB_MMA_LOOKUP(float, 48, MmaGeom, fused_mma_kernel)
 }  // namespace qb

@@ -365,7 +365,7 @@ class Plan final : public qb200_plan {
     std::vector<int> fused_grid_;               // per set
     std::vector<size_t> fused_smem_;            // per set: dynamic shared memory of its launch
     std::vector<size_t> fused_dw_, fused_dw0_;  // per set: elements of running weight-gradient sums kept in global memory
-    float* fused_dw_scratch_ = nullptr;
+    T* fused_dw_scratch_ = nullptr;
     float* fused_scales_ = nullptr;             // of the weight images
     // Every set has its own saved-jet scratch and gradient rows, so that the small sets run beside
     // the first one on a second stream; rows of all sets are consecutive for the final reduction.
@@ -702,7 +702,7 @@ qb200_status Plan<T>::init() {
         for (const auto& e : fused_entries_) fused_tensor_core_ = fused_tensor_core_ || e.tensor_core;
         if (fused_tensor_core_) {
             unsigned char* raw = nullptr;
-            QB_TRY(dev_alloc(&raw, fused_weight_image_bytes(hidden - 1, fused_entries_[0].width)));
+            QB_TRY(dev_alloc(&raw, fused_weight_image_bytes<T>(hidden - 1, fused_entries_[0].width)));
             fused_images_ = raw;
             QB_TRY(dev_alloc(&fused_scales_, (size_t)hidden));
         }
@@ -996,10 +996,12 @@ bool Plan<T>::choose_fused() {
         if (!s.merge_w.empty()) code += SIG_MERGED;
         FusedEntry<T>& entry = fused_entries_[si];
         if (!fused_lookup<T>(width, uniform, hidden, code, desc_.activation, &entry)) return false;
-        // Padded networks (widths other than 16, 32 and 64): from PADDED_MIN_POINTS points on, where the idle units
-        // cost less than the layer-wise engine's launches per layer and point set.
-        const bool padded = entry.tensor_core && (!uniform || (width != 16 && width != 32 && width != 64));
-        if (padded && points < PADDED_MIN_POINTS) return false;
+        // The layer-wise engine costs some nine launches per layer and point set, the fused one a launch per set: for
+        // every width and signature it is ahead from four layers (over all sets) or PADDED_MIN_POINTS points on.
+        // Below that only the widths 16, 32 and 64 that fill their kernels take it.
+        const bool fills = uniform && (sizeof(T) == 4 ? width == 16 || width == 32 || width == 64
+                                                      : (width == 16 || width == 32) && s.merge_w.empty());
+        if (entry.tensor_core && !fills && hidden * (int)desc_.sets.size() < 4 && points < PADDED_MIN_POINTS) return false;
         size_t smem = fused_smem_bytes(entry, (int)s.code.size() / 4);
         if (smem > FUSED_MAX_SMEM) return false;
         const long long tiles = (s.n + entry.tile_points - 1) / entry.tile_points;
@@ -1011,7 +1013,7 @@ bool Plan<T>::choose_fused() {
             if (smem + dw <= FUSED_MAX_SMEM && (smem + dw + FUSED_CTA_SMEM) * per_sm <= FUSED_SM_SMEM)
                 smem += dw;
             else
-                fused_dw_[si] = dw / sizeof(float) * (size_t)fused_grid_[si];
+                fused_dw_[si] = dw / sizeof(T) * (size_t)fused_grid_[si];
         }
         fused_smem_[si] = smem;
     }
@@ -1021,16 +1023,11 @@ bool Plan<T>::choose_fused() {
 
 template <typename T>
 qb200_status Plan<T>::prepare_weight_images() {
-    return fail(QB200_UNSUPPORTED, "the tensor-core fused engine is float32 only");
-}
-
-template <>
-qb200_status Plan<float>::prepare_weight_images() {
     const int hidden_to_hidden = L_ - 2;
     if (hidden_to_hidden < 1) return QB200_OK;
     int w_off[FUSED_MAX_LAYERS + 1];
     for (int i = 0; i < hidden_to_hidden; ++i) w_off[i] = (int)leaves_[w_leaf_[1 + i]].offset;
-    cudaError_t e = fused_prep_launch(d_params_, w_off, &desc_.sizes[1], &desc_.sizes[2], hidden_to_hidden, fused_entries_[0].width,
+    cudaError_t e = fused_prep_launch<T>(d_params_, w_off, &desc_.sizes[1], &desc_.sizes[2], hidden_to_hidden, fused_entries_[0].width,
                                       fused_images_, fused_scales_, stream_);
     ++launches_;
     if (e != cudaSuccess) return fail(QB200_CUDA_ERROR, "launch of prep_weights_kernel failed: %s", cudaGetErrorString(e));
@@ -1821,7 +1818,7 @@ qb200_status Plan<T>::query(int key, int64_t* out) {
         case QB200_Q_FLAT_DEVICE_PTR: *out = (int64_t)(intptr_t)d_flat_; return QB200_OK;
         case QB200_Q_SCRATCH_BYTES: *out = (int64_t)scratch_bytes_; return QB200_OK;
         case QB200_Q_STEP_COUNT: *out = steps_; return QB200_OK;
-        case QB200_Q_ENGINE: *out = fused_ ? (fused_tensor_core_ && fused_width_ > 32 ? 2 : 1) : (tc_any_ ? 3 : 0); return QB200_OK;
+        case QB200_Q_ENGINE: *out = fused_ ? (fused_tensor_core_ && sizeof(T) == 4 && fused_width_ > 32 ? 2 : 1) : (tc_any_ ? 3 : 0); return QB200_OK;
         case QB200_Q_ALLREDUCE_NANOSECONDS: {
             if (!ev_ar_valid_) {
                 *out = 0;  // no communicator attached, or no execute yet

@@ -1,4 +1,4 @@
-"""The split-operand fused kernels against the CPU oracle at the edges of what they take: every padded width, unequal
+"""The tensor-core fused kernels (split float32, FP64 MMA) against the CPU oracle at the edges of what they take: every padded width, unequal
 widths, one to many hidden layers (running weight-gradient sums in shared and in global memory), ragged point counts,
 every derivative signature, and operands whose blocks differ by many orders of magnitude."""
 
@@ -40,14 +40,14 @@ def _residual(kind):
     return residual
 
 
-def _check(sizes, points, kind, activation="tanh", scale=1.0):
+def _check(sizes, points, kind, activation="tanh", scale=1.0, dtype=np.float32):
     u = workloads.make_u(qb, activation)
-    params = workloads.init_mlp(qb.random.key(11), sizes, np.float32)
+    params = workloads.init_mlp(qb.random.key(11), sizes, dtype)
     for i, layer in enumerate(params):
-        layer["b"] = qb.random.uniform(qb.random.key(50 + i), layer["b"].shape, np.float32, -0.5, 0.5)
+        layer["b"] = qb.random.uniform(qb.random.key(50 + i), layer["b"].shape, dtype, -0.5, 0.5)
     if scale != 1.0:  # input directions on very different scales: streams of very different size
-        params[0]["w"] = params[0]["w"] * np.float32(scale)
-    p = np.stack([qb.random.uniform(qb.random.fold_in(qb.random.key(5), j), (points,), np.float32, -1.0, 1.0)
+        params[0]["w"] = params[0]["w"] * dtype(scale)
+    p = np.stack([qb.random.uniform(qb.random.fold_in(qb.random.key(5), j), (points,), dtype, -1.0, 1.0)
                   for j in range(sizes[0])], axis=1)
 
     def loss(params, p):
@@ -61,27 +61,29 @@ def _check(sizes, points, kind, activation="tanh", scale=1.0):
     compiled.bind(args)
     compiled.plan.execute()
     got = compiled.plan.outputs()
-    tol = TOLERANCE[np.dtype(np.float32)]
+    tol = TOLERANCE[np.dtype(dtype)]
     assert relative_error(got[0], value) <= tol
     for (name, _, _), g, expected in zip(compiled.spec.parameters, got[1:], grads):
         assert relative_error(g.reshape(expected.shape), expected) <= tol, name
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("sizes,points", [
-    ([1, 16, 1], 1), ([2, 16, 16, 1], 17), ([2, 32, 32, 32, 1], 255), ([2, 64, 64, 1], 15),
+    ([1, 16, 1], 1), ([2, 16, 16, 1], 17), ([2, 32, 32, 32, 1], 255), ([2, 64, 64, 64, 64, 1], 15),
     ([2, 3, 5, 1], 1024), ([3, 17, 17, 17, 1], 1025), ([4, 48, 48, 48, 1], 1031), ([2, 33, 64, 20, 1], 1100),
     ([2, 63, 50, 1], 1999), ([1] + [64] * 12 + [1], 1050), ([2] + [16] * 12 + [1], 5000), ([2, 64, 64, 64, 64, 1], 9001),
 ], ids=lambda v: "-".join(map(str, v)) if isinstance(v, list) else str(v))
-def test_widths_depths_and_point_counts(cuda_device, sizes, points):
-    _check(sizes, points, "second")
+def test_widths_depths_and_point_counts(cuda_device, sizes, points, dtype):
+    _check(sizes, points, "second", dtype=dtype)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("activation", ["tanh", "sin"])
 @pytest.mark.parametrize("width,kind,inputs", [
     (64, "value", 2), (64, "first", 2), (64, "burgers", 2), (64, "laplacian", 2), (64, "laplacian", 3), (64, "laplacian", 4),
     (50, "laplacian", 4), (48, "burgers", 2), (32, "laplacian", 3), (16, "laplacian", 4)])
-def test_signatures(cuda_device, activation, width, kind, inputs):
-    _check([inputs, width, width, width, 1], 1037, kind, activation)
+def test_signatures(cuda_device, activation, width, kind, inputs, dtype):
+    _check([inputs, width, width, width, 1], 1037, kind, activation, dtype=dtype)
 
 
 @pytest.mark.parametrize("scale", [2.0 ** -40, 2.0 ** -12, 16.0])
