@@ -81,12 +81,20 @@ __device__ __forceinline__ float block_scale(uint32_t largest, float* inverse) {
     return __uint_as_float((e - 13u) << 23);
 }
 
-// Two scaled elements as packed float16 hi and lo pairs.
-__device__ __forceinline__ void split_f16(float x0, float x1, float inverse, uint32_t& hi, uint32_t& lo) {
+// Mean relative loss of mma_step's truncating accumulations: a factor common to all contractions, which neither the
+// number of points nor of terms averages out, so it is put back where that costs nothing: into the weights' lo parts and
+// into the finished weight-gradient sums.  Measured as <error, exact> / <exact, exact> of 40,000 16 x 16 x 16 steps against float64:
+// -3.9e-8 (normal operands), -4.1e-8 (uniform), -4.4e-8 (positive).  Without it gradients of networks of width 16, 32 and
+// 50 were 2 to 5 times further from float64 than plain float32 multiply-adds.
+constexpr float MMA_TRUNCATION = 4.1e-8f;
+
+// Two scaled elements as packed float16 hi and lo pairs, raised by `gain` of themselves.
+__device__ __forceinline__ void split_f16(float x0, float x1, float inverse, uint32_t& hi, uint32_t& lo, float gain = 0.0f) {
     const float y0 = x0 * inverse, y1 = x1 * inverse;
     const __half2 h = __floats2half2_rn(y0, y1);
     const float2 back = __half22float2(h);
-    const __half2 l = __floats2half2_rn(y0 - back.x, y1 - back.y);
+    const __half2 l = gain == 0.0f ? __floats2half2_rn(y0 - back.x, y1 - back.y)
+                                   : __floats2half2_rn(fmaf(y0, gain, y0 - back.x), fmaf(y1, gain, y1 - back.y));
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
@@ -162,7 +170,7 @@ static __global__ void __launch_bounds__(1024) prep_weights_kernel(const float* 
         const float x0 = (r < rows && c < cols) ? w[r * cols + c] : 0.0f;
         const float x1 = (r < rows && c + 1 < cols) ? w[r * cols + c + 1] : 0.0f;
         uint32_t hi, lo;
-        split_f16(x0, x1, inverse, hi, lo);
+        split_f16(x0, x1, inverse, hi, lo, MMA_TRUNCATION);
         img[r * stride + c / 2] = hi;
         img[plane + r * stride + c / 2] = lo;
     }
@@ -695,7 +703,11 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
             const int rows = a.width[l - 1], cols = a.width[l];
             float* out = my_grad + a.w_off[l];
             for (int q = 0; q < 2 * NW; ++q) {
-                const float4 v = dws[((size_t)(l - 1) * 2 * NW + q) * THREADS + tid];
+                float4 v = dws[((size_t)(l - 1) * 2 * NW + q) * THREADS + tid];
+                v.x = fmaf(v.x, MMA_TRUNCATION, v.x);
+                v.y = fmaf(v.y, MMA_TRUNCATION, v.y);
+                v.z = fmaf(v.z, MMA_TRUNCATION, v.z);
+                v.w = fmaf(v.w, MMA_TRUNCATION, v.w);
                 const int k = col0 + g, n = (q >> 1) * 16 + (q & 1) * 8 + 2 * t;
                 if (k < rows && n < cols) out[k * cols + n] = v.x;
                 if (k < rows && n + 1 < cols) out[k * cols + n + 1] = v.y;

@@ -91,3 +91,23 @@ def test_streams_of_very_different_size(cuda_device, scale):
     # Derivative streams grow with the scale of the first weights, to the first and second power: block scales keep
     # each stream's relative accuracy (a plain float16 operand would be subnormal or infinite here).
     _check([2, 64, 64, 1], 1040, "burgers", "sin", scale=scale)
+
+
+@pytest.mark.parametrize("width", [16, 32, 50, 64])
+def test_truncation_leaves_no_common_factor(cuda_device, width):
+    # The tensor core's truncation lowers every contraction by about 4e-8 of itself, which no sum over points averages
+    # out and which the residual of the heat equation amplifies (2e-6 on these gradients before the weights made up for
+    # it).  What is left is random: 1e-7 per factor (2^-23), averaged over 10,007 points; 5e-7 allows for the residual.
+    loss = workloads.make("heat3d", 128).loss
+    params = workloads.init_mlp(qb.random.key(10007 + width), [4] + [width] * 4 + [1], np.float32)
+    points = np.random.default_rng(10007 + width).uniform(0.0, 1.0, (10007, 4)).astype(np.float32)
+
+    def flat(tree):
+        return np.concatenate([np.asarray(layer[k], np.float64).ravel() for layer in tree for k in ("w", "b")])
+
+    wide = [{k: v.astype(np.float64) for k, v in layer.items()} for layer in params]
+    step = qb.jit(qb.value_and_grad(loss), device="cuda:0")
+    value, grads = step(params, points)
+    exact_value, exact = step(wide, points.astype(np.float64))
+    assert np.linalg.norm(flat(grads) - flat(exact)) <= 5e-7 * np.linalg.norm(flat(exact))
+    assert abs(float(value) - float(exact_value)) <= 5e-7 * abs(float(exact_value))
