@@ -20,7 +20,7 @@ LIMIT = 128 << 20
 IDLE_LIMIT = 32 << 20
 _SMALLEST = 4096
 
-_lock = threading.Lock()
+_lock = threading.RLock()  # a collection inside a locked section may run _Block.__del__ on the same thread
 _idle: dict[int, list[int]] = {}   # block size -> addresses
 _total = 0                         # page-locked bytes, handed out or idle
 _idle_bytes = 0

@@ -47,13 +47,13 @@ void staging_detach(int device) {
     if (--p.users == 0) p.clear();
 }
 
-cudaError_t staging_acquire(int device, StagingBlock** out) {
+cudaError_t staging_acquire(int device, int limit, StagingBlock** out) {
     StagingBlock* block = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         Pool& p = pool(device);
         const bool oldest_done = !p.idle.empty() && (!p.idle.front()->queued || cudaEventQuery(p.idle.front()->done) == cudaSuccess);
-        if (!oldest_done && (int)p.blocks.size() < STAGING_BLOCKS) {
+        if (!oldest_done && (int)p.blocks.size() < (p.idle.empty() ? STAGING_BLOCKS : limit)) {
             std::unique_ptr<StagingBlock> fresh(new StagingBlock());
             void* raw = nullptr;
             cudaError_t e = cudaHostAlloc(&raw, STAGING_BLOCK_BYTES, cudaHostAllocPortable);

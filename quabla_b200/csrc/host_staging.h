@@ -13,6 +13,10 @@ namespace qb {
 
 constexpr size_t STAGING_BLOCK_BYTES = (size_t)1 << 20;  // one transfer; larger arrays go in pieces, so that the
                                                          // host copy of one piece overlaps the transfer of the last
+// A block costs 1 to 3 ms to page-lock and its transfer 0.03 ms: a plan's first inputs, which nothing runs ahead of, go
+// through two blocks (a 16 MiB batch through sixteen new ones made the first bind of a plan 50 ms longer); later
+// batches, queued behind steps still running, may take the pool to its bound.
+constexpr int STAGING_FIRST_BLOCKS = 2;
 constexpr int STAGING_BLOCKS = 16;                       // bound of the pool: 16 MiB of pinned memory per device
 
 struct StagingBlock {
@@ -24,9 +28,9 @@ struct StagingBlock {
 // Users of the pool of `device` (the current device of the calling thread); the last one out frees the memory.
 void staging_attach(int device);
 void staging_detach(int device);
-// A block no transfer is reading (waits for the oldest transfer when every block has one); *out is null when all
-// blocks are in other callers' hands, and the caller then copies without staging.
-cudaError_t staging_acquire(int device, StagingBlock** out);
+// A block no transfer is reading; while all have one, a new block up to `limit` of them, else the oldest after its transfer.
+// *out is null when all blocks are in other callers' hands, and the caller then copies without staging.
+cudaError_t staging_acquire(int device, int limit, StagingBlock** out);
 // Transfers from `block` queued on `stream` so far must finish before it is handed out again.
 cudaError_t staging_release(int device, StagingBlock* block, cudaStream_t stream);
 

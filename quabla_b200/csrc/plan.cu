@@ -236,7 +236,7 @@ class Plan final : public qb200_plan {
     }
     qb200_status run(bool forward_only);
     qb200_status enqueue(bool forward_only);
-    qb200_status upload(size_t offset, const void* host, size_t nbytes, cudaStream_t stream);
+    qb200_status upload(size_t offset, const void* host, size_t nbytes, int staging_limit, cudaStream_t stream);
     qb200_status run_chunk(int si, long long point0, int C, int partial_slot, bool forward_only);
     qb200_status run_fused(int si, bool forward_only);
     qb200_status prepare_weight_images();
@@ -782,13 +782,13 @@ qb200_status Plan<T>::bind(const char* name, const void* host, size_t nbytes) {
 // Host array into the arena through pinned blocks: the caller's buffer is free when this returns, the transfers
 // are queued on `stream`.
 template <typename T>
-qb200_status Plan<T>::upload(size_t offset, const void* host, size_t nbytes, cudaStream_t stream) {
+qb200_status Plan<T>::upload(size_t offset, const void* host, size_t nbytes, int staging_limit, cudaStream_t stream) {
     const unsigned char* src = static_cast<const unsigned char*>(host);
     unsigned char* dst = reinterpret_cast<unsigned char*>(d_arena_ + offset);
     for (size_t at = 0; at < nbytes; at += STAGING_BLOCK_BYTES) {
         const size_t piece = std::min(STAGING_BLOCK_BYTES, nbytes - at);
         StagingBlock* block = nullptr;
-        QB_CUDA(staging_acquire(device_, &block));
+        QB_CUDA(staging_acquire(device_, staging_limit, &block));
         if (block == nullptr) {
             QB_CUDA(cudaMemcpyAsync(dst + at, src + at, piece, cudaMemcpyHostToDevice, stream));
             QB_CUDA(cudaStreamSynchronize(stream));
@@ -826,6 +826,9 @@ qb200_status Plan<T>::bind_many(const int32_t* slots, const void* const* hosts, 
     }
     std::lock_guard<std::recursive_mutex> lock(mutex_);
     QB_TRY(use_device());
+    int staging_limit = STAGING_BLOCKS;
+    for (int i = 0; i < n; ++i)
+        if (!(slots[i] < np ? leaves_[slots[i]].bound : inputs_[slots[i] - np].bound)) staging_limit = STAGING_FIRST_BLOCKS;
     cudaStream_t stream = stream_;
     if (!params && total >= COPY_STREAM_BYTES) {
         if (copy_stream_ == nullptr) QB_CUDA(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
@@ -848,9 +851,9 @@ qb200_status Plan<T>::bind_many(const int32_t* slots, const void* const* hosts, 
             ++j;
         }
         StagingBlock* block = nullptr;
-        if (j > i + 1) QB_CUDA(staging_acquire(device_, &block));
+        if (j > i + 1) QB_CUDA(staging_acquire(device_, staging_limit, &block));
         if (block == nullptr) {
-            for (; i < j; ++i) QB_TRY(upload(offset_of(slots[i]), hosts[i], nbytes[i], stream));
+            for (; i < j; ++i) QB_TRY(upload(offset_of(slots[i]), hosts[i], nbytes[i], staging_limit, stream));
             continue;
         }
         size_t at = first;
@@ -1114,7 +1117,7 @@ qb200_status Plan<float>::tc_setup() {
         tc_fwd_[l] = tc_rows_ok(N, K);
         tc_bwd_[l] = l > 0 && tc_rows_ok(K, N);
         tc_wgrad_[l] = tc_wgrad_ok(K, N);
-        if (tc_fwd_[l] || tc_bwd_[l]) QB_TRY(dev_alloc(&tc_image_[l], 2 * tc_image_words(K, N)));  // one image per scheme
+        if (tc_fwd_[l] || tc_bwd_[l]) QB_TRY(dev_alloc(&tc_image_[l], tc_image_words(K, N)));
         tc_any_ = tc_any_ || tc_fwd_[l] || tc_bwd_[l] || tc_wgrad_[l];
     }
     return QB200_OK;
