@@ -336,11 +336,14 @@ class Plan final : public qb200_plan {
         T* U = nullptr;
         T* Uhat = nullptr;
         T* wpartial = nullptr;
+        size_t wpartial_elems = 0;
         double* acc = nullptr;     // gradient accumulators of the chunks that went down this lane
         cudaEvent_t done = nullptr;
     };
     std::vector<Lane> lanes_;
     cudaStream_t cs_ = nullptr;    // stream of the lane in use
+    bool by_set_ = false;          // two lanes: the largest set down the first, the others down the second
+    int main_set_ = 0;             // the largest set
     bool single_lane_ = false;     // option QB200_OPT_SINGLE_LANE: every chunk down lane 0 (for per-kernel timing)
     cudaEvent_t ev_lanes_ = nullptr;
     void select_lane(int k) {
@@ -352,6 +355,7 @@ class Plan final : public qb200_plan {
         U_ = ln.U;
         Uhat_ = ln.Uhat;
         wpartial_ = ln.wpartial;
+        wpartial_elems_ = ln.wpartial_elems;
         d_acc_ = ln.acc;
         cs_ = ln.stream;
     }
@@ -591,11 +595,32 @@ qb200_status Plan<T>::init() {
         const char* env = getenv("QB200_LANES");
         const int asked = env != nullptr ? atoi(env) : 0;
         if (largest >= 16384 && (asked == 2 || (asked != 1 && sizeof(T) == 8))) n_lanes = 2;
+        // Plans that keep one lane for their largest set send the other sets down a second one: a boundary set is some
+        // fifty launches of a few microseconds each, which come on top of the interior's work on its stream and cost next to
+        // nothing beside it (Burgers gradients, 10,007 + 312 + 312 points: 2682 us on one lane, 1995 us on two).  Only
+        // where no set is cut into chunks by half the scratch budget.
+        if (n_lanes == 1 && asked != 1 && desc_.sets.size() > 1) {
+            by_set_ = true;
+            for (size_t si = 0; si < desc_.sets.size(); ++si) {
+                const long long S = desc_.sets[si].streams(), n = desc_.sets[si].n;
+                const size_t per_point = (size_t)S * (sum_h + sum_z + 2 * (size_t)dmax + 2) * sizeof(T);
+                if (n > chunk_cap || n > (long long)K_CHUNK_ROWS * 512 / S || (size_t)n > budget / 2 / per_point) by_set_ = false;
+                if (n > desc_.sets[main_set_].n) main_set_ = (int)si;
+            }
+            if (by_set_) n_lanes = 2;
+        }
     }
     budget /= (size_t)n_lanes;
-    size_t max_rows = 0, max_chunk = 0;
-    std::vector<size_t> h_elems(L_, 0), z_elems(L_, 0);
-    size_t g_elems = 0;
+    // What each lane must hold: every set for the first (QB200_OPT_SINGLE_LANE), its own for a second one by sets.
+    struct LaneSize {
+        size_t rows = 0, g = 0;
+        std::vector<size_t> h, z;
+    };
+    std::vector<LaneSize> lane_size(n_lanes);
+    for (auto& ls : lane_size) {
+        ls.h.assign(L_, 0);
+        ls.z.assign(L_, 0);
+    }
     sets_.resize(desc_.sets.size());
     for (size_t si = 0; si < desc_.sets.size(); ++si) {
         const auto& s = desc_.sets[si];
@@ -627,7 +652,7 @@ qb200_status Plan<T>::init() {
         // Bound the split-K slices of a weight gradient (512: the 3-D heat step then runs in six chunks).
         chunk = std::min<long long>(chunk, (long long)K_CHUNK_ROWS * 512 / (long long)S);
         // With two lanes a set is cut into at least two chunks.
-        if (n_lanes > 1 && s.n >= 16384) chunk = std::min<long long>(chunk, ((s.n + 1) / 2 + 255) / 256 * 256);
+        if (n_lanes > 1 && !by_set_ && s.n >= 16384) chunk = std::min<long long>(chunk, ((s.n + 1) / 2 + 255) / 256 * 256);
         if (chunk >= s.n) {
             chunk = s.n;
         } else {
@@ -637,13 +662,16 @@ qb200_status Plan<T>::init() {
             chunk = std::min(chunk, ((s.n + count - 1) / count + 255) / 256 * 256);
         }
         st.chunk = (int)chunk;
-        max_chunk = std::max(max_chunk, (size_t)chunk);
-        max_rows = std::max(max_rows, S * (size_t)chunk);
-        for (int l = 0; l < L_; ++l) {
-            h_elems[l] = std::max(h_elems[l], S * (size_t)chunk * desc_.sizes[l]);
-            if (l >= 1) z_elems[l] = std::max(z_elems[l], S * (size_t)chunk * desc_.sizes[l]);
+        for (int k = 0; k < n_lanes; ++k) {
+            if (k == 1 && by_set_ && (int)si == main_set_) continue;
+            LaneSize& ls = lane_size[k];
+            ls.rows = std::max(ls.rows, S * (size_t)chunk);
+            for (int l = 0; l < L_; ++l) {
+                ls.h[l] = std::max(ls.h[l], S * (size_t)chunk * desc_.sizes[l]);
+                if (l >= 1) ls.z[l] = std::max(ls.z[l], S * (size_t)chunk * desc_.sizes[l]);
+            }
+            ls.g = std::max(ls.g, S * (size_t)chunk * dmax);
         }
-        g_elems = std::max(g_elems, S * (size_t)chunk * dmax);
 
         QB_TRY(dev_alloc(&st.table, (size_t)s.n * st.ncols));
         std::vector<T> dirs(std::max<size_t>(1, s.dirs.size() * d0));
@@ -713,15 +741,17 @@ qb200_status Plan<T>::init() {
         return QB200_OK;
     }
     QB_TRY(tc_setup());
-    const size_t slices = (max_rows + K_CHUNK_ROWS - 1) / K_CHUNK_ROWS + SM_COUNT + 1;  // see slice_rows()
-    // Weight-gradient slices, or the (at most BIAS_SLICES) row slices of a bias gradient.
-    const size_t partial_elems = std::max(slices * std::max<size_t>(wmax, (size_t)dmax), (size_t)BIAS_SLICES * dmax);
-    wpartial_elems_ = partial_elems;
+    // Weight-gradient slices (see slice_rows()), or the (at most BIAS_SLICES) row slices of a bias gradient.
+    auto partial_elems = [&](size_t rows) {
+        const size_t slices = (rows + K_CHUNK_ROWS - 1) / K_CHUNK_ROWS + SM_COUNT + 1;
+        return std::max(slices * std::max<size_t>(wmax, (size_t)dmax), (size_t)BIAS_SLICES * dmax);
+    };
     scratch_bytes_ = 0;
     lanes_.resize(n_lanes);
     QB_CUDA(cudaEventCreateWithFlags(&ev_lanes_, cudaEventDisableTiming));
     for (int k = 0; k < n_lanes; ++k) {
         Lane& ln = lanes_[k];
+        const LaneSize& size = lane_size[k];
         if (k == 0)
             ln.stream = stream_;
         else
@@ -730,20 +760,21 @@ qb200_status Plan<T>::init() {
         ln.H.assign(L_, nullptr);
         ln.Z.assign(L_, nullptr);
         for (int l = 0; l < L_; ++l) {
-            QB_TRY(dev_alloc(&ln.H[l], h_elems[l]));
-            scratch_bytes_ += h_elems[l] * sizeof(T);
+            QB_TRY(dev_alloc(&ln.H[l], size.h[l]));
+            scratch_bytes_ += size.h[l] * sizeof(T);
             if (l >= 1) {
-                QB_TRY(dev_alloc(&ln.Z[l], z_elems[l]));
-                scratch_bytes_ += z_elems[l] * sizeof(T);
+                QB_TRY(dev_alloc(&ln.Z[l], size.z[l]));
+                scratch_bytes_ += size.z[l] * sizeof(T);
             }
         }
-        QB_TRY(dev_alloc(&ln.G[0], g_elems));
-        QB_TRY(dev_alloc(&ln.G[1], g_elems));
-        QB_TRY(dev_alloc(&ln.U, max_rows));
-        QB_TRY(dev_alloc(&ln.Uhat, max_rows));
-        QB_TRY(dev_alloc(&ln.wpartial, partial_elems));
+        ln.wpartial_elems = partial_elems(size.rows);
+        QB_TRY(dev_alloc(&ln.G[0], size.g));
+        QB_TRY(dev_alloc(&ln.G[1], size.g));
+        QB_TRY(dev_alloc(&ln.U, size.rows));
+        QB_TRY(dev_alloc(&ln.Uhat, size.rows));
+        QB_TRY(dev_alloc(&ln.wpartial, ln.wpartial_elems));
         QB_TRY(dev_alloc(&ln.acc, n_params_));
-        scratch_bytes_ += (2 * g_elems + 2 * max_rows + partial_elems) * sizeof(T);
+        scratch_bytes_ += (2 * size.g + 2 * size.rows + ln.wpartial_elems) * sizeof(T);
     }
     select_lane(0);
     return QB200_OK;
@@ -1551,6 +1582,7 @@ qb200_status Plan<T>::enqueue(bool forward_only) {
         }
         for (long long p0 = 0; p0 < n; p0 += st.chunk) {
             const int C = (int)std::min<long long>(st.chunk, n - p0);
+            if (by_set_) next_lane = single_lane_ || (int)si == main_set_ ? 0 : 1;
             select_lane(next_lane);
             next_lane = single_lane_ ? 0 : (next_lane + 1) % (int)lanes_.size();
             QB_TRY(run_chunk((int)si, p0, C, slot, forward_only));
