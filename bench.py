@@ -349,7 +349,7 @@ class Rig:
 
 
 ENGINES = {0: "layer-wise (FP64 tensor-core / SIMT GEMMs)", 1: "fused (FP32/FP64 pipe)",
-           2: "fused (tensor cores, 3xTF32 mma)", 3: "layer-wise (tcgen05 split-float32 GEMMs)"}
+           2: "fused (tensor cores, float16 pairs)", 3: "layer-wise (tcgen05 split-float32 GEMMs)"}
 
 
 def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: int, peaks: dict, live: dict,
@@ -389,10 +389,10 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
         gemm_ns = plan.query(_lib.Q_GEMM_NANOSECONDS)
         gemm_launches = max(1, plan.query(_lib.Q_GEMM_LAUNCHES))
         gemm_flops = float(plan.query(_lib.Q_GEMM_FLOPS))
-        # Tensor-pipe work of the same launches at the bf16 rate: 6 passes per FLOP for a product made of three
-        # tf32 instructions, 4 where the two correction products are bf16 instructions (0 off the tensor pipe).
+        # Tensor-pipe work of the same launches at the bf16 rate: 3 passes per FLOP for three float16 products, 6 for
+        # three tf32 ones, 4 for a tf32 product with two bf16 corrections (0 off the tensor pipe).
         pipe_flops = float(plan.query(_lib.Q_GEMM_PIPE_FLOPS))
-        kernel = {"name": "tc_tma_gemm_kernel (tcgen05: tf32 product + two correction products)" if engine == 3 else
+        kernel = {"name": "tc_tma_gemm_kernel (tcgen05: three float16 or tf32 products)" if engine == 3 else
                   "dmma_gemm_kernel (FP64 MMA) / gemm_kernel" if dtype_name == "f64" else "gemm_kernel",
                   "launches_per_step": int(gemm_launches), "us_per_launch": gemm_ns * 1e-3 / gemm_launches,
                   "flops_per_launch": gemm_flops / gemm_launches, "us_per_step": gemm_ns * 1e-3,
@@ -406,7 +406,7 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
         flops = w.flops_per_point(interior.streams) * local_points
         kernel = {"name": "fused_mma_kernel" if engine == 2 else "fused_step_kernel", "launches_per_step": 1,
                   "us_per_launch": set0_ns * 1e-3, "flops_per_launch": flops, "us_per_step": set0_ns * 1e-3,
-                  "bf16_rate_passes_per_flop": 6.0 if dtype_name == "f32" else 0.0}
+                  "bf16_rate_passes_per_flop": 3.0 if engine == 2 else 6.0 if dtype_name == "f32" else 0.0}
         achieved = flops / max(set0_ns, 1) * 1e-3
     allreduce_us = plan.query(_lib.Q_ALLREDUCE_NANOSECONDS) * 1e-3 if rig.world > 1 else 0.0
 
@@ -448,9 +448,8 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
     step_flops = (w.flops_per_point(streams) * w.interior_points
                   + sum(w.flops_per_point(s) * n for n, s in w.extra))
     if dtype_name == "f32":
-        # Split float32 on the tensor pipe: a tf32 instruction runs at half the bf16 rate, so three tf32 products
-        # cost 6 bf16-rate passes per FLOP and a tf32 product with two bf16 correction products costs 4; the
-        # denominator is the bf16 rate over the passes the timed launches actually execute.  The burst figure
+        # Split float32 on the tensor pipe: three float16 products cost 3 bf16-rate passes per FLOP and three tf32
+        # products, at half that rate, 6; the denominator is the bf16 rate over the passes the timed launches actually execute.  The burst figure
         # for kernels timed alone in a short step, the sustained one (seconds-long loop under the power cap)
         # when the timed kernels keep the GPU busy for tens of milliseconds per step.
         sustained = kernel["us_per_step"] > 2e4 and "bf16_tflops_sustained" in peaks
@@ -493,18 +492,9 @@ def parity_step(rig: Rig, name: str) -> dict:
     from quabla_b200._transforms import CompiledLoss
 
     w = workloads.make(name, PARITY_POINTS)
-    # The timed step's tcgen05 GEMMs run the scheme the library picks for large launches (bfloat16 correction
-    # products); a launch of this size would get the other one, so the parity step asks for the timed one.
-    forced = "QB200_TC_COR" not in os.environ
-    if forced:
-        os.environ["QB200_TC_COR"] = "bf16"
-    try:
-        trainer, plan = rig.trainer(w, rig.shard(w))
-        plan.execute()
-        outputs = plan.outputs()
-    finally:
-        if forced:
-            del os.environ["QB200_TC_COR"]
+    trainer, plan = rig.trainer(w, rig.shard(w))
+    plan.execute()
+    outputs = plan.outputs()
     dtype_name = "f32" if np.dtype(w.dtype) == np.float32 else "f64"
     tolerance = PARITY_TOLERANCE[dtype_name]
     worst = 0.0
