@@ -251,10 +251,7 @@ class Plan final : public qb200_plan {
     bool tc_fwd_ok(int layer) const { return !tc_fwd_.empty() && tc_fwd_[layer]; }
     bool tc_bwd_ok(int layer) const { return !tc_bwd_.empty() && tc_bwd_[layer]; }
     // Tensor-pipe passes of a forward or data-gradient product at the bfloat16 rate (QB200_Q_GEMM_PIPE_FLOPS).
-    static double tc_rows_weight() {
-        const TcScheme scheme = tc_scheme();
-        return scheme == TC_F16 ? 3.0 : scheme == TC_BF16 ? 4.0 : 6.0;
-    }
+    static double tc_rows_weight(long long rows) { return tc_cor16_for(rows) ? 4.0 : 6.0; }
     bool tc_wgrad_ok_layer(int layer) const { return !tc_wgrad_.empty() && tc_wgrad_[layer]; }
     StepStatus<T> step_status(bool with_flat_flag) const {
         StepStatus<T> s;
@@ -398,7 +395,6 @@ class Plan final : public qb200_plan {
     std::vector<uint32_t*> tc_image_;   // per layer: pre-split weight images (null: not eligible)
     std::vector<char> tc_fwd_, tc_bwd_, tc_wgrad_;
     bool tc_any_ = false;
-    TcScheme tc_scheme_ = TC_F16;  // of the weight images in place; a step's launches follow it
     cudaEvent_t ev_begin_ = nullptr, ev_end_ = nullptr;  // around the kernels of point set 0
     cudaEvent_t ev_ar0_ = nullptr, ev_ar1_ = nullptr;    // around the gradient all-reduce
     bool ev_valid_ = false, ev_ar_valid_ = false;
@@ -1160,14 +1156,24 @@ qb200_status Plan<float>::tc_setup() {
 
 template <>
 qb200_status Plan<float>::tc_prepare() {
-    tc_scheme_ = tc_scheme();
     for (int l = 0; l < L_; ++l) {
         if (tc_image_[l] == nullptr) continue;
-        const cudaError_t e = tc2_prepare_launch(weight(l), desc_.sizes[l], desc_.sizes[l + 1],
-                                                 reinterpret_cast<float*>(tc_image_[l]), tc_scheme_, stream_);
-        ++launches_;
-        if (e != cudaSuccess)
-            return fail(QB200_CUDA_ERROR, "launch of the weight image kernel failed: %s", cudaGetErrorString(e));
+        // TMA kernels take the weight unsplit plus its lo plane: W itself for the data gradient, W^T for the
+        // forward product.  Image: four parts of K*N words (tc_image_words).
+        // The first image serves launches with bfloat16 corrections, the second those with tf32 corrections; which
+        // of the two a launch takes depends on its rows (tc_cor16_for), so both are written unless one is forced.
+        const size_t kn = (size_t)desc_.sizes[l] * desc_.sizes[l + 1];
+        const int mode = tc_cor_mode();
+        for (int scheme = 0; scheme < 2; ++scheme) {
+            const bool cor16 = scheme == 0;
+            if ((mode == 0 && cor16) || (mode == 1 && !cor16)) continue;
+            float* image = reinterpret_cast<float*>(tc_image_[l]) + (cor16 ? 0 : 4 * kn);
+            cudaError_t e = tc2_prepare_launch(weight(l), desc_.sizes[l], desc_.sizes[l + 1], image, image + kn, image + 2 * kn,
+                                               image + 3 * kn, cor16, stream_);
+            ++launches_;
+            if (e != cudaSuccess)
+                return fail(QB200_CUDA_ERROR, "launch of tc_prep_weight_kernel failed: %s", cudaGetErrorString(e));
+        }
     }
     return QB200_OK;
 }
@@ -1175,9 +1181,11 @@ qb200_status Plan<float>::tc_prepare() {
 template <>
 bool Plan<float>::tc_forward(int layer, const float* A, float* C, long long rows, int bias_rows, qb200_status* st) {
     if (!tc_fwd_[layer]) return false;
-    const cudaError_t e = tc2_rows_launch(A, (int)rows, desc_.sizes[layer], desc_.sizes[layer + 1], weight(layer),
-                                          reinterpret_cast<float*>(tc_image_[layer]), false, C, bias(layer), bias_rows,
-                                          tc_scheme_, d_error_, cs_);
+    const int K = desc_.sizes[layer], N = desc_.sizes[layer + 1];
+    const bool cor16 = tc_cor16_for(rows);
+    const float* image = reinterpret_cast<const float*>(tc_image_[layer]) + (cor16 ? 0 : 4 * (size_t)K * N);
+    cudaError_t e = tc2_rows_launch(A, K, image, image + (size_t)K * N, K, C, N, bias(layer), bias_rows, (int)rows, N, K, cor16,
+                                    d_error_, cs_);
     ++launches_;
     *st = e == cudaSuccess ? QB200_OK : fail(QB200_CUDA_ERROR, "launch of tc_gemm_kernel(forward) failed: %s", cudaGetErrorString(e));
     return true;
@@ -1186,9 +1194,12 @@ bool Plan<float>::tc_forward(int layer, const float* A, float* C, long long rows
 template <>
 bool Plan<float>::tc_dgrad(int layer, const float* G, float* Gprev, long long rows, qb200_status* st) {
     if (!tc_bwd_[layer]) return false;
-    const cudaError_t e = tc2_rows_launch(G, (int)rows, desc_.sizes[layer], desc_.sizes[layer + 1], weight(layer),
-                                          reinterpret_cast<float*>(tc_image_[layer]), true, Gprev, nullptr, 0, tc_scheme_,
-                                          d_error_, cs_);
+    const int K = desc_.sizes[layer], N = desc_.sizes[layer + 1];
+    // The weight itself is the K-major operand here (its tf32-rounded copy when the corrections run in bfloat16).
+    const bool cor16 = tc_cor16_for(rows);
+    const float* image = reinterpret_cast<const float*>(tc_image_[layer]) + (cor16 ? 0 : 4 * (size_t)K * N);
+    cudaError_t e = tc2_rows_launch(G, N, cor16 ? image + 3 * (size_t)K * N : weight(layer), image + 2 * (size_t)K * N, N, Gprev,
+                                    K, nullptr, 0, (int)rows, K, N, cor16, d_error_, cs_);
     ++launches_;
     *st = e == cudaSuccess ? QB200_OK : fail(QB200_CUDA_ERROR, "launch of tc_gemm_kernel(dgrad) failed: %s", cudaGetErrorString(e));
     return true;
@@ -1264,7 +1275,7 @@ qb200_status Plan<T>::run_chunk(int si, long long point0, int C, int partial_slo
         g.k_chunk = g.K;
         qb200_status tc_status = QB200_OK;
         const bool narrow = g.K <= 4 && g.N % 4 == 0 && g.N >= 32 && 256 % (g.N / 4) == 0;
-        if (tc_fwd_ok(l - 1) || !narrow) timer_begin(2.0 * (double)rows * g.N * g.K, tc_fwd_ok(l - 1) ? tc_rows_weight() : 0.0);
+        if (tc_fwd_ok(l - 1) || !narrow) timer_begin(2.0 * (double)rows * g.N * g.K, tc_fwd_ok(l - 1) ? tc_rows_weight(rows) : 0.0);
         if (tc_forward(l - 1, H_[l - 1], Z_[l], rows, C, &tc_status)) {
             QB_TRY(tc_status);
             timer_end();
@@ -1482,7 +1493,7 @@ qb200_status Plan<T>::run_chunk(int si, long long point0, int C, int partial_slo
             g.bias_rows = 0;
             g.k_chunk = g.K;
             qb200_status tc_status = QB200_OK;
-            timer_begin(2.0 * (double)rows * g.N * g.K, tc_bwd_ok(l - 1) ? tc_rows_weight() : 0.0);
+            timer_begin(2.0 * (double)rows * g.N * g.K, tc_bwd_ok(l - 1) ? tc_rows_weight(rows) : 0.0);
             if (tc_dgrad(l - 1, G_[cur], G_[cur ^ 1], rows, &tc_status)) {
                 QB_TRY(tc_status);
             } else {

@@ -13,22 +13,31 @@ static bool tc_switch_on() {
     return !(env != nullptr && strcmp(env, "0") == 0);
 }
 
-// How the forward and data-gradient GEMMs split their float32 operands (tc_tma_gemm.cuh): two float16 parts of scaled
-// rows at every size; it is both the fastest (six tensor instructions and 32 KB of loads per k-tile against eight and
-// 48 KB, and twelve and 48 KB) and the most accurate of the three.  QB200_TC_COR=tf32 or =bf16 (read at every call)
-// selects one of the others for comparisons: three tf32 products, or tf32 with bfloat16 corrections.
-TcScheme tc_scheme() {
+// Correction products of the forward and data-gradient GEMMs: bfloat16 instructions on tf32-rounded hi parts, or
+// tf32 instructions on truncated hi parts (the plain 3xTF32 scheme).  The bfloat16 scheme is about 9 % faster per
+// GEMM and leaves a random error of 6.7e-7 per output against ~1e-7 (its systematic part is smaller); in sums over
+// the rows of a launch (bias gradients above all) random errors shrink with the square root of the row count, so
+// it is used for launches of at least TC_COR16_MIN_ROWS rows, where it stays below what a plain float32 FMA product
+// leaves on a few hundred rows.  QB200_TC_COR=tf32 or =bf16 (read at every call) forces one scheme.
+constexpr long long TC_COR16_MIN_ROWS = 65536;
+
+int tc_cor_mode() {
     const char* env = getenv("QB200_TC_COR");
-    if (env != nullptr && strcmp(env, "tf32") == 0) return TC_TF32;
-    if (env != nullptr && strcmp(env, "bf16") == 0) return TC_BF16;
-    return TC_F16;
+    if (env != nullptr && strcmp(env, "tf32") == 0) return 0;
+    if (env != nullptr && strcmp(env, "bf16") == 0) return 1;
+    return 2;
+}
+
+bool tc_cor16_for(long long rows) {
+    const int mode = tc_cor_mode();
+    return mode == 1 || (mode == 2 && rows >= TC_COR16_MIN_ROWS);
 }
 
 bool tc_rows_ok(int N, int K) { return N % 64 == 0 && N >= 64 && N <= 256 && K % TC_BK == 0 && K >= TC_BK; }
 
 bool tc_wgrad_ok(int Mw, int N) { return Mw % TC_BM == 0 && N % 64 == 0 && N >= 64 && N <= 256; }
 
-size_t tc_image_words(int K, int N) { return (size_t)4 * K * N; }
+size_t tc_image_words(int K, int N) { return (size_t)4 * K * N; }  // one image; a plan keeps one per scheme
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -64,7 +73,7 @@ static bool make_map(CUtensorMap* map, const float* base, long long rows, int co
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// 16-bit pair matrix of tc2_prepare_launch: [rows][2 * inner] halves, boxes of 64 halves (128 bytes) x box_rows under
+// bfloat16 pair matrix of tc2_prepare_launch: [rows][2 * inner] halves, boxes of 64 halves (128 bytes) x box_rows under
 // the 128-byte swizzle.
 static bool make_map16(CUtensorMap* map, const void* base, long long rows, int inner, int box_rows) {
     const cuuint64_t dims[2] = {(cuuint64_t)(2 * inner), (cuuint64_t)rows};
@@ -76,56 +85,41 @@ static bool make_map16(CUtensorMap* map, const void* base, long long rows, int i
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-TcImage tc_image(float* words, int K, int N) {
-    const size_t kn = (size_t)K * N;
-    TcImage im;
-    im.first = words;
-    im.second = words + kn;
-    im.third = words + 2 * kn;
-    im.fourth = words + 3 * kn;
-    return im;
-}
-
-cudaError_t tc2_prepare_launch(const float* w, int K, int N, float* words, TcScheme scheme, cudaStream_t stream) {
-    const TcImage im = tc_image(words, K, N);
-    const dim3 tiles((N + 31) / 32, (K + 31) / 32), block(32, 8);
-    if (scheme == TC_F16)
-        t2_prepare_f16_kernel<<<(N + K + 7) / 8, 256, 0, stream>>>(w, K, N, reinterpret_cast<__half*>(im.first),
-                                                                    reinterpret_cast<__half*>(im.second), im.third, im.third + N);
-    else if (scheme == TC_BF16)
-        t2_prepare16_kernel<<<tiles, block, 0, stream>>>(w, K, N, im.first, reinterpret_cast<uint16_t*>(im.second),
-                                                         reinterpret_cast<uint16_t*>(im.third), im.fourth);
-    else
-        t2_prepare_kernel<<<tiles, block, 0, stream>>>(w, K, N, im.first, reinterpret_cast<uint32_t*>(im.second),
-                                                       reinterpret_cast<uint32_t*>(im.third));
+cudaError_t tc2_prepare_launch(const float* w, int K, int N, float* wt, float* wt_lo, float* w_lo, float* w_hi,
+                               bool cor16, cudaStream_t stream) {
+    if (cor16) {
+        t2_prepare16_kernel<<<dim3((N + 31) / 32, (K + 31) / 32), dim3(32, 8), 0, stream>>>(
+            w, K, N, wt, reinterpret_cast<uint16_t*>(wt_lo), reinterpret_cast<uint16_t*>(w_lo), w_hi);
+        return cudaGetLastError();
+    }
+    t2_prepare_kernel<<<dim3((N + 31) / 32, (K + 31) / 32), dim3(32, 8), 0, stream>>>(
+        w, K, N, wt, reinterpret_cast<uint32_t*>(wt_lo), reinterpret_cast<uint32_t*>(w_lo));
     return cudaGetLastError();
 }
 
-template <bool WGRAD, int BN, bool PRELO, bool C16 = false, bool F16 = false>
+template <bool WGRAD, int BN, bool PRELO, bool C16 = false>
 static cudaError_t launch2(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mblo, const CUtensorMap& mc,
                            const TcTmaArgs& a, dim3 grid, cudaStream_t stream) {
-    typedef T2Geom<WGRAD, BN, PRELO, C16, F16> G;
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(tc_tma_gemm_kernel<WGRAD, BN, PRELO, C16, F16>),
+    typedef T2Geom<WGRAD, BN, PRELO, C16> G;
+    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(tc_tma_gemm_kernel<WGRAD, BN, PRELO, C16>),
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    tc_tma_gemm_kernel<WGRAD, BN, PRELO, C16, F16><<<grid, T2_THREADS_TOTAL, G::SMEM_BYTES, stream>>>(ma, mb, mblo, mc, a);
+    tc_tma_gemm_kernel<WGRAD, BN, PRELO, C16><<<grid, T2_THREADS_TOTAL, G::SMEM_BYTES, stream>>>(ma, mb, mblo, mc, a);
     return cudaGetLastError();
 }
 
-cudaError_t tc2_rows_launch(const float* A, int M, int K_w, int N_w, const float* w, float* words, bool dgrad, float* C,
-                            const float* bias, int bias_rows, TcScheme scheme, int* error, cudaStream_t stream) {
-    const int N = dgrad ? K_w : N_w, K = dgrad ? N_w : K_w;
+cudaError_t tc2_rows_launch(const float* A, int lda, const float* Bt, const float* Bt_lo, int ldb, float* C, int ldc,
+                            const float* bias, int bias_rows, int M, int N, int K, bool cor16, int* error,
+                            cudaStream_t stream) {
     const int BN = N % 128 == 0 ? 128 : 64;
-    const TcImage im = tc_image(words, K_w, N_w);
-    // Bt and its second matrix; F16 has the pair matrix alone.
-    const float* pair = scheme == TC_F16 ? (dgrad ? im.second : im.first) : (dgrad ? im.third : im.second);
-    const float* Bt = scheme == TC_F16 ? pair : !dgrad ? im.first : scheme == TC_BF16 ? im.fourth : w;
     CUtensorMap ma, mb, mblo, mc;
-    if (!make_map(&ma, A, M, K, K, T2_BK, T2_BM, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_map(&mb, Bt, N, K, K, T2_BK, BN, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !(scheme == TC_TF32 ? make_map(&mblo, pair, N, K, K, T2_BK, BN, CU_TENSOR_MAP_SWIZZLE_128B)
-                            : make_map16(&mblo, pair, N, K, BN)) ||
-        !make_map(&mc, C, M, N, N, 32, T2_BM, CU_TENSOR_MAP_SWIZZLE_128B))
+    if (Bt_lo == nullptr) return cudaErrorInvalidValue;
+    const bool c16 = cor16;  // Bt_lo is then the bfloat16 pair matrix, N rows of 2 K halves (dense: ldb == K)
+    if (!make_map(&ma, A, M, K, lda, T2_BK, T2_BM, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_map(&mb, Bt, N, K, ldb, T2_BK, BN, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !(c16 ? make_map16(&mblo, Bt_lo, N, K, BN)
+              : make_map(&mblo, Bt_lo, N, K, ldb, T2_BK, BN, CU_TENSOR_MAP_SWIZZLE_128B)) ||
+        !make_map(&mc, C, M, N, ldc, 32, T2_BM, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
     TcTmaArgs a;
     memset(&a, 0, sizeof(a));
@@ -134,16 +128,12 @@ cudaError_t tc2_rows_launch(const float* A, int M, int K_w, int N_w, const float
     a.M = M;
     a.N = N;
     a.K = K;
-    a.ldc = N;
+    a.ldc = ldc;
     a.bias_rows = bias_rows;
     a.units = ((M + T2_BM - 1) / T2_BM) * (N / BN);
-    a.scale = im.third + (dgrad ? N_w : 0);
     a.error = error;
     const dim3 grid(a.units < 148 ? a.units : 148);
-    if (scheme == TC_F16)
-        return BN == 128 ? launch2<false, 128, true, false, true>(ma, mb, mblo, mc, a, grid, stream)
-                         : launch2<false, 64, true, false, true>(ma, mb, mblo, mc, a, grid, stream);
-    if (scheme == TC_BF16)
+    if (c16)
         return BN == 128 ? launch2<false, 128, true, true>(ma, mb, mblo, mc, a, grid, stream)
                          : launch2<false, 64, true, true>(ma, mb, mblo, mc, a, grid, stream);
     return BN == 128 ? launch2<false, 128, true>(ma, mb, mblo, mc, a, grid, stream)

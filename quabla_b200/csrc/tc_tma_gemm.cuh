@@ -52,7 +52,6 @@ constexpr int T2_BK = 32;
 constexpr int T2_THREADS = 256;                    // consumer threads
 constexpr int T2_THREADS_TOTAL = T2_THREADS + 64;  // + the loading warp and the issuing warp
 constexpr int T2_STAGES = 4;
-constexpr int T2_MAX_STAGES = 5;
 constexpr int T2_A_BYTES = T2_BM * T2_BK * 4;  // 16 KB
 
 struct TcTmaArgs {
@@ -63,7 +62,6 @@ struct TcTmaArgs {
     int bias_rows;
     int k_slice;        // WGRAD: rows per slice (multiple of T2_BK)
     int units;          // ROWS: output tiles in total
-    const float* scale; // F16: factor of every row of Bt (output column)
     int* error;
 };
 
@@ -80,23 +78,13 @@ struct TcTmaArgs {
 // The weight operand comes prepared: Bt already rounded to tf32, and a bfloat16 pair matrix whose 128-byte rows
 // hold [bf16(Bt) | bf16(lo(Bt))] of one k-tile (BN rows per stage, 128-byte swizzle).  The consumers write
 // the activation tile's tf32(x), bf16(x) and bf16(lo(x)) to tensor memory.
-//
-// F16 (with PRELO, the default): every operand is a pair of float16 parts of a scaled element.  A row of the
-// k-tile (32 elements of one row of A) and a whole row of Bt are each scaled by a power of two so that their largest
-// element lies in [2^13, 2^14); y = hi + lo with hi = f16(y), lo = f16(y - hi) then carries y to 2^-23 of itself down to
-// 2^-16 of the row's largest element and to 2^-39 of that element below.  The product lo.hi + hi.lo + hi.hi is six
-// instructions of k = 16 per k-tile (eight with C16, twelve with three tf32 products), the weight operand is the pair
-// matrix alone (16 KB per stage, no float32 tile beside it), and the row's factor multiplies the k-tile's partial on
-// its way into the float32 registers: a multiply-add where the addition was.  The factor of a row of Bt
-// multiplies the finished sum.  One thread converts a whole row of the k-tile, so that its largest element needs no
-// exchange: consumer warps 0-3 convert the even items, warps 4-7 the odd ones, all eight drain every item.
-template <bool WGRAD, int BN, bool PRELO = false, bool C16 = false, bool F16 = false>
+template <bool WGRAD, int BN, bool PRELO = false, bool C16 = false>
 struct T2Geom {
     static_assert(WGRAD != PRELO, "ROWS loads the prepared weight planes; the weight gradient has no weight operand");
-    static_assert(PRELO || !(C16 || F16), "16-bit parts need the prepared weight planes");
-    static constexpr int STAGES = F16 ? T2_MAX_STAGES : PRELO ? 3 : T2_STAGES;
+    static_assert(PRELO || !C16, "bfloat16 corrections need the prepared weight planes");
+    static constexpr int STAGES = PRELO ? 3 : T2_STAGES;
     static constexpr int B_BYTES = BN * T2_BK * 4;
-    static constexpr int STAGE_BYTES = T2_A_BYTES + B_BYTES + (PRELO && !F16 ? B_BYTES : 0);  // multiple of 1024
+    static constexpr int STAGE_BYTES = T2_A_BYTES + B_BYTES + (PRELO ? B_BYTES : 0);  // multiple of 1024
     static constexpr int LO_OFFSET = STAGES * STAGE_BYTES;
     // The first operand's hi and lo parts live in tensor memory, so only the second operand has a lo plane here
     // (and in ROWS with PRELO that one is loaded with the stage).
@@ -106,10 +94,7 @@ struct T2Geom {
     static constexpr int OUT_BYTES = T2_BM * BN * 4;
     static constexpr int OUT_OFFSET = WGRAD ? 0 : LO_OFFSET + 2 * LO_BYTES;
     static constexpr int BAR_OFFSET = LO_OFFSET + 2 * LO_BYTES + (WGRAD ? 0 : OUT_BYTES);
-    static constexpr int EXP_OFFSET = BAR_OFFSET + 128;  // F16: exponents of the rows' largest elements, four items
-    static constexpr int SCALE_OFFSET = EXP_OFFSET + (F16 ? 4 * T2_BM : 0);  // F16: factors of the rows of Bt (at most 256)
-    static constexpr int SMEM_BYTES = SCALE_OFFSET + (F16 ? 1024 : 0) + 1024;  // barriers, TMEM slot, alignment slack
-    static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
+    static constexpr int SMEM_BYTES = BAR_OFFSET + 128 + 1024;          // barriers, TMEM slot, alignment slack
     static constexpr int VECTORS = STAGE_BYTES / 16;                    // 16-byte vectors per stage
     static_assert(!WGRAD || OUT_BYTES <= LO_OFFSET, "the output staging must fit in the stage ring");
 };
@@ -135,11 +120,6 @@ __device__ __forceinline__ uint32_t t2_idesc(int N, bool mn_major) {
     uint32_t d = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(T2_BM >> 4) << 24);
     if (mn_major) d |= (1u << 15) | (1u << 16);
     return d;
-}
-
-// The same with float16 operands (kind::f16), K-major.
-__device__ __forceinline__ uint32_t t2_idesc_f16(int N) {
-    return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(T2_BM >> 4) << 24);
 }
 
 // The same with bfloat16 operands (kind::f16), K-major.
@@ -243,27 +223,23 @@ __device__ __forceinline__ void t2_arrive(uint64_t* bar) {
 //   empty[stage]  the item's MMAs completed        tcgen05.commit  -> producer (stage reusable)
 // A consumer arrives on ready[buf] of item i only after it drained item i-2, so that arrival
 // also tells the issuer that accumulator buffer `buf` is free.
-template <bool WGRAD, int BN, bool PRELO, bool C16, bool F16>
+template <bool WGRAD, int BN, bool PRELO, bool C16>
 __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
     tc_tma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_blo, const __grid_constant__ CUtensorMap map_c,
                        TcTmaArgs a) {
-    typedef T2Geom<WGRAD, BN, PRELO, C16, F16> G;
+    typedef T2Geom<WGRAD, BN, PRELO, C16> G;
     constexpr int STAGES = G::STAGES;
     extern __shared__ unsigned char t2_smem_raw[];
     // Swizzled tiles need 1024-byte alignment.
     unsigned char* const smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(t2_smem_raw) + 1023) &
                                                                  ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint64_t* const full = reinterpret_cast<uint64_t*>(smem + G::BAR_OFFSET);  // [T2_MAX_STAGES]
-    uint64_t* const empty = full + T2_MAX_STAGES;                              // [T2_MAX_STAGES]
-    uint64_t* const ready = empty + T2_MAX_STAGES;                             // [2]
+    uint64_t* const full = reinterpret_cast<uint64_t*>(smem + G::BAR_OFFSET);  // [T2_STAGES]
+    uint64_t* const empty = full + T2_STAGES;                                  // [T2_STAGES]
+    uint64_t* const ready = empty + T2_STAGES;                                 // [2]
     uint64_t* const done = ready + 2;                                          // [2]
     uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(done + 2);
-    unsigned char* const row_exp = smem + G::EXP_OFFSET;                       // [4][T2_BM]
-    float* const col_scale = reinterpret_cast<float*>(smem + G::SCALE_OFFSET);  // [N]
-    if (F16)
-        for (int i = tid; i < a.N; i += T2_THREADS_TOTAL) col_scale[i] = a.scale[i];
     // The first operand (hi and lo, 32 columns each, two buffers) sits in tensor memory behind the two accumulator
     // buffers, written there by the consumer warps, so an MMA reads only the second operand from shared memory:
     // both kernels are bound by shared-memory bandwidth (loads written, operands read by the MMAs, tiles moved by
@@ -280,7 +256,7 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
     }
     if (tid == 0) {
 #pragma unroll
-        for (int s = 0; s < T2_MAX_STAGES; ++s) {
+        for (int s = 0; s < T2_STAGES; ++s) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);
         }
@@ -328,10 +304,8 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
                 mbar_expect_tx(full + s, G::STAGE_BYTES);
                 if (!WGRAD) {
                     t2_tma_load(stage, &map_a, k0, m0, full + s);               // box {32 k, 128 rows}
-                    // F16: 64 halves per row of the pair matrix, [hi | lo] of this k-tile
-                    if (F16) t2_tma_load(stage + T2_A_BYTES, &map_blo, 2 * k0, n0, full + s);
-                    else t2_tma_load(stage + T2_A_BYTES, &map_b, k0, n0, full + s);  // box {32 k, BN rows}
-                    if (PRELO && !C16 && !F16) t2_tma_load(stage + T2_A_BYTES + G::B_BYTES, &map_blo, k0, n0, full + s);
+                    t2_tma_load(stage + T2_A_BYTES, &map_b, k0, n0, full + s);  // box {32 k, BN rows}
+                    if (PRELO && !C16) t2_tma_load(stage + T2_A_BYTES + G::B_BYTES, &map_blo, k0, n0, full + s);
                     // C16: 64 halves per row of the pair matrix, [bf16(Bt) | bf16(lo(Bt))] of this k-tile
                     if (C16) t2_tma_load(stage + T2_A_BYTES + G::B_BYTES, &map_blo, 2 * k0, n0, full + s);
                 } else {
@@ -366,19 +340,6 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
                 // of an MN-major atom.  The small correction products go first (they add onto a
                 // small accumulator without loss), the full-magnitude products last.
                 constexpr uint32_t STEP = WGRAD ? 1024 : 32;
-                if (F16) {
-                    // Operand buffer b: hi parts in columns 0-15 (two k per column), lo parts in 16-31; sixteen k
-                    // (32 bytes of a pair-matrix row: hi in bytes 0-63, lo in 64-127) per instruction.
-                    const uint32_t idesc16 = t2_idesc_f16(BN), ta = tmem_base + (uint32_t)(A_COL0 + b * 64);
-#pragma unroll
-                    for (int kc = 0; kc < T2_BK / 16; ++kc) {
-                        t2_mma16_tmem_a(dst, ta + 16 + kc * 8, t2_desc_kmajor(bh + kc * 32), idesc16, kc == 0 ? 0u : 1u);
-                        t2_mma16_tmem_a(dst, ta + kc * 8, t2_desc_kmajor(bh + 64 + kc * 32), idesc16, 1u);
-                    }
-#pragma unroll
-                    for (int kc = 0; kc < T2_BK / 16; ++kc)
-                        t2_mma16_tmem_a(dst, ta + kc * 8, t2_desc_kmajor(bh + kc * 32), idesc16, 1u);
-                }
                 if (C16) {
                     // Operand buffer b: x in columns 0-31, bf16(x) in 32-47, bf16(lo(x)) in 48-63; sixteen k
                     // (32 bytes of a weight-plane row) per instruction.
@@ -393,7 +354,7 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
                     }
                 }
 #pragma unroll
-                for (int kb = 0; kb < (C16 || F16 ? 0 : T2_BK / 8); ++kb) {
+                for (int kb = 0; kb < (C16 ? 0 : T2_BK / 8); ++kb) {
                     const uint32_t o = kb * STEP;
                     const uint32_t ta = tmem_base + (uint32_t)(A_COL0 + b * 64 + kb * 8);  // hi; lo is 32 columns on
                     if (WGRAD) {
@@ -405,7 +366,7 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
                     }
                 }
 #pragma unroll
-                for (int kb = 0; kb < (F16 ? 0 : T2_BK / 8); ++kb) {
+                for (int kb = 0; kb < T2_BK / 8; ++kb) {
                     const uint32_t o = kb * STEP;
                     t2_mma_tmem_a(dst, tmem_base + (uint32_t)(A_COL0 + b * 64 + kb * 8),
                                   WGRAD ? t2_desc_mnmajor(bh + o) : t2_desc_kmajor(bh + o), idesc, 1u);
@@ -428,14 +389,6 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
 #endif
         // Partial of item q: wait for its instructions, add its buffer into the registers.
         auto drain = [&](int q) {
-            float factor = 1.0f;
-            if (F16) {
-                // Orders the converting warps' row exponents before the read; here its latency lies under the wait for the MMAs.
-                mbar_wait(ready + (q & 1), (uint32_t)((q >> 1) & 1), a.error);
-                // 2^(e - 127 - 13) of the row, and the 2^-13 of the weight's scaling here rather than at the end,
-                // which keeps the running sum at the size of the result over the weights' size.
-                factor = __uint_as_float(((uint32_t)row_exp[(q & 3) * T2_BM + trow] - 13u) << 23) * 0x1p-13f;
-            }
             mbar_wait(done + (q & 1), (uint32_t)((q >> 1) & 1), a.error);
             QB_T2_PHASE(4);  // wait for the MMAs
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -446,8 +399,7 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             QB_T2_PHASE(5);  // tensor-memory loads
 #pragma unroll
-            for (int i = 0; i < NH; ++i)
-                acc[i] = F16 ? fmaf(__uint_as_float(v[i]), factor, acc[i]) : acc[i] + __uint_as_float(v[i]);
+            for (int i = 0; i < NH; ++i) acc[i] += __uint_as_float(v[i]);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         };
         // Output of unit u: registers -> staging in shared memory (boxes of [128 rows][32 columns],
@@ -468,13 +420,6 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
                 for (int c = 0; c < 8; ++c) {
                     float4 v = make_float4(acc[j * 32 + 4 * c], acc[j * 32 + 4 * c + 1], acc[j * 32 + 4 * c + 2],
                                            acc[j * 32 + 4 * c + 3]);
-                    if (F16) {
-                        const float4 sv = *reinterpret_cast<const float4*>(col_scale + n0 + half * NH + j * 32 + 4 * c);
-                        v.x *= sv.x;
-                        v.y *= sv.y;
-                        v.z *= sv.z;
-                        v.w *= sv.w;
-                    }
                     if (biased) {
                         const float4 bv = *reinterpret_cast<const float4*>(a.bias + n0 + half * NH + j * 32 + 4 * c);
                         v.x += bv.x;
@@ -507,38 +452,10 @@ __global__ void __launch_bounds__(T2_THREADS_TOTAL, 1)
             const int s = it % STAGES, b = it & 1;
             const unsigned char* hi = smem + s * G::STAGE_BYTES;
             unsigned char* lo = smem + G::LO_OFFSET + b * G::LO_BYTES;
-            if (!F16 || b == half) mbar_wait(full + s, (uint32_t)((it / STAGES) & 1), a.error);
+            mbar_wait(full + s, (uint32_t)((it / STAGES) & 1), a.error);
             QB_T2_PHASE(0);  // wait for the loads
             // The lo buffer b was last read by item it-2, which this thread has drained.
-            if (F16) {
-                // Item it's converting warps: this thread's row (its accumulator lane) of the activation tile, all 32 k,
-                // read through the 128-byte swizzle.
-                if (b == half) {
-                    uint32_t x[32], largest = 0;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(hi + trow * 128 + ((c ^ (trow & 7)) << 4));
-                        x[4 * c + 0] = v.x; x[4 * c + 1] = v.y; x[4 * c + 2] = v.z; x[4 * c + 3] = v.w;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) largest = max(largest, x[i] & 0x7fffffffu);
-                    float inverse;
-                    block_scale(largest, &inverse);
-                    uint32_t h16[16], l16[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        split_f16(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]), inverse, h16[i], l16[i]);
-                    const uint32_t ta = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(A_COL0 + b * 64);
-                    t2_store16(ta, h16);
-                    t2_store16(ta + 16, l16);
-                    // Slot it & 3 was last read in the drain of item it-4, which every thread has behind it: each
-                    // arrived for item it-2, whose instructions have completed, after that drain.
-                    row_exp[(it & 3) * T2_BM + trow] = (unsigned char)max(largest >> 23, 14u);
-                    QB_T2_PHASE(1);
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    QB_T2_PHASE(2);
-                }
-            } else if (!WGRAD) {
+            if (!WGRAD) {
                 // Activation tile: this thread's row (its accumulator lane), 16 of the 32 k (by column
                 // half), read through the 128-byte swizzle (chunk c of row r sits at c ^ (r & 7)) and
                 // written, hi and lo, to the operand buffer b in tensor memory.
@@ -685,36 +602,6 @@ __global__ void t2_prepare16_kernel(const float* __restrict__ w, int K, int N, f
     for (int r = threadIdx.y; r < 32; r += blockDim.y) {
         const int n = n0 + r, k = k0 + threadIdx.x;
         if (n < N && k < K) split(tile[threadIdx.x][r], wt + (size_t)n * K + k, wt16, (size_t)n, K, k);
-    }
-}
-
-// Mean relative loss of a k-tile's six truncating accumulations, put back into the weight operand (its lo part has room for
-// it; the finished float32 sum has not).  Measured as <error, exact> / <exact, exact> over 65,536 x 256 products against
-// float64: -5.6e-8 for normal operands, -8.2e-8 for positive ones, independent of K; with it the two are 0 and -2e-8.
-constexpr float T2_TRUNCATION = 6.0e-8f;
-
-// The weight operands of the F16 kernels: one warp per row of W^T (the forward product's Bt) or of W (the data
-// gradient's), scaled by its largest element.  Pair rows hold, per 32 contraction elements, 32 hi then 32 lo parts.
-__global__ void t2_prepare_f16_kernel(const float* __restrict__ w, int K, int N, __half* __restrict__ pair_t,
-                                      __half* __restrict__ pair, float* __restrict__ scale_t, float* __restrict__ scale) {
-    const int row = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (row >= N + K) return;
-    const bool transposed = row < N;
-    const int r = transposed ? row : row - N, inner = transposed ? K : N;
-    const float* const src = transposed ? w + r : w + (size_t)r * N;
-    const size_t step = transposed ? (size_t)N : 1;
-    uint32_t largest = 0;
-    for (int c = lane; c < inner; c += 32) largest = max(largest, __float_as_uint(src[c * step]) & 0x7fffffffu);
-    largest = __reduce_max_sync(0xffffffffu, largest);
-    float inverse;
-    const float factor = block_scale(largest, &inverse);
-    if (lane == 0) (transposed ? scale_t : scale)[r] = factor * 0x1p13f;  // the kernel took 2^-13 out already
-    __half* const dst = (transposed ? pair_t : pair) + (size_t)r * 2 * inner;
-    for (int c = lane; c < inner; c += 32) {
-        const float y = src[c * step] * inverse;
-        const __half hi = __float2half_rn(y);
-        dst[2 * (c - lane) + lane] = hi;
-        dst[2 * (c - lane) + 32 + lane] = __float2half_rn(fmaf(y, T2_TRUNCATION, y - __half2float(hi)));
     }
 }
 
