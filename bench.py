@@ -389,10 +389,10 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
         gemm_ns = plan.query(_lib.Q_GEMM_NANOSECONDS)
         gemm_launches = max(1, plan.query(_lib.Q_GEMM_LAUNCHES))
         gemm_flops = float(plan.query(_lib.Q_GEMM_FLOPS))
-        # Tensor-pipe work of the same launches at the bf16 rate: 3 passes per FLOP for three float16 products, 6 for
-        # three tf32 ones, 4 for a tf32 product with two bf16 corrections (0 off the tensor pipe).
+        # Tensor-pipe work of the same launches at the bf16 rate: 6 passes per FLOP for a product made of three
+        # tf32 instructions, 4 where the two correction products are bf16 instructions (0 off the tensor pipe).
         pipe_flops = float(plan.query(_lib.Q_GEMM_PIPE_FLOPS))
-        kernel = {"name": "tc_tma_gemm_kernel (tcgen05: three float16 or tf32 products)" if engine == 3 else
+        kernel = {"name": "tc_tma_gemm_kernel (tcgen05: tf32 product + two correction products)" if engine == 3 else
                   "dmma_gemm_kernel (FP64 MMA) / gemm_kernel" if dtype_name == "f64" else "gemm_kernel",
                   "launches_per_step": int(gemm_launches), "us_per_launch": gemm_ns * 1e-3 / gemm_launches,
                   "flops_per_launch": gemm_flops / gemm_launches, "us_per_step": gemm_ns * 1e-3,
@@ -448,8 +448,9 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
     step_flops = (w.flops_per_point(streams) * w.interior_points
                   + sum(w.flops_per_point(s) * n for n, s in w.extra))
     if dtype_name == "f32":
-        # Split float32 on the tensor pipe: three float16 products cost 3 bf16-rate passes per FLOP and three tf32
-        # products, at half that rate, 6; the denominator is the bf16 rate over the passes the timed launches actually execute.  The burst figure
+        # Split float32 on the tensor pipe: a tf32 instruction runs at half the bf16 rate, so three tf32 products
+        # cost 6 bf16-rate passes per FLOP and a tf32 product with two bf16 correction products costs 4; the
+        # denominator is the bf16 rate over the passes the timed launches actually execute.  The burst figure
         # for kernels timed alone in a short step, the sustained one (seconds-long loop under the power cap)
         # when the timed kernels keep the GPU busy for tens of milliseconds per step.
         sustained = kernel["us_per_step"] > 2e4 and "bf16_tflops_sustained" in peaks
@@ -492,9 +493,18 @@ def parity_step(rig: Rig, name: str) -> dict:
     from quabla_b200._transforms import CompiledLoss
 
     w = workloads.make(name, PARITY_POINTS)
-    trainer, plan = rig.trainer(w, rig.shard(w))
-    plan.execute()
-    outputs = plan.outputs()
+    # The timed step's tcgen05 GEMMs run the scheme the library picks for large launches (bfloat16 correction
+    # products); a launch of this size would get the other one, so the parity step asks for the timed one.
+    forced = "QB200_TC_COR" not in os.environ
+    if forced:
+        os.environ["QB200_TC_COR"] = "bf16"
+    try:
+        trainer, plan = rig.trainer(w, rig.shard(w))
+        plan.execute()
+        outputs = plan.outputs()
+    finally:
+        if forced:
+            del os.environ["QB200_TC_COR"]
     dtype_name = "f32" if np.dtype(w.dtype) == np.float32 else "f64"
     tolerance = PARITY_TOLERANCE[dtype_name]
     worst = 0.0

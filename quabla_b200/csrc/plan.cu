@@ -1148,7 +1148,7 @@ qb200_status Plan<float>::tc_setup() {
         tc_fwd_[l] = tc_rows_ok(N, K);
         tc_bwd_[l] = l > 0 && tc_rows_ok(K, N);
         tc_wgrad_[l] = tc_wgrad_ok(K, N);
-        if (tc_fwd_[l] || tc_bwd_[l]) QB_TRY(dev_alloc(&tc_image_[l], tc_image_words(K, N)));
+        if (tc_fwd_[l] || tc_bwd_[l]) QB_TRY(dev_alloc(&tc_image_[l], 2 * tc_image_words(K, N)));  // one image per scheme
         tc_any_ = tc_any_ || tc_fwd_[l] || tc_bwd_[l] || tc_wgrad_[l];
     }
     return QB200_OK;
