@@ -871,12 +871,12 @@ qb200_status Plan<T>::bind_many(const int32_t* slots, const void* const* hosts, 
         QB_CUDA(cudaStreamWaitEvent(stream, ev_inputs_, 0));
     }
     for (int i = 0; i < n;) {
-        // A run of slots that follow one another in the arena and fit one block together: one transfer (the
-        // padding between them, which stays zero, included).
+        // A run of slots that follow one another and fit one block together: one transfer, the padding between them,
+        // which stays zero, included.  Successive slots only: a short leaf left out fits between two others as well.
         const size_t first = offset_of(slots[i]);
         size_t end = first + count_of(slots[i]);
         int j = i + 1;
-        while (j < n && offset_of(slots[j]) >= end && offset_of(slots[j]) - end < 256 / sizeof(T) &&
+        while (j < n && slots[j] == slots[j - 1] + 1 &&
                (offset_of(slots[j]) + count_of(slots[j]) - first) * sizeof(T) <= STAGING_BLOCK_BYTES) {
             end = offset_of(slots[j]) + count_of(slots[j]);
             ++j;

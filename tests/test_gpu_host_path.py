@@ -57,6 +57,25 @@ def test_wrong_slots_and_sizes_upload_nothing(cuda_device):
     assert caught.value.status == _lib.NOT_BOUND
 
 
+@pytest.mark.parametrize("name", ["poisson1d", "poisson2d"])
+@pytest.mark.parametrize("choose", [lambda n: range(0, n, 2), lambda n: range(1, n, 2), lambda n: reversed(range(n)),
+                                    lambda n: [2, 1, 3], lambda n: [1, 0, n - 1], lambda n: [0, 0, 1]],
+                         ids=["even", "odd", "reversed", "one before its predecessor", "last input", "twice"])
+def test_any_choice_and_order_of_slots_leaves_the_others_alone(cuda_device, name, choose):
+    # A bias is shorter than the padding a run of slots may contain: it must not be taken for padding.
+    w, compiled, inputs = traced(name, 64)
+    plan = Plan(compiled.spec, 0)
+    names = [n for n, _, _ in compiled.spec.parameters] + [n for n, _, _, _ in compiled.spec.inputs]
+    expected = {n: np.asarray(inputs[n]) + 1 for n in names}  # no zeros, biases included
+    plan.bind_many([plan.slot(n) for n in names], [expected[n] for n in names])
+    chosen = list(choose(len(names)))
+    for slot in chosen:
+        expected[names[slot]] = expected[names[slot]] * 2
+    plan.bind_many(chosen, [expected[names[slot]] for slot in chosen])
+    for n in names:
+        np.testing.assert_array_equal(plan.read_input(n, expected[n].shape), expected[n], err_msg=n)
+
+
 def test_read_back_buffers_are_recycled_and_bounded(cuda_device):
     first = _host.empty(1000, np.dtype(np.float32))
     address = first.__array_interface__["data"][0]
