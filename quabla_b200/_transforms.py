@@ -62,14 +62,17 @@ def _normalize_argnums(argnums, count: int) -> tuple[int, ...]:
 
 
 # Shape of an argument as last seen, for calls that repeat it: ("dict", keys, children), ("list" | "tuple", children),
-# ("array", shape, dtype), ("none",) or ("static", value).
+# ("array", shape, dtype), ("none",) or ("static", value).  None where any node is of another container type (a subclass
+# of dict, list or tuple): such trees are flattened on every call.
 def _template(node):
-    if isinstance(node, dict):
-        keys = sorted(node)
-        return ("dict", tuple(keys), tuple(_template(node[k]) for k in keys)) if type(node) is dict else None
-    if isinstance(node, (list, tuple)) and not hasattr(node, "_fields"):
-        kind = {list: "list", tuple: "tuple"}.get(type(node))
-        return (kind, tuple(_template(child) for child in node)) if kind else None
+    if isinstance(node, dict) or (isinstance(node, (list, tuple)) and not hasattr(node, "_fields")):
+        if type(node) not in (dict, list, tuple):
+            return None
+        keys = tuple(sorted(node)) if type(node) is dict else ()
+        children = tuple(_template(child) for child in ([node[k] for k in keys] if type(node) is dict else node))
+        if any(child is None for child in children):
+            return None
+        return ("dict", keys, children) if type(node) is dict else (type(node).__name__, children)
     if node is None:
         return ("none",)
     if _is_array(node):
@@ -79,8 +82,6 @@ def _template(node):
 
 def _match(template, node, leaves: list) -> bool:
     """Appends the array leaves of `node` in flattening order; False when it is not of the template's shape."""
-    if template is None:
-        return False
     kind = template[0]
     if kind == "array":
         if type(node) is not np.ndarray or node.shape != template[1] or node.dtype != template[2]:
@@ -225,13 +226,13 @@ class CompiledLoss:
             return False
         leaves: list = []
         for template, arg in zip(self._templates, args):
-            if not _match(template, arg, leaves):
+            if template is None or not _match(template, arg, leaves):
                 return False
         self.plan.bind_many([slot for _, slot in self._bound], [leaves[at] for at, _ in self._bound])
         return True
 
-    def gradients(self, args: tuple):
-        """(value, grads) with grads shaped like the differentiated arguments."""
+    def gradients(self, args: tuple, same: bool = False):
+        """(value, grads) with grads shaped like the differentiated arguments.  `same`: `bind_if_same` took them."""
         outputs = self.plan.outputs()
         value = outputs[0]
         flat = []
@@ -245,7 +246,7 @@ class CompiledLoss:
         it = iter(flat)
         trees = []
         for index in self.argnums:
-            if self._templates[index] is not None:
+            if same:
                 trees.append(_rebuild(self._templates[index], it))
                 continue
             leaves, rebuild = tr.flatten(args[index])
@@ -272,17 +273,17 @@ class _Transform:
         self._latest = None  # (device ordinal, cache key, compiled loss) of the last call
 
     def _bound(self, args: tuple, argnums_of, device_ordinal: int):
-        """The compiled loss for these arguments, with them bound.  A call shaped like the last one skips the
-        signature."""
+        """(compiled loss, same): the compiled loss for these arguments, with them bound.  A call shaped like the last
+        one skips the signature (same); other container types around the same leaves share a compiled loss."""
         latest = self._latest
         if latest is not None and latest[0] == device_ordinal and latest[1] in self._cache and latest[2].bind_if_same(args):
-            return latest[2]
+            return latest[2], True
         argnums = argnums_of(len(args))
         key = _signature(args, argnums, device_ordinal)
         compiled = self._lookup(key, lambda: CompiledLoss(self._fun, args, argnums, device_ordinal))
         compiled.bind(args)
         self._latest = (device_ordinal, key, compiled)
-        return compiled
+        return compiled, False
 
     def _lookup(self, key, build):
         found = self._cache.get(key)
@@ -313,9 +314,9 @@ class _ValueAndGrad(_Transform):
         return self._run(args, 0)
 
     def _run(self, args: tuple, device_ordinal: int):
-        compiled = self._bound(args, lambda count: _normalize_argnums(self._argnums, count), device_ordinal)
+        compiled, same = self._bound(args, lambda count: _normalize_argnums(self._argnums, count), device_ordinal)
         compiled.plan.execute()
-        value, trees = compiled.gradients(args)
+        value, trees = compiled.gradients(args, same)
         grads = trees[0] if isinstance(self._argnums, int) else tuple(trees)
         return grads if self._mode == "grad" else (value, grads)
 
@@ -324,7 +325,7 @@ class _LossOnly(_Transform):
     """jit(loss): forward evaluation of the loss on the device."""
 
     def _run(self, args: tuple, device_ordinal: int):
-        return self._bound(args, lambda count: (0,), device_ordinal).plan.loss()
+        return self._bound(args, lambda count: (0,), device_ordinal)[0].plan.loss()
 
     def __call__(self, *args):
         if _any_traced(args):
