@@ -181,22 +181,32 @@ class Plan:
         """Bind from a host address (for example a pinned staging buffer)."""
         _lib.check(self._lib.qb200_plan_bind(self._handle, name.encode(), C.c_void_p(address), nbytes))
 
-    def slot(self, name: str) -> int:
+    def slot(self, name: str, *default) -> int:
         """Number of a parameter or data input in `bind_many`."""
         slots = getattr(self, "_slots", None)
         if slots is None:
             names = [n for n, _, _ in self.spec.parameters] + [n for n, _, _, _ in self.spec.inputs]
             slots = self._slots = {n: i for i, n in enumerate(names)}
-        return slots[name]
+        return slots.get(name, *default) if default else slots[name]
 
     def bind_many(self, slots: list[int], values: list) -> None:
         """Several inputs in one call: arrays of the plan dtype (anything else is converted), by slot."""
         n = len(slots)
-        arrays = [v if v.dtype == self.dtype and v.flags.c_contiguous else self._host(v) for v in values]
+        # Only an array owns the memory behind its address (a NumPy scalar's is gone with the expression).
+        arrays = [v if isinstance(v, np.ndarray) and v.dtype == self.dtype and v.flags.c_contiguous else self._host(v)
+                  for v in values]
         _lib.check(self._lib.qb200_plan_bind_many(
             self._handle, (C.c_int32 * n)(*slots),
             (C.c_void_p * n)(*[a.__array_interface__["data"][0] for a in arrays]),
             (C.c_size_t * n)(*[a.nbytes for a in arrays]), n))
+
+    def bind_named(self, inputs: dict) -> None:
+        """Anything `bind` takes, by name: parameters and data inputs in one call, other names one by one."""
+        known = [name for name in inputs if self.slot(name, None) is not None]
+        for name in inputs:
+            if name not in known:
+                self.bind(name, inputs[name])
+        self.bind_many([self.slot(name) for name in known], [inputs[name] for name in known])
 
     def execute(self) -> None:
         _lib.check(self._lib.qb200_plan_execute(self._handle))

@@ -226,7 +226,7 @@ class CudaTrainerExecutor:
 
     def _bind(self, inputs: dict | None) -> None:
         if inputs:
-            self._plan.bind_many([self._plan.slot(name) for name in inputs], list(inputs.values()))
+            self._plan.bind_named(inputs)
 
     def step(self, inputs: dict | None = None) -> None:
         config = self._config()
