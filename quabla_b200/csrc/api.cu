@@ -416,8 +416,11 @@ qb200_status qb200_plan_train_step(qb200_plan* plan, const qb200_opt_config* con
 qb200_status qb200_host_alloc(size_t nbytes, void** out) {
     if (out == nullptr || nbytes == 0) return fail(QB200_INVALID, "host_alloc needs a size and an output");
     *out = nullptr;
-    QB_CUDA(cudaHostAlloc(out, nbytes, cudaHostAllocPortable));
-    return QB200_OK;
+    const cudaError_t e = cudaHostAlloc(out, nbytes, cudaHostAllocPortable);
+    if (e == cudaSuccess) return QB200_OK;
+    cudaGetLastError();  // the caller goes on with ordinary memory: the next launch must not find this error
+    *out = nullptr;
+    return fail(QB200_CUDA_ERROR, "page-locking %zu bytes failed: %s", nbytes, cudaGetErrorString(e));
 }
 
 void qb200_host_free(void* host) {

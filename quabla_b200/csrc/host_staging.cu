@@ -47,34 +47,40 @@ void staging_detach(int device) {
     if (--p.users == 0) p.clear();
 }
 
+// Null when page-locked memory or an event is not to be had; no error is left pending.
+static std::unique_ptr<StagingBlock> new_block() {
+    std::unique_ptr<StagingBlock> fresh(new StagingBlock());
+    void* raw = nullptr;
+    if (cudaHostAlloc(&raw, STAGING_BLOCK_BYTES, cudaHostAllocPortable) == cudaSuccess) {
+        if (cudaEventCreateWithFlags(&fresh->done, cudaEventDisableTiming) == cudaSuccess) {
+            fresh->host = static_cast<unsigned char*>(raw);
+            return fresh;
+        }
+        cudaFreeHost(raw);
+    }
+    cudaGetLastError();
+    return nullptr;
+}
+
 cudaError_t staging_acquire(int device, int limit, StagingBlock** out) {
+    *out = nullptr;
     StagingBlock* block = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         Pool& p = pool(device);
         const bool oldest_done = !p.idle.empty() && (!p.idle.front()->queued || cudaEventQuery(p.idle.front()->done) == cudaSuccess);
         if (!oldest_done && (int)p.blocks.size() < (p.idle.empty() ? STAGING_BLOCKS : limit)) {
-            std::unique_ptr<StagingBlock> fresh(new StagingBlock());
-            void* raw = nullptr;
-            cudaError_t e = cudaHostAlloc(&raw, STAGING_BLOCK_BYTES, cudaHostAllocPortable);
-            if (e != cudaSuccess) return e;
-            e = cudaEventCreateWithFlags(&fresh->done, cudaEventDisableTiming);
-            if (e != cudaSuccess) {
-                cudaFreeHost(raw);
-                return e;
+            if (std::unique_ptr<StagingBlock> fresh = new_block()) {
+                *out = fresh.get();
+                p.blocks.push_back(std::move(fresh));
+                return cudaSuccess;
             }
-            fresh->host = static_cast<unsigned char*>(raw);
-            *out = fresh.get();
-            p.blocks.push_back(std::move(fresh));
-            return cudaSuccess;
         }
-        if (!p.idle.empty()) {
-            block = p.idle.front();
-            p.idle.pop_front();
-        }
+        if (p.idle.empty()) return cudaSuccess;  // none to be had, or all in other callers' hands at this instant
+        block = p.idle.front();
+        p.idle.pop_front();
     }
     *out = block;
-    if (block == nullptr) return cudaSuccess;  // every block is in some other caller's hands at this instant
     const cudaError_t e = block->queued ? cudaEventSynchronize(block->done) : cudaSuccess;
     block->queued = false;
     return e;

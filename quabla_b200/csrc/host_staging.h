@@ -29,7 +29,8 @@ struct StagingBlock {
 void staging_attach(int device);
 void staging_detach(int device);
 // A block no transfer is reading; while all have one, a new block up to `limit` of them, else the oldest after its transfer.
-// *out is null when all blocks are in other callers' hands, and the caller then copies without staging.
+// *out is null when all blocks are in other callers' hands or no memory can be page-locked, and the caller then copies
+// without staging.
 cudaError_t staging_acquire(int device, int limit, StagingBlock** out);
 // Transfers from `block` queued on `stream` so far must finish before it is handed out again.
 cudaError_t staging_release(int device, StagingBlock* block, cudaStream_t stream);

@@ -1,6 +1,8 @@
 """Uploads through the pinned staging blocks, captured step sequences and flat read-backs against the per-name calls
 and single launches they stand for: the same bits."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -74,6 +76,18 @@ def test_any_choice_and_order_of_slots_leaves_the_others_alone(cuda_device, name
     plan.bind_many(chosen, [expected[names[slot]] for slot in chosen])
     for n in names:
         np.testing.assert_array_equal(plan.read_input(n, expected[n].shape), expected[n], err_msg=n)
+
+
+def test_a_refused_page_lock_leaves_the_next_step_alone(cuda_device):
+    # More host memory than any machine has: refused on the host, and not the next launch's error.
+    w, compiled, inputs = traced("poisson1d", 64)
+    plan = Plan(compiled.spec, 0)
+    for n, value in inputs.items():
+        plan.bind(n, value)
+    out = C.c_void_p()
+    assert _lib.load().qb200_host_alloc(1 << 60, C.byref(out)) == _lib.CUDA_ERROR and out.value is None
+    plan.execute()
+    assert np.isfinite(plan.loss())
 
 
 def test_read_back_buffers_are_recycled_and_bounded(cuda_device):
