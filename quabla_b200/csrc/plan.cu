@@ -14,6 +14,7 @@
 #include "host_staging.h"
 #include "layer_kernels.cuh"
 #include "point_kernels.cuh"
+#include "step_graph.h"
 #include "tc_gemm.h"
 
 namespace qb {
@@ -223,12 +224,6 @@ class Plan final : public qb200_plan {
     }
     qb200_status check_bound() const;
     qb200_status refresh_tables();
-    // The kernel sequence of a step (or of a loss evaluation) as a CUDA graph: see run().
-    struct StepGraph {
-        int uses = 0;
-        cudaGraphExec_t exec = nullptr;
-        int64_t launches = 0;
-    };
     void drop_graphs() {
         for (auto& g : graphs_)
             if (g.second.exec != nullptr) cudaGraphExecDestroy(g.second.exec);
@@ -312,7 +307,7 @@ class Plan final : public qb200_plan {
     T* d_ct_ = nullptr;
     T* h_loss_ = nullptr;      // mapped host word that a loss evaluation writes
     T* d_loss_only_ = nullptr; // the same as the device sees it
-    std::map<uint32_t, StepGraph> graphs_;
+    std::map<uint32_t, StepGraph> graphs_;  // the kernel sequence of a step and of a loss evaluation: see run()
     // Large batches are uploaded on a stream of their own, under the previous step's kernels (which read the point
     // tables, not the inputs); ev_inputs_ is the last point of the main stream that touched the inputs.
     cudaStream_t copy_stream_ = nullptr;
@@ -1519,31 +1514,18 @@ qb200_status Plan<T>::run(bool forward_only) {
     QB_TRY(check_bound());
     QB_TRY(refresh_tables());
     StepGraph& g = graphs_[forward_only ? 1 : 0];
-    if (timers_ || g.uses == 0 || g.launches > GRAPH_MAX_LAUNCHES) {
-        const int64_t before = launches_;
+    const int64_t before = launches_;
+    if (g.uses > 0 && g.exec == nullptr && !timers_ && !g.single && g.launches <= GRAPH_MAX_LAUNCHES) {
+        capturing_ = true;
+        capture_sequence(stream_, g, [&] { return enqueue(forward_only) == QB200_OK; });
+        capturing_ = false;
+        launches_ = before;
+    }
+    if (timers_ || g.exec == nullptr) {
         QB_TRY(enqueue(forward_only));
         ++g.uses;
         g.launches = launches_ - before;
         return QB200_OK;
-    }
-    if (g.exec == nullptr) {
-        const int64_t before = launches_;
-        QB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        capturing_ = true;
-        const qb200_status st = enqueue(forward_only);
-        capturing_ = false;
-        cudaGraph_t graph = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(stream_, &graph);
-        launches_ = before;
-        if (st != QB200_OK) {
-            if (graph != nullptr) cudaGraphDestroy(graph);
-            return st;
-        }
-        QB_CUDA(e);
-        const cudaError_t made = cudaGraphInstantiate(&g.exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (made != cudaSuccess) g.exec = nullptr;
-        QB_CUDA(made);
     }
     QB_CUDA(cudaGraphLaunch(g.exec, stream_));
     launches_ += g.launches;
@@ -1552,6 +1534,7 @@ qb200_status Plan<T>::run(bool forward_only) {
 
 template <typename T>
 qb200_status Plan<T>::enqueue(bool forward_only) {
+    if (!lanes_.empty()) select_lane(0);  // also after a sequence that failed half way
     if (!forward_only) {
         timer_used_ = 0;
         timer_flops_ = 0.0;

@@ -16,8 +16,8 @@ RUNTIME = r"""
 #include <cstdio>
 #include <cstdlib>
 static cudaError_t last = cudaSuccess;
-static bool fail_alloc, fail_event;
-static int allocated, queries_done;
+static bool fail_alloc, fail_event, fail_begin, fail_end, fail_instantiate;
+static int allocated, capturing, graphs, queries_done;
 static cudaError_t result(bool failed, cudaError_t e) { if (failed) last = e; return failed ? e : cudaSuccess; }
 extern "C" {
 cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
@@ -31,6 +31,20 @@ cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t) { return queries_done ? cudaSuccess : cudaErrorNotReady; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
+    if (!fail_begin) ++capturing;
+    return result(fail_begin, cudaErrorUnknown);
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
+    --capturing;
+    if (!fail_end) { *g = (cudaGraph_t)1; ++graphs; }
+    return result(fail_end, cudaErrorStreamCaptureInvalidated);
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+    *e = (cudaGraphExec_t)1;
+    return result(fail_instantiate, cudaErrorMemoryAllocation);
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t) { --graphs; return cudaSuccess; }
 }
 #define CHECK(c) do { if (!(c)) { printf("line %d: %s\n", __LINE__, #c); return 1; } } while (0)
 """
@@ -61,7 +75,27 @@ int main() {
 }
 """
 
-@pytest.mark.parametrize("program", [STAGING], ids=["staging blocks"])
+GRAPHS = r"""
+#include "step_graph.h"
+using namespace qb;
+int main() {
+    for (int failing = 0; failing < 5; ++failing) {
+        fail_begin = failing == 1;
+        fail_end = failing == 2;
+        fail_instantiate = failing == 3;
+        StepGraph g;
+        int queued = 0;
+        const bool made = capture_sequence((cudaStream_t)1, g, [&] { ++queued; return failing != 4; });
+        CHECK(made == (failing == 0) && g.single == (failing != 0) && (g.exec != nullptr) == (failing == 0));
+        CHECK(queued == (failing != 1) && capturing == 0 && graphs == 0);
+        CHECK(cudaGetLastError() == cudaSuccess);
+    }
+    return 0;
+}
+"""
+
+
+@pytest.mark.parametrize("program", [STAGING, GRAPHS], ids=["staging blocks", "captured sequences"])
 def test_failing_runtime_calls_leave_the_plain_path(tmp_path, program):
     source = tmp_path / "program.cpp"
     source.write_text(RUNTIME + program)
