@@ -4,12 +4,13 @@ A device-to-host copy into fresh pageable memory pays for the driver's bounce bu
 (1.3 MB of gradients: 0.57 ms); into a page-locked block it runs at link speed (0.03 ms).  Arrays handed out here are views of such
 a block; when the last one is gone the block goes back to the pool.  The pool is shared by all plans and threads and
 bounded: beyond `LIMIT` bytes in use the caller gets ordinary memory, and at most `IDLE_LIMIT` bytes stay page-locked
-without an owner.
+without an owner.  A forked child has copies of the arrays, as of any other memory; its own arrays are ordinary ones.
 """
 
 from __future__ import annotations
 
 import ctypes as C
+import os
 import threading
 
 import numpy as np
@@ -24,6 +25,17 @@ _lock = threading.RLock()  # a collection inside a locked section may run _Block
 _idle: dict[int, list[int]] = {}   # block size -> addresses
 _total = 0                         # page-locked bytes, handed out or idle
 _idle_bytes = 0
+_forked = False                    # in a child: the blocks are the parent's, the CUDA runtime is not usable
+
+
+def _after_fork() -> None:
+    global _lock, _forked
+    _lock = threading.RLock()  # another thread of the parent may have held it
+    _forked = True
+    _idle.clear()
+
+
+os.register_at_fork(after_in_child=_after_fork)
 
 
 class _Block:
@@ -42,6 +54,8 @@ class _Block:
 
 def _give_back(address: int, size: int) -> None:
     global _total, _idle_bytes
+    if _forked:
+        return
     with _lock:
         if _idle_bytes + size <= IDLE_LIMIT:
             _idle.setdefault(size, []).append(address)
@@ -54,6 +68,8 @@ def _give_back(address: int, size: int) -> None:
 def empty(count: int, dtype: np.dtype) -> np.ndarray:
     """An uninitialised one-dimensional array, page-locked when the pool has room."""
     global _total, _idle_bytes
+    if _forked:
+        return np.empty((count,), dtype=dtype)
     size = _SMALLEST
     while size < count * dtype.itemsize:
         size *= 2

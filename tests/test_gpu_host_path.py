@@ -2,6 +2,8 @@
 and single launches they stand for: the same bits."""
 
 import ctypes as C
+import os
+import signal
 
 import numpy as np
 import pytest
@@ -104,6 +106,46 @@ def test_read_back_buffers_are_recycled_and_bounded(cuda_device):
     assert _host._total <= _host.LIMIT
     del held
     assert _host._idle_bytes <= _host.IDLE_LIMIT
+
+
+@pytest.mark.filterwarnings("ignore::DeprecationWarning")  # fork beside threads: the child only compares and exits
+def test_a_forked_child_has_arrays_of_its_own(cuda_device):
+    # As when a child writes a checkpoint while its parent trains on; the child makes no CUDA call.
+    w, compiled, inputs = traced("poisson2d", 64)
+    plan = Plan(compiled.spec, 0)
+    for n, value in inputs.items():
+        plan.bind(n, value)
+    plan.execute()
+    grads = plan.outputs()[1:]
+    kept = [g.copy() for g in grads]
+    address = grads[0].__array_interface__["data"][0]
+    (go, went), (answer, told) = os.pipe(), os.pipe()
+    child = os.fork()
+    if child == 0:
+        try:
+            signal.alarm(60)
+            os.read(go, 1)  # the parent has overwritten its block by now
+            same = all(g.tobytes() == k.tobytes() for g, k in zip(grads, kept))
+            for g in grads:
+                g.fill(7.0)
+            del g, grads
+            fresh = _host.empty(1000, np.dtype(np.float32))
+            os.write(told, b"y" if same and fresh.flags.owndata else b"n")
+        finally:
+            os._exit(0)
+    del grads
+    plan.bind(compiled.spec.parameters[1][0], 2.0 * np.asarray(inputs[compiled.spec.parameters[1][0]]))
+    plan.execute()
+    later = plan.outputs()[1:]
+    assert later[0].__array_interface__["data"][0] == address
+    os.write(went, b"g")
+    said = os.read(answer, 1)
+    os.waitpid(child, 0)
+    for end in (go, went, answer, told):
+        os.close(end)
+    assert said == b"y"
+    for i, g in enumerate(later):
+        assert g.tobytes() == plan.read_output(1 + i).tobytes() and g.tobytes() != kept[i].tobytes()
 
 
 def test_repeated_calls_follow_changed_arguments(cuda_device):
