@@ -18,6 +18,7 @@ from . import _host, _lib
 from ._symbolic import Program
 
 COTANGENT_NAME = "__quabla_loss_cotangent"
+SMALL_LEAF_BYTES = 16384  # copied out of a read-back buffer: about a microsecond
 
 
 @dataclass
@@ -155,9 +156,11 @@ class Plan:
         return found
 
     def _leaves(self, flat: np.ndarray, base: int = 0) -> list[np.ndarray]:
-        """Views of a flat buffer, one per parameter."""
+        """One array per parameter from a flat buffer: views of it, small leaves copies (one bias kept for long does not
+        keep the whole buffer, which may be page-locked)."""
         item = self.dtype.itemsize
-        return [np.ndarray(shape, self.dtype, flat, (base + first) * item) for shape, first in self._layout()]
+        views = [np.ndarray(shape, self.dtype, flat, (base + first) * item) for shape, first in self._layout()]
+        return [v.copy() if v.nbytes <= SMALL_LEAF_BYTES else v for v in views]
 
     def close(self) -> None:
         if getattr(self, "_handle", None) and self._owned:
@@ -218,7 +221,8 @@ class Plan:
         return out
 
     def outputs(self) -> list[np.ndarray]:
-        """The loss and every gradient, read in one transfer."""
+        """The loss and every gradient, read in one transfer.  Large gradients are views of one buffer: keeping one keeps
+        the buffer (`.copy()` what is kept for long); the arrays share no elements."""
         self._layout()
         flat = _host.empty(1 + self._flat_size, self.dtype)
         _lib.check(self._lib.qb200_plan_read_outputs(self._handle, flat.__array_interface__["data"][0], flat.nbytes))
