@@ -1513,7 +1513,8 @@ qb200_status Plan<T>::run(bool forward_only) {
     QB_TRY(use_device());
     QB_TRY(check_bound());
     QB_TRY(refresh_tables());
-    StepGraph& g = graphs_[forward_only ? 1 : 0];
+    // The correction scheme of the tcgen05 GEMMs is read at every call: a sequence for each.
+    StepGraph& g = graphs_[(forward_only ? 1 : 0) + (tc_any_ ? 2 * tc_cor_mode() : 0)];
     const int64_t before = launches_;
     if (g.uses > 0 && g.exec == nullptr && !timers_ && !g.single && g.launches <= GRAPH_MAX_LAUNCHES) {
         capturing_ = true;

@@ -80,6 +80,30 @@ def test_any_choice_and_order_of_slots_leaves_the_others_alone(cuda_device, name
         np.testing.assert_array_equal(plan.read_input(n, expected[n].shape), expected[n], err_msg=n)
 
 
+def test_a_captured_plan_follows_the_correction_scheme(cuda_device, monkeypatch):
+    # QB200_TC_COR is read at every call, by a replayed sequence as by single launches.
+    w, compiled, inputs = traced("heat3d", 640)
+    plan, fresh = Plan(compiled.spec, 0), {}
+    for n, value in inputs.items():
+        plan.bind(n, value)
+
+    def outputs(p):
+        p.execute()
+        return [o.tobytes() for o in p.outputs()] + [p.loss().tobytes()]
+
+    for scheme in ("tf32", "bf16"):
+        monkeypatch.setenv("QB200_TC_COR", scheme)
+        single = Plan(compiled.spec, 0)
+        for n, value in inputs.items():
+            single.bind(n, value)
+        fresh[scheme] = outputs(single)
+        single.close()
+    assert fresh["tf32"] != fresh["bf16"]
+    for scheme in ("tf32", "tf32", "tf32", "bf16", "bf16", "bf16", "tf32", "bf16"):
+        monkeypatch.setenv("QB200_TC_COR", scheme)
+        assert outputs(plan) == fresh[scheme]
+
+
 def test_a_refused_page_lock_leaves_the_next_step_alone(cuda_device):
     # More host memory than any machine has: refused on the host, and not the next launch's error.
     w, compiled, inputs = traced("poisson1d", 64)
