@@ -1,9 +1,12 @@
 """Point sets of one plan on two streams: the largest down the first lane, the others down the second."""
 
+import numpy as np
 import pytest
 
+import quabla_b200 as qb
 from quabla_b200 import _lib
 from quabla_b200._plan import Plan
+from quabla_b200._transforms import CompiledLoss
 
 from _util import relative_error, traced
 
@@ -43,3 +46,42 @@ def test_sets_on_two_lanes_are_repeatable_and_agree_with_one(cuda_device, monkey
     for other in (run(None), run(None, single=True) if scratch is None else one):
         for a, b in zip(other, one):
             assert relative_error(a, b) <= 1e-12  # two double accumulators added instead of one
+
+
+def _two_sets(first, second, dtype=np.float64, width=128):
+    """A residual of second order on `first` points, values on `second`, one hidden-to-hidden layer."""
+    def loss(params, p, q):
+        u = lambda x: (qb.tanh(qb.tanh(x.reshape(1, -1) @ params["w"] + params["b"]) @ params["m"]) @ params["v"]).reshape(())
+        laplacian = lambda x: (lambda h: h[0, 0] + h[1, 1])(qb.hessian(u)(x))
+        return qb.mean(qb.vmap(laplacian)(p) ** 2) + qb.mean(qb.vmap(u)(q) ** 2)
+
+    rng = np.random.default_rng(2)
+    params = {"w": rng.normal(size=(2, width)), "b": rng.normal(size=width), "m": rng.normal(size=(width, width)) / 12,
+              "v": rng.normal(size=(width, 1)) / 12}
+    params = {k: v.astype(dtype) for k, v in params.items()}
+    return loss, (params, rng.uniform(size=(first, 2)).astype(dtype), rng.uniform(size=(second, 2)).astype(dtype))
+
+
+@pytest.mark.parametrize("first,second", [(7000, 9000), (9000, 700), (20480, 700)])
+def test_time_of_the_first_set_on_either_lane(cuda_device, first, second):
+    # The set goes down the second lane, the first one, or (cut into chunks) both; beside other work it takes as long
+    # as alone or longer.
+    loss, args = _two_sets(first, second)
+    compiled = CompiledLoss(loss, args, (0,), 0)
+    plan = compiled.plan
+    assert [s.n_points for s in compiled.spec.sets] == [first, second] and plan.query(_lib.Q_LANES) == 2
+    compiled.bind(args)
+
+    def times():
+        out = []
+        for _ in range(6):  # captured from the second on
+            plan.execute()
+            plan.synchronize()
+            out.append(plan.query(_lib.Q_SET0_NANOSECONDS))
+        return out[1:]
+
+    both = times()
+    plan.set_option(_lib.OPT_SINGLE_LANE, 1)
+    alone = sorted(times())[2]
+    # Two lanes halve the time of a set cut into chunks at best.
+    assert min(both) >= 0.4 * alone, (both, alone)
