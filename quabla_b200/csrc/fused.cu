@@ -77,8 +77,10 @@ bool fused_lookup<double>(int width, bool, int layers, int code, int act, FusedE
 
 template <typename T>
 cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, size_t smem, cudaStream_t stream, const FusedArgs<T>& args) {
+    // The bound of every launch, not of this one: plans of other depths share the kernel, and a thread that launches one
+    // of them must not lower what another has just raised.
     cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(entry.kernel),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FUSED_MAX_SMEM);
     if (e != cudaSuccess) return e;
     if (entry.ctas_per_sm > 1) {
         // Co-residency needs the whole shared-memory carve-out.

@@ -4,13 +4,15 @@ and single launches they stand for: the same bits."""
 import ctypes as C
 import os
 import signal
+import threading
 
 import numpy as np
 import pytest
 
 import quabla_b200 as qb
-from quabla_b200 import _host, _lib
+from quabla_b200 import _host, _lib, workloads
 from quabla_b200._plan import Plan, opt_config
+from quabla_b200._transforms import CompiledLoss
 
 from _util import traced
 
@@ -102,6 +104,37 @@ def test_a_captured_plan_follows_the_correction_scheme(cuda_device, monkeypatch)
     for scheme in ("tf32", "tf32", "tf32", "bf16", "bf16", "bf16", "tf32", "bf16"):
         monkeypatch.setenv("QB200_TC_COR", scheme)
         assert outputs(plan) == fresh[scheme]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_plans_of_different_depth_on_two_threads(cuda_device, dtype):
+    # They share a kernel and need different amounts of shared memory; single launches, so that every one sets it.
+    def plan_of(depth):
+        loss = workloads.make("poisson2d", 64).loss
+        params = workloads.init_mlp(qb.random.key(depth), [2] + [64] * depth + [1], dtype)
+        points = np.random.default_rng(depth).uniform(size=(64, 2)).astype(dtype)
+        compiled = CompiledLoss(loss, (params, points, points), (0,), 0)
+        compiled.bind((params, points, points))
+        compiled.plan.set_option(_lib.OPT_KERNEL_TIMERS, 1)
+        compiled.plan.execute()
+        return compiled.plan, [o.tobytes() for o in compiled.plan.outputs()]
+
+    failures = []
+
+    def run(plan, expected):
+        try:
+            for _ in range(400):
+                plan.execute()
+            assert [o.tobytes() for o in plan.outputs()] == expected
+        except Exception as e:  # reported below, on the test's thread
+            failures.append(e)
+
+    threads = [threading.Thread(target=run, args=plan_of(depth)) for depth in (1, 8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
 
 
 def test_a_refused_page_lock_leaves_the_next_step_alone(cuda_device):
