@@ -94,7 +94,7 @@ cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, size_t smem, cuda
 
 template <>
 size_t fused_weight_image_bytes<float>(int hidden_to_hidden, int width) {
-    return (size_t)std::max(hidden_to_hidden, 1) * 4 * width * (width + 8);
+    return (size_t)std::max(hidden_to_hidden, 1) * 6 * width * (width + 8);
 }
 template <>
 size_t fused_weight_image_bytes<double>(int hidden_to_hidden, int width) {
@@ -114,15 +114,20 @@ static PrepArgs prep_args(const int* w_off, const int* rows, const int* cols, in
 
 template <>
 cudaError_t fused_prep_launch<float>(const float* params, const int* w_off, const int* rows, const int* cols,
-                                     int hidden_to_hidden, int width, void* images, float* scales, cudaStream_t stream) {
+                                     int hidden_to_hidden, int width, void* images, cudaStream_t stream) {
     if (hidden_to_hidden < 1) return cudaSuccess;
-    prep_weights_kernel<<<hidden_to_hidden, 1024, 0, stream>>>(params, prep_args(w_off, rows, cols, hidden_to_hidden), width,
-                                                               static_cast<uint32_t*>(images), scales);
+    const PrepArgs p = prep_args(w_off, rows, cols, hidden_to_hidden);
+    const dim3 grid(4, hidden_to_hidden);
+    uint32_t* out = static_cast<uint32_t*>(images);
+    if (width == 16) prep_weights_kernel<16><<<grid, 256, 0, stream>>>(params, p, out);
+    if (width == 32) prep_weights_kernel<32><<<grid, 256, 0, stream>>>(params, p, out);
+    if (width == 48) prep_weights_kernel<48><<<grid, 256, 0, stream>>>(params, p, out);
+    if (width == 64) prep_weights_kernel<64><<<grid, 256, 0, stream>>>(params, p, out);
     return cudaGetLastError();
 }
 template <>
 cudaError_t fused_prep_launch<double>(const double* params, const int* w_off, const int* rows, const int* cols,
-                                      int hidden_to_hidden, int width, void* images, float*, cudaStream_t stream) {
+                                      int hidden_to_hidden, int width, void* images, cudaStream_t stream) {
     if (hidden_to_hidden < 1) return cudaSuccess;
     prep_weights64_kernel<<<dim3(4, hidden_to_hidden), 256, 0, stream>>>(
         params, prep_args(w_off, rows, cols, hidden_to_hidden), width, static_cast<double*>(images));

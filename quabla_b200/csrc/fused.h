@@ -50,11 +50,11 @@ cudaError_t fused_launch(const FusedEntry<T>& entry, int grid, size_t smem, cuda
 // Bytes of the weight images of `hidden_to_hidden` layers padded to `width`.
 template <typename T>
 size_t fused_weight_image_bytes(int hidden_to_hidden, int width);
-// Writes the images (and, for float32, their scales) from the flat parameters; image i is network layer 1 + i, of
+// Writes the images from the flat parameters; image i is network layer 1 + i, of
 // rows[i] x cols[i] at offset w_off[i].
 template <typename T>
 cudaError_t fused_prep_launch(const T* params, const int* w_off, const int* rows, const int* cols, int hidden_to_hidden,
-                              int width, void* images, float* scales, cudaStream_t stream);
+                              int width, void* images, cudaStream_t stream);
 // One thread's bounded wait on a barrier that is never completed: raises *error when it gives up.
 cudaError_t unarmed_wait_launch(int* error, cudaStream_t stream);
 

@@ -92,7 +92,6 @@ struct FusedArgs {
     double* loss_cta;   // [gridDim.x]
     int forward_only;
     const void* weight_images;  // tensor-core variant: pre-split weight images (prep_weights_kernel)
-    const float* image_scales;  // and their scales
     T* dw_scratch;              // tensor-core variant: running weight-gradient sums, or null: in shared memory
     int* error;                 // set to 1 when a bounded wait inside the kernel gave up
 };

@@ -1,14 +1,15 @@
 // Fused engine, float32, hidden widths up to 64, weight contractions on the tensor cores with operands split into
-// two float16 parts.
+// three bfloat16 parts.
 //
-// Split.  A block of 16 x 16 elements (16 points x 16 units of one stream) is scaled by a power of two so that its
-// largest element lies in [2^13, 2^14), and every scaled element y is written as hi + lo with hi = f16(y) and
-// lo = f16(y - hi).  The pair carries y to 2^-23 of itself down to 2^-16 of the block's largest element and to
-// 2^-39 of that largest element below (hi and lo are then subnormal).  A product A.B is lo.hi + hi.lo + hi.hi,
-// three m16n8k16 instructions per 16 contraction elements: half the tensor-pipe time and half the instructions of three
-// tf32 products, which left 2e-7 per product against 1e-7 here (the dropped lo.lo is of random sign).  One
-// contraction step of 16 reads exactly one block of either operand, so the blocks' scales multiply the step's
-// partial sum on its way into the running sum: a multiply-add where a plain addition was needed anyway.
+// Split.  x = hi + mid + lo with hi = bf16(x), mid = bf16(x - hi) and lo the rest, which is a bfloat16 as well: 24 bits in
+// three parts of 8, every element with an exponent of its own and float32's range, so the split loses nothing.  A
+// product A.B is hi.hi + (hi.mid + mid.hi) + (mid.mid + hi.lo + lo.hi); the dropped mid.lo, lo.mid and lo.lo are below
+// 2^-25 of it and of random sign.  The tensor core truncates what it adds, a loss of one sign that no number of points
+// averages out, so hi.hi runs twice, the second time onto minus its own result: that leaves exactly what the first run
+// dropped, and the smaller products are added to it.  Seven m16n8k16 instructions per 16 contraction elements.  Mean
+// relative loss of such a step, <error, exact> / <exact, exact> over 500,000 sums of 16 products against float64: 6e-12
+// (normal operands), 1.3e-11 (uniform), 1.2e-9 (positive), 1.5e-10 (exponents spread by 2^40); of hi.hi run once 0.8e-8 to
+// 3.7e-8, a factor that changes with the operands and cannot be put back by a constant.
 //
 // Same structure as fused_step_kernel (fused_kernel.cuh): persistent CTAs walk tiles of 16 points, run forward /
 // residual / reverse sweep per tile, keep the saved jets in an L2-resident per-CTA scratch and accumulate weight
@@ -18,20 +19,26 @@
 // Networks narrower than W (or of unequal widths) run padded with zero weights: a padded unit's activation meets
 // only zero weights and its cotangent is zero.
 //
-// Bound: issue slots and latencies of the epilogues between the contractions (the tensor pipe is not the limit), which
-// is why a CTA is one point group with as few registers as its stream count allows: as many CTAs as fit
-// overlap one another's phases (three per SM at width 64 and up to four streams).
-// Measured against the 3xTF32 kernel before it: 65,536-point 2-D Poisson interior 590 -> 330 us, 1,048,576-point beam step
-// 11.15 -> 7.24 ms, width 50 at 20,000 points 845 -> 150 us per step (layer by layer before).
+// Bound: the contractions, 63 % of a tile's cycles (width 64, four streams: 69,000 cycles per tile with two CTAs on an SM;
+// head and residual program 10 %, transposed jets 8 %, staging 3 %), in which the tensor pipe is busy 70 % of the time (45 %
+// over all), and the number of CTAs that overlap one another's other phases: shared memory holds two of 80 KB.
+// Measured, microseconds per step or call at width 64 (50) with three tf32 products or, at width 50, layer by layer; with two
+// float16 parts; and now: 65,536-point 2-D Poisson 727, 407, 597; 10,007-point gradients 595, 204, 240; 1,048,576-point beam
+// 11,150, 7,250, 9,990; 20,000 points at width 50 848, 155, 218.  Error of float32 gradients against float64 in
+// parts of the first of these (geometric mean over four workloads, two activations, two weight scales, six seeds, 1,003 and 20,011
+// points): 0.65, 0.59, 0.69, 0.59 and 0.64 at widths 16, 24, 32, 48 and 50, where the former kernels multiplied and added in
+// float32, and 0.08 at width 64.  Two float16 parts with an exponent per 16 x 16 block were 1.15 to 1.33 times as far off and lost
+// entries that are small beside their neighbours altogether (5e-2 of themselves at 2^-30).
 //
 // Replaces the reference's per-node plan execution (crates/quabla-core/src/tensor_ir/cuda.rs:1792-2972) and its
 // cuBLAS strided-batched GEMV-shaped calls (cuda.rs:4936-5035).
 #pragma once
-#include <cuda_fp16.h>
+#include <cuda_bf16.h>
 
 #include <cstdint>
 #include <cstdio>
 
+#include "fused.h"
 #include "fused_kernel.cuh"
 
 namespace qb {
@@ -39,7 +46,7 @@ namespace qb {
 // Four 8x8 matrices of 16-bit elements; thread (g, t) receives elements 2t, 2t + 1 of row g of each (TRANS: of
 // column g), the m16n8k16 fragment layouts.
 template <bool TRANS>
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const __half* row_ptr) {
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const __nv_bfloat16* row_ptr) {
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(row_ptr);
     if (TRANS)
         asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -51,57 +58,63 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const __half* row_
                      : "r"(at));
 }
 
-// d += a (16x16, row) * b (16x8, col), float16 operands, float32 accumulate.  Not volatile: the accumulator operands
+// d += a (16x16, row) * b (16x8, col), bfloat16 operands, float32 accumulate.  Not volatile: the accumulator operands
 // carry the dependencies, the compiler may interleave independent chains.
-__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// acc += f * (A_lo.B_hi + A_hi.B_lo + A_hi.B_hi) of one 16 x 16 by 16 x 16 step.  The tensor core adds into its
-// accumulator with truncation, so every step chains its three products from zero and the partial is added to the
-// running sum with a round-to-nearest multiply-add.
-__device__ __forceinline__ void mma_step(float (&acc)[2][4], const uint32_t (&ahi)[4], const uint32_t (&alo)[4],
-                                         const uint32_t (&bhi)[4], const uint32_t (&blo)[4], float f) {
+// N steps of 16 x 16 by 16 x 16 on {hi, mid, lo} fragments, of A(n) and B(n) each: acc[n] += (hi.hi as the tensor
+// core leaves it) + (what it left out and the five smaller products).  The 2 N chains of seven dependent instructions
+// are issued side by side (one pair of streams at a time instead of one: 1 to 3 % of a step).
+template <int N, typename FragA, typename FragB>
+__device__ __forceinline__ void mma_steps(float (*acc)[2][4], FragA A, FragB B) {
+    constexpr int PRODUCTS[7][2] = {{0, 0}, {0, 0}, {2, 0}, {0, 2}, {1, 1}, {1, 0}, {0, 1}};
+    float part[N][2][4], rest[N][2][4];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        mma_f16(part, alo, bhi[2 * j], bhi[2 * j + 1]);
-        mma_f16(part, ahi, blo[2 * j], blo[2 * j + 1]);
-        mma_f16(part, ahi, bhi[2 * j], bhi[2 * j + 1]);
+    for (int q = 0; q < 7; ++q)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(part[c], f, acc[j][c]);
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float(&d)[4] = rest[n][j];
+                if (q == 0) d[0] = d[1] = d[2] = d[3] = 0.0f;
+                const uint32_t(&b)[4] = B(n)[PRODUCTS[q][1]];
+                mma_bf16(d, A(n)[PRODUCTS[q][0]], b[2 * j], b[2 * j + 1]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (q == 0) {
+                        part[n][j][c] = d[c];
+                        d[c] = -d[c];
+                    }
+                    if (q == 6) acc[n][j][c] += part[n][j][c] + d[c];
+                }
+            }
+}
+
+// Two elements as packed bfloat16 {hi, mid, lo} pairs.
+__device__ __forceinline__ void split_bf16(float x0, float x1, uint32_t (&parts)[3]) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const __nv_bfloat162 pair = __floats2bfloat162_rn(x0, x1);
+        parts[q] = *reinterpret_cast<const uint32_t*>(&pair);
+        x0 -= __uint_as_float(parts[q] << 16);
+        x1 -= __uint_as_float(parts[q] & 0xffff0000u);
     }
 }
 
-// Power-of-two scale of a block whose largest magnitude has the bit pattern `largest`: *inverse maps it into
-// [2^13, 2^14), the returned factor maps back.  Blocks below 2^-113 (and empty ones) share the scale of that size.
-__device__ __forceinline__ float block_scale(uint32_t largest, float* inverse) {
-    const uint32_t e = max(largest >> 23, 14u);
-    *inverse = __uint_as_float((267u - e) << 23);
-    return __uint_as_float((e - 13u) << 23);
-}
+// Operand planes: rows of W elements in chunks of eight, laid out so that the eight row addresses of an ldmatrix tile
+// (one chunk of eight successive rows) fall into distinct bank groups: padded by a chunk, or, at width 64, where the
+// padding would cost a resident CTA at six streams, unpadded with the chunks of a row permuted by its number.
+template <int W>
+struct PlaneLayout {
+    static constexpr int LD = W == 64 ? 64 : W + 8;
+    static __host__ __device__ constexpr int at(int row, int chunk) { return row * LD + 8 * (W == 64 ? chunk ^ (row & 7) : chunk); }
+};
 
-// Mean relative loss of mma_step's truncating accumulations: a factor common to all contractions, which neither the
-// number of points nor of terms averages out, so it is put back where that costs nothing: into the weights' lo parts and
-// into the finished weight-gradient sums.  Measured as <error, exact> / <exact, exact> of 40,000 16 x 16 x 16 steps against float64:
-// -3.9e-8 (normal operands), -4.1e-8 (uniform), -4.4e-8 (positive).  Without it gradients of networks of width 16, 32 and
-// 50 were 2 to 5 times further from float64 than plain float32 multiply-adds.
-constexpr float MMA_TRUNCATION = 4.1e-8f;
-
-// Two scaled elements as packed float16 hi and lo pairs, raised by `gain` of themselves.
-__device__ __forceinline__ void split_f16(float x0, float x1, float inverse, uint32_t& hi, uint32_t& lo, float gain = 0.0f) {
-    const float y0 = x0 * inverse, y1 = x1 * inverse;
-    const __half2 h = __floats2half2_rn(y0, y1);
-    const float2 back = __half22float2(h);
-    const __half2 l = gain == 0.0f ? __floats2half2_rn(y0 - back.x, y1 - back.y)
-                                   : __floats2half2_rn(fmaf(y0, gain, y0 - back.x), fmaf(y1, gain, y1 - back.y));
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
-// ---- asynchronous staging: bulk copies (TMA engine, no multicast) and cp.async ----
+// ---- asynchronous staging: bulk copies (TMA engine, no multicast) ----
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
@@ -134,16 +147,10 @@ __device__ __forceinline__ void mbar_wait_limited(uint64_t* bar, uint32_t parity
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int* error) {
     mbar_wait_limited(bar, parity, error, 1 << 22);
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-
-// Weight images written by prep_weights_kernel, one per hidden-to-hidden layer: {hi, lo} planes [W][W + 8] halves of
-// the row-major [in][out] matrix, zero-padded to W x W, scaled as one block; its factor goes to scales[layer].  The
-// forward contraction reads it transposed (ldmatrix .trans), the data gradient as it is.
+// Weight images written by prep_weights_kernel, one per hidden-to-hidden layer: {hi, mid, lo} planes [W][W] of the
+// row-major [in][out] matrix, zero-padded to W x W.  The forward contraction reads it transposed (ldmatrix .trans), the
+// data gradient as it is.
 struct PrepArgs {
     int layers;                       // hidden-to-hidden layers
     int w_off[FUSED_MAX_LAYERS + 1];  // parameter offset of network layer 1 + i
@@ -151,30 +158,20 @@ struct PrepArgs {
     int cols[FUSED_MAX_LAYERS + 1];
 };
 
-static __global__ void __launch_bounds__(1024) prep_weights_kernel(const float* __restrict__ params, PrepArgs p, int W,
-                                                                   uint32_t* __restrict__ images, float* __restrict__ scales) {
-    __shared__ uint32_t warp_max[32];
-    const int layer = blockIdx.x, rows = p.rows[layer], cols = p.cols[layer];
+template <int W>
+static __global__ void __launch_bounds__(256) prep_weights_kernel(const float* __restrict__ params, PrepArgs p,
+                                                                  uint32_t* __restrict__ images) {
+    typedef PlaneLayout<W> P;
+    const int layer = blockIdx.y, rows = p.rows[layer], cols = p.cols[layer];
     const float* w = params + p.w_off[layer];
-    uint32_t largest = 0;
-    for (int e = threadIdx.x; e < rows * cols; e += blockDim.x) largest = max(largest, __float_as_uint(w[e]) & 0x7fffffffu);
-    largest = __reduce_max_sync(0xffffffffu, largest);
-    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = largest;
-    __syncthreads();
-    largest = __reduce_max_sync(0xffffffffu, (threadIdx.x & 31) < (blockDim.x >> 5) ? warp_max[threadIdx.x & 31] : 0u);
-    float inverse;
-    const float scale = block_scale(largest, &inverse);
-    if (threadIdx.x == 0) scales[layer] = scale;
-    const int pairs = W / 2, stride = (W + 8) / 2, plane = W * stride;  // in 32-bit words
-    uint32_t* img = images + (size_t)layer * 2 * plane;
-    for (int e = threadIdx.x; e < W * pairs; e += blockDim.x) {
-        const int r = e / pairs, c = 2 * (e % pairs);
-        const float x0 = (r < rows && c < cols) ? w[r * cols + c] : 0.0f;
-        const float x1 = (r < rows && c + 1 < cols) ? w[r * cols + c + 1] : 0.0f;
-        uint32_t hi, lo;
-        split_f16(x0, x1, inverse, hi, lo, MMA_TRUNCATION);
-        img[r * stride + c / 2] = hi;
-        img[plane + r * stride + c / 2] = lo;
+    constexpr int PLANE = W * P::LD / 2;  // 32-bit words
+    uint32_t* img = images + (size_t)layer * 3 * PLANE;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < W * W / 2; e += gridDim.x * blockDim.x) {
+        const int r = e / (W / 2), c = 2 * (e % (W / 2));
+        uint32_t parts[3];
+        split_bf16((r < rows && c < cols) ? w[r * cols + c] : 0.0f, (r < rows && c + 1 < cols) ? w[r * cols + c + 1] : 0.0f, parts);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) img[q * PLANE + (P::at(r, c / 8) + c % 8) / 2] = parts[q];
     }
 }
 
@@ -187,14 +184,12 @@ struct MmaGeom {
     static constexpr int THREADS = 32 * NW;
     static constexpr int TP = 16;
     static constexpr int ROWS = S * TP;
-    // Rows of W + 8 halves: 16-byte aligned, and the eight row addresses of an ldmatrix tile fall into distinct
-    // bank groups for every W used (stride 4 (mod 8) words).
-    static constexpr int LD = W + 8;
-    static constexpr int PLANE = ROWS * LD;      // halves per operand plane
-    static constexpr int WPLANE = W * LD;        // halves per weight plane
-    static constexpr int ACT_BYTES = 4 * PLANE;  // hi and lo
-    static constexpr int WIMG_BYTES = 4 * WPLANE;
-    static constexpr int OFF_ACT = 0;                      // activations / cotangents, [hi, lo][ROWS][LD]
+    static constexpr int LD = PlaneLayout<W>::LD;
+    static constexpr int PLANE = ROWS * LD;      // elements per operand plane
+    static constexpr int WPLANE = W * LD;        // elements per weight plane
+    static constexpr int ACT_BYTES = 6 * PLANE;  // hi, mid and lo
+    static constexpr int WIMG_BYTES = 6 * WPLANE;
+    static constexpr int OFF_ACT = 0;                      // activations / cotangents, [hi, mid, lo][ROWS][LD]
     static constexpr int OFF_HT = OFF_ACT + ACT_BYTES;     // previous layer's jets (weight-gradient operand), same layout
     static constexpr int OFF_WB = OFF_HT + ACT_BYTES;      // weight image of the contraction at hand
     static constexpr int OFF_RED = OFF_WB + WIMG_BYTES;    // [NW][S][TP] output-layer partials
@@ -202,18 +197,17 @@ struct MmaGeom {
     static constexpr int OFF_UH = OFF_U + 4 * ROWS;        // [S][TP]
     static constexpr int OFF_BAR = OFF_UH + 4 * ROWS;      // two mbarriers
     static constexpr int OFF_VAR = OFF_BAR + 16;           // regions that depend on the depth:
-    // block scales [L + 1][S][NW], weight scales [L], parameters {biases [L][W], first layer [4][W], output layer
-    // [W]}, gradient sums of the same, of the output bias
-    static __host__ __device__ constexpr size_t var_bytes(int L) {
-        return 4 * ((size_t)(L + 1) * S * NW + L + 2 * (size_t)(L + 5) * W + 4);
-    }
-    static __host__ __device__ constexpr size_t base_bytes(int L) { return ((size_t)OFF_VAR + var_bytes(L) + 15) / 16 * 16; }
+    // parameters {biases [L][W], first layer [4][W], output layer [W]} and gradient sums of the same
+    static __host__ __device__ constexpr size_t base_bytes(int L) { return (size_t)OFF_VAR + 4 * 2 * (size_t)(L + 5) * W; }
     static constexpr size_t DW_BYTES = 4 * (size_t)W * W;  // running weight-gradient sums of one layer
-    // Registers decide how many CTAs share an SM: 168 per thread hold up to four streams, 224 to 255 more.
-    static constexpr int MIN_CTAS = (S <= 4 ? 12 : 8) / NW;
+    // CTAs that share an SM: as many as its shared memory holds of a network of four hidden layers, and up to 12 warps of
+    // 168 registers a thread (up to four streams) or 8 of 224 to 255.
+    static constexpr int FIT = (int)(FUSED_SM_SMEM / (base_bytes(4) + FUSED_CTA_SMEM + 512));
+    static constexpr int BY_REGISTERS = (S <= 4 ? 12 : 8) / NW;
+    static constexpr int MIN_CTAS = FIT < 1 ? 1 : FIT < BY_REGISTERS ? FIT : BY_REGISTERS;
     // Saved jets: the operand planes as they sit in shared memory, one bulk copy per layer.  Saved pre-activations:
     // read back by the thread that wrote them, so laid out per thread.
-    static constexpr size_t SCRATCH_PER_CTA = (size_t)ROWS * LD;
+    static constexpr size_t SCRATCH_PER_CTA = (size_t)ACT_BYTES / 4;
 };
 
 // Optional per-phase cycle counters of CTA 0 (compile with -DQB_PHASE_TIMING), printed once per launch.
@@ -230,65 +224,59 @@ struct MmaGeom {
 #define QB_PHASE(i)
 #endif
 
-// The warp's 16 x 16 block of every stream as scaled float16 pairs into the operand planes; scales [S][NW].
-template <int S, int NW, int LD, int PLANE>
-__device__ __forceinline__ void store_blocks(const float (&acc)[S][2][4], __half* planes, float* scales, int warp, int g, int t) {
-    uint32_t largest[S];
+// The warp's 16 x 16 block of every stream, split, into the operand planes.
+template <int S, int W>
+__device__ __forceinline__ void store_blocks(const float (&acc)[S][2][4], __nv_bfloat16* planes, int warp, int g, int t) {
+    typedef PlaneLayout<W> P;
+    constexpr int PLANE = S * 16 * P::LD / 2;  // 32-bit words
+    uint32_t* words = reinterpret_cast<uint32_t*>(planes);
 #pragma unroll
-    for (int s = 0; s < S; ++s) {
-        uint32_t m = 0;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) m = max(m, __float_as_uint(acc[s][j][c]) & 0x7fffffffu);
-        largest[s] = __reduce_max_sync(0xffffffffu, m);
-    }
-    uint32_t* words = reinterpret_cast<uint32_t*>(planes) + (g * LD + 16 * warp + 2 * t) / 2;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        float inverse;
-        const float scale = block_scale(largest[s], &inverse);
-        if (g == 0 && t == 0) scales[s * NW + warp] = scale;
+    for (int s = 0; s < S; ++s)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                uint32_t hi, lo;
-                split_f16(acc[s][j][2 * i], acc[s][j][2 * i + 1], inverse, hi, lo);
-                uint32_t* at = words + ((s * 16 + 8 * i) * LD + 8 * j) / 2;
-                at[0] = hi;
-                at[PLANE / 2] = lo;
+                uint32_t parts[3];
+                split_bf16(acc[s][j][2 * i], acc[s][j][2 * i + 1], parts);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) words[q * PLANE + P::at(s * 16 + 8 * i + g, 2 * warp + j) / 2 + t] = parts[q];
             }
-    }
 }
 
 // acc[s] = A[rows of stream s][W] * B[W][16 columns of this warp].  FORWARD: B(k, n) = W[k][n]; else B(k, n) = W[n][k].
-template <int S, int NW, int LD, int PLANE, int WPLANE, bool FORWARD>
-__device__ __forceinline__ void warp_contract(const __half* __restrict__ A, const __half* __restrict__ Wimg,
-                                              const float* __restrict__ scales, float wscale, int warp, int lane,
-                                              float (&acc)[S][2][4]) {
+template <int S, int W, bool FORWARD>
+__device__ __forceinline__ void warp_contract(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ Wimg,
+                                              int warp, int lane, float (&acc)[S][2][4]) {
+    typedef PlaneLayout<W> P;
+    constexpr int PLANE = S * 16 * P::LD, WPLANE = W * P::LD;
 #pragma unroll
     for (int s = 0; s < S; ++s)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[s][j][c] = 0.0f;
-    const int mi = lane >> 3, rr = lane & 7;
-    const __half* a_lane = A + (rr + (mi & 1) * 8) * LD + (mi >> 1) * 8;
-    const __half* b_lane = FORWARD ? Wimg + ((mi & 1) * 8 + rr) * LD + 16 * warp + (mi >> 1) * 8
-                                   : Wimg + (16 * warp + (mi >> 1) * 8 + rr) * LD + (mi & 1) * 8;
+    const int mi = lane >> 3, rr = lane & 7, low = mi & 1, high = mi >> 1;
 #pragma unroll
-    for (int kb = 0; kb < NW; ++kb) {
-        uint32_t bhi[4], blo[4];
-        const __half* b = b_lane + (FORWARD ? kb * 16 * LD : kb * 16);
-        ldmatrix_x4<FORWARD>(bhi, b);
-        ldmatrix_x4<FORWARD>(blo, b + WPLANE);
+    for (int kb = 0; kb < W / 16; ++kb) {
+        uint32_t b[3][4];
+        const int b_at = FORWARD ? P::at(16 * kb + 8 * low + rr, 2 * warp + high) : P::at(16 * warp + 8 * high + rr, 2 * kb + low);
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            uint32_t ahi[4], alo[4];
-            ldmatrix_x4<false>(ahi, a_lane + s * 16 * LD + kb * 16);
-            ldmatrix_x4<false>(alo, a_lane + s * 16 * LD + kb * 16 + PLANE);
-            mma_step(acc[s], ahi, alo, bhi, blo, scales[s * NW + kb] * wscale);
+        for (int q = 0; q < 3; ++q) ldmatrix_x4<FORWARD>(b[q], Wimg + q * WPLANE + b_at);
+        uint32_t a[2][3][4];
+        auto load_a = [&](int s) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) ldmatrix_x4<false>(a[s & 1][q], A + q * PLANE + P::at(16 * s + 8 * low + rr, 2 * kb + high));
+        };
+        auto frag_b = [&](int) -> const uint32_t(&)[3][4] { return b; };
+#pragma unroll
+        for (int s = 0; s + 1 < S; s += 2) {
+            load_a(s);
+            load_a(s + 1);
+            mma_steps<2>(acc + s, [&](int n) -> const uint32_t(&)[3][4] { return a[n]; }, frag_b);
+        }
+        if (S % 2 == 1) {
+            load_a(S - 1);
+            mma_steps<1>(acc + S - 1, [&](int) -> const uint32_t(&)[3][4] { return a[(S - 1) & 1]; }, frag_b);
         }
     }
 }
@@ -314,11 +302,11 @@ template <int CODE, int W, int ACT>
 __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::MIN_CTAS) fused_mma_kernel(FusedArgs<float> a) {
     typedef MmaGeom<CODE, W> G;
     typedef Sig<CODE> SG;
-    constexpr int THREADS = G::THREADS, NW = G::NW, S = G::S, TP = G::TP, LD = G::LD, PLANE = G::PLANE, WPLANE = G::WPLANE;
+    constexpr int THREADS = G::THREADS, NW = G::NW, S = G::S, TP = G::TP, PLANE = G::PLANE, WPLANE = G::WPLANE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __half* act = reinterpret_cast<__half*>(smem_raw + G::OFF_ACT);
-    __half* ht = reinterpret_cast<__half*>(smem_raw + G::OFF_HT);
-    __half* wbuf = reinterpret_cast<__half*>(smem_raw + G::OFF_WB);
+    __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(smem_raw + G::OFF_ACT);
+    __nv_bfloat16* ht = reinterpret_cast<__nv_bfloat16*>(smem_raw + G::OFF_HT);
+    __nv_bfloat16* wbuf = reinterpret_cast<__nv_bfloat16*>(smem_raw + G::OFF_WB);
     float* red = reinterpret_cast<float*>(smem_raw + G::OFF_RED);
     float* us = reinterpret_cast<float*>(smem_raw + G::OFF_U);
     float* uh = reinterpret_cast<float*>(smem_raw + G::OFF_UH);
@@ -329,10 +317,7 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
     const int col0 = warp * 16;  // first unit of the warp
     const int L = a.L, d0 = a.d0, HL = L - 1;
     const bool backward = a.forward_only == 0;
-    float* scl = reinterpret_cast<float*>(smem_raw + G::OFF_VAR);  // [L][S][NW] activations, then one row for the cotangents
-    float* scl_z = scl + L * S * NW;
-    float* wscl = scl_z + S * NW;        // [L], by hidden-to-hidden layer
-    float* pbias = wscl + L;             // [L][W]
+    float* pbias = reinterpret_cast<float*>(smem_raw + G::OFF_VAR);  // [L][W]
     float* pfirst = pbias + L * W;       // [4][W]
     float* phead = pfirst + 4 * W;       // [W]
     float* gbias = phead + W;            // gradient sums in the same order
@@ -365,7 +350,6 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
         phead[i] = i < a.width[L - 1] ? a.params[a.w_off[L] + i] : 0.0f;
         ghead[i] = 0.0f;
     }
-    if (tid < HL) wscl[tid] = a.image_scales[tid];
     if (backward)
         for (int i = tid; i < HL * 2 * NW * THREADS; i += THREADS) dws[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     double loss_sum = 0.0;
@@ -391,14 +375,14 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
     long long loads_left = (long long)my_tiles * uses_per_tile;
     int next_use = 0;              // position of the next load in the tile's order
     uint32_t wphase = 0, hphase = 0;
-    const __half* images = static_cast<const __half*>(a.weight_images);
+    const __nv_bfloat16* images = static_cast<const __nv_bfloat16*>(a.weight_images);
     auto load_weights = [&]() {  // thread 0
         if (loads_left-- <= 0) return;
         const int layer = next_use < HL ? next_use : 2 * HL - 1 - next_use;
         if (++next_use == uses_per_tile) next_use = 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(wbar, G::WIMG_BYTES);
-        bulk_load(wbuf, images + (size_t)layer * 2 * WPLANE, G::WIMG_BYTES, wbar);
+        bulk_load(wbuf, images + (size_t)layer * 3 * WPLANE, G::WIMG_BYTES, wbar);
     };
     if (tid == 0) load_weights();
 
@@ -450,7 +434,7 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
                 QB_PHASE(0);  // wait for the weight image
-                warp_contract<S, NW, LD, PLANE, WPLANE, true>(act, wbuf, scl + (l - 1) * S * NW, wscl[l - 1], warp, lane, acc);
+                warp_contract<S, W, true>(act, wbuf, warp, lane, acc);
                 // The epilogue overwrites the operand: the bulk copy must have read it.
                 if (backward && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 __syncthreads();
@@ -486,7 +470,7 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
                 for (int j = 0; j < 2; ++j) zl[j * THREADS] = make_float4(acc[0][j][0], acc[0][j][1], acc[0][j][2], acc[0][j][3]);
             }
             if (l + 1 < L) {
-                store_blocks<S, NW, LD, PLANE>(acc, act, scl + l * S * NW, warp, g, t);
+                store_blocks<S, W>(acc, act, warp, g, t);
                 // The next iteration saves these planes with a bulk copy: make the writes visible to that proxy.
                 if (backward) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
@@ -625,7 +609,7 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
             }
             QB_PHASE(4);  // transposed jets, bias partials
             // Cotangents of the pre-activations: operand of both contractions below.
-            store_blocks<S, NW, LD, PLANE>(acc, act, scl_z, warp, g, t);
+            store_blocks<S, W>(acc, act, warp, g, t);
             mbar_wait(hbar, hphase, a.error);
             hphase ^= 1;
             __syncthreads();
@@ -633,44 +617,58 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
             // Weight gradient: dW[k][n] += sum_rows H[row][k] * Zhat[row][n]; this warp: its 16 k x all n.
             {
                 float4* gw = dws + (size_t)(l - 1) * 2 * NW * THREADS + tid;
-                // Starts from the running sums, loaded before the loop so that their latency hides behind the contraction.
+                // The running sums, loaded before the loop so that their latency hides behind the contraction, take this tile's
+                // in one addition.
+                float4 sums[NW][2];
                 float dw[NW][2][4];
 #pragma unroll
                 for (int nb = 0; nb < NW; ++nb)
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        const float4 q = gw[(2 * nb + j) * THREADS];
-                        dw[nb][j][0] = q.x; dw[nb][j][1] = q.y; dw[nb][j][2] = q.z; dw[nb][j][3] = q.w;
+                        sums[nb][j] = gw[(2 * nb + j) * THREADS];
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) dw[nb][j][c] = 0.0f;
                     }
-                const int mi = lane >> 3, rr = lane & 7;
-                const __half* a_lane = ht + ((mi >> 1) * 8 + rr) * LD + col0 + (mi & 1) * 8;
-                const __half* b_lane = act + ((mi & 1) * 8 + rr) * LD + (mi >> 1) * 8;
-                const float* scl_h = scl + (l - 1) * S * NW;
+                typedef PlaneLayout<W> P;
+                const int mi = lane >> 3, rr = lane & 7, low = mi & 1, high = mi >> 1;
 #pragma unroll
                 for (int s = 0; s < S; ++s) {
-                    uint32_t ahi[4], alo[4];
-                    ldmatrix_x4<true>(ahi, a_lane + s * 16 * LD);
-                    ldmatrix_x4<true>(alo, a_lane + s * 16 * LD + PLANE);
-                    const float fh = scl_h[s * NW + warp];
+                    uint32_t ha[3][4];
 #pragma unroll
-                    for (int nb = 0; nb < NW; ++nb) {
-                        uint32_t bhi[4], blo[4];
-                        ldmatrix_x4<true>(bhi, b_lane + s * 16 * LD + nb * 16);
-                        ldmatrix_x4<true>(blo, b_lane + s * 16 * LD + nb * 16 + PLANE);
-                        mma_step(dw[nb], ahi, alo, bhi, blo, fh * scl_z[s * NW + nb]);
+                    for (int q = 0; q < 3; ++q) ldmatrix_x4<true>(ha[q], ht + q * PLANE + P::at(16 * s + 8 * high + rr, 2 * warp + low));
+                    uint32_t zb[2][3][4];
+                    auto load_b = [&](int nb) {
+#pragma unroll
+                        for (int q = 0; q < 3; ++q)
+                            ldmatrix_x4<true>(zb[nb & 1][q], act + q * PLANE + P::at(16 * s + 8 * low + rr, 2 * nb + high));
+                    };
+                    auto frag_a = [&](int) -> const uint32_t(&)[3][4] { return ha; };
+#pragma unroll
+                    for (int nb = 0; nb + 1 < NW; nb += 2) {
+                        load_b(nb);
+                        load_b(nb + 1);
+                        mma_steps<2>(dw + nb, frag_a, [&](int n) -> const uint32_t(&)[3][4] { return zb[n]; });
+                    }
+                    if (NW % 2 == 1) {
+                        load_b(NW - 1);
+                        mma_steps<1>(dw + NW - 1, frag_a,
+                                     [&](int) -> const uint32_t(&)[3][4] { return zb[(NW - 1) & 1]; });
                     }
                 }
 #pragma unroll
                 for (int nb = 0; nb < NW; ++nb)
 #pragma unroll
-                    for (int j = 0; j < 2; ++j)
-                        gw[(2 * nb + j) * THREADS] = make_float4(dw[nb][j][0], dw[nb][j][1], dw[nb][j][2], dw[nb][j][3]);
+                    for (int j = 0; j < 2; ++j) {
+                        const float4 q = sums[nb][j];
+                        gw[(2 * nb + j) * THREADS] =
+                            make_float4(q.x + dw[nb][j][0], q.y + dw[nb][j][1], q.z + dw[nb][j][2], q.w + dw[nb][j][3]);
+                    }
             }
             QB_PHASE(6);  // weight gradient
             // Cotangents of layer l-1's jets: G = Zhat W^T.
             mbar_wait(wbar, wphase, a.error);
             wphase ^= 1;
-            warp_contract<S, NW, LD, PLANE, WPLANE, false>(act, wbuf, scl_z, wscl[l - 1], warp, lane, acc);
+            warp_contract<S, W, false>(act, wbuf, warp, lane, acc);
             __syncthreads();
             if (tid == 0) {
                 load_weights();
@@ -705,11 +703,7 @@ __global__ void __launch_bounds__(MmaGeom<CODE, W>::THREADS, MmaGeom<CODE, W>::M
             const int rows = a.width[l - 1], cols = a.width[l];
             float* out = my_grad + a.w_off[l];
             for (int q = 0; q < 2 * NW; ++q) {
-                float4 v = dws[((size_t)(l - 1) * 2 * NW + q) * THREADS + tid];
-                v.x = fmaf(v.x, MMA_TRUNCATION, v.x);
-                v.y = fmaf(v.y, MMA_TRUNCATION, v.y);
-                v.z = fmaf(v.z, MMA_TRUNCATION, v.z);
-                v.w = fmaf(v.w, MMA_TRUNCATION, v.w);
+                const float4 v = dws[((size_t)(l - 1) * 2 * NW + q) * THREADS + tid];
                 const int k = col0 + g, n = (q >> 1) * 16 + (q & 1) * 8 + 2 * t;
                 if (k < rows && n < cols) out[k * cols + n] = v.x;
                 if (k < rows && n + 1 < cols) out[k * cols + n + 1] = v.y;

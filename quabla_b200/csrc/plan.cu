@@ -365,7 +365,6 @@ class Plan final : public qb200_plan {
     std::vector<size_t> fused_smem_;            // per set: dynamic shared memory of its launch
     std::vector<size_t> fused_dw_, fused_dw0_;  // per set: elements of running weight-gradient sums kept in global memory
     T* fused_dw_scratch_ = nullptr;
-    float* fused_scales_ = nullptr;             // of the weight images
     // Every set has its own saved-jet scratch and gradient rows, so that the small sets run beside
     // the first one on a second stream; rows of all sets are consecutive for the final reduction.
     std::vector<size_t> fused_jet0_, fused_row0_;  // per set: first scratch element, first gradient row
@@ -730,7 +729,6 @@ qb200_status Plan<T>::init() {
             unsigned char* raw = nullptr;
             QB_TRY(dev_alloc(&raw, fused_weight_image_bytes<T>(hidden - 1, fused_entries_[0].width)));
             fused_images_ = raw;
-            QB_TRY(dev_alloc(&fused_scales_, (size_t)hidden));
         }
         return QB200_OK;
     }
@@ -1060,7 +1058,7 @@ qb200_status Plan<T>::prepare_weight_images() {
     int w_off[FUSED_MAX_LAYERS + 1];
     for (int i = 0; i < hidden_to_hidden; ++i) w_off[i] = (int)leaves_[w_leaf_[1 + i]].offset;
     cudaError_t e = fused_prep_launch<T>(d_params_, w_off, &desc_.sizes[1], &desc_.sizes[2], hidden_to_hidden, fused_entries_[0].width,
-                                      fused_images_, fused_scales_, stream_);
+                                      fused_images_, stream_);
     ++launches_;
     if (e != cudaSuccess) return fail(QB200_CUDA_ERROR, "launch of prep_weights_kernel failed: %s", cudaGetErrorString(e));
     return QB200_OK;
@@ -1116,7 +1114,6 @@ qb200_status Plan<T>::run_fused(int si, bool forward_only) {
     a.loss_cta = d_partials_ + st.partial_offset;
     a.forward_only = forward_only ? 1 : 0;
     a.weight_images = fused_images_;
-    a.image_scales = fused_scales_;
     a.dw_scratch = fused_dw_[si] > 0 ? fused_dw_scratch_ + fused_dw0_[si] : nullptr;
     a.error = d_error_;
     // Sets after the first run on the side stream, between the fork and join events of run().

@@ -1,6 +1,6 @@
 """The tensor-core fused kernels (split float32, FP64 MMA) against the CPU oracle at the edges of what they take: every padded width, unequal
 widths, one to many hidden layers (running weight-gradient sums in shared and in global memory), ragged point counts,
-every derivative signature, and operands whose blocks differ by many orders of magnitude."""
+every derivative signature, and operands that differ by many orders of magnitude, between streams and inside one block."""
 
 import math
 
@@ -88,16 +88,16 @@ def test_signatures(cuda_device, activation, width, kind, inputs, dtype):
 
 @pytest.mark.parametrize("scale", [2.0 ** -40, 2.0 ** -12, 16.0])
 def test_streams_of_very_different_size(cuda_device, scale):
-    # Derivative streams grow with the scale of the first weights, to the first and second power: block scales keep
-    # each stream's relative accuracy (a plain float16 operand would be subnormal or infinite here).
+    # Derivative streams grow with the scale of the first weights, to the first and second power: the parts have
+    # float32's range (a float16 operand would be subnormal or infinite here).
     _check([2, 64, 64, 1], 1040, "burgers", "sin", scale=scale)
 
 
 @pytest.mark.parametrize("width", [16, 32, 50, 64])
 def test_truncation_leaves_no_common_factor(cuda_device, width):
-    # The tensor core's truncation lowers every contraction by about 4e-8 of itself, which no sum over points averages
-    # out and which the residual of the heat equation amplifies (2e-6 on these gradients before the weights made up for
-    # it).  What is left is random: 1e-7 per factor (2^-23), averaged over 10,007 points; 5e-7 allows for the residual.
+    # The tensor core's truncation would lower every contraction by up to 4e-8 of itself, which no sum over points
+    # averages out and which the residual of the heat equation amplifies (2e-6 on these gradients).  What is left is
+    # random: float32's rounding (2^-24) in every factor, averaged over 10,007 points; 5e-7 allows for the residual.
     loss = workloads.make("heat3d", 128).loss
     params = workloads.init_mlp(qb.random.key(10007 + width), [4] + [width] * 4 + [1], np.float32)
     points = np.random.default_rng(10007 + width).uniform(0.0, 1.0, (10007, 4)).astype(np.float32)
@@ -111,3 +111,34 @@ def test_truncation_leaves_no_common_factor(cuda_device, width):
     exact_value, exact = step(wide, points.astype(np.float64))
     assert np.linalg.norm(flat(grads) - flat(exact)) <= 5e-7 * np.linalg.norm(flat(exact))
     assert abs(float(value) - float(exact_value)) <= 5e-7 * abs(float(exact_value))
+
+
+@pytest.mark.parametrize("width", [16, 50, 64])
+@pytest.mark.parametrize("place", ["columns", "rows", "output"])
+@pytest.mark.parametrize("power", [12, 30])
+def test_every_entry_keeps_its_own_size(cuda_device, width, place, power):
+    # Every third column or row of a hidden weight, or every third output weight, is 2^-power of its neighbours in the same
+    # 16 x 16 block.  Columns and rows of all weight gradients are right relative to themselves, not to the largest
+    # (with an exponent shared by a block they were off by up to 5e-2 at 2^-30): 2^-24 for each of some hundred factors
+    # and sums per entry and an amplification of a few by the second derivative.
+    loss = workloads.make("poisson2d", 128).loss
+    params = workloads.init_mlp(qb.random.key(3), [2] + [width] * 3 + [1], np.float32)
+    f = np.where(np.arange(width) % 3 == 1, 2.0 ** -power, 1.0).astype(np.float32)
+    if place == "columns":
+        params[1]["w"] = params[1]["w"] * f[None, :]
+    elif place == "rows":
+        params[1]["w"] = params[1]["w"] * f[:, None]
+    else:
+        params[-1]["w"] = params[-1]["w"] * f[:, None]
+    rng = np.random.default_rng(width)
+    interior = rng.uniform(0.0, 1.0, (2003, 2)).astype(np.float32)
+    edge = rng.uniform(0.0, 1.0, (124, 2)).astype(np.float32)
+    step = qb.jit(qb.value_and_grad(loss), device="cuda:0")
+    _, grads = step(params, interior, edge)
+    _, exact = step([{k: v.astype(np.float64) for k, v in layer.items()} for layer in params],
+                    interior.astype(np.float64), edge.astype(np.float64))
+    for i in range(3):
+        g, e = grads[i]["w"].astype(np.float64), exact[i]["w"]
+        for axis in (0, 1):
+            error = np.linalg.norm(g - e, axis=axis) / np.linalg.norm(e, axis=axis)
+            assert error.max() <= 2e-5, (i, axis, error.max())
