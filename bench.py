@@ -348,8 +348,11 @@ class Rig:
         return sum(a.elapsed_time(b) for a, b in zip(starts, stops))
 
 
-ENGINES = {0: "layer-wise (FP64 tensor-core / SIMT GEMMs)", 1: "fused (FP32/FP64 pipe)",
-           2: "fused (tensor cores, float16 pairs)", 3: "layer-wise (tcgen05 split-float32 GEMMs)"}
+ENGINES = {0: "layer-wise (FP64 tensor-core / SIMT GEMMs)", 3: "layer-wise (tcgen05 split-float32 GEMMs)"}
+# Fused kernels by QB200_Q_FUSED_KERNEL: (engine, name, tensor-pipe passes per FLOP at the bf16 rate).
+FUSED = {1: ("fused (FP32 pipe)", "fused_step_kernel", 0.0),
+         2: ("fused (tensor cores, three bfloat16 parts)", "fused_mma_kernel", 7.0),
+         3: ("fused (FP64 MMA)", "fused_dmma_kernel", 0.0)}
 
 
 def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: int, peaks: dict, live: dict,
@@ -372,13 +375,14 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
     launches0 = plan.query(_lib.Q_KERNEL_LAUNCHES)
     device_ms = rig.timed_loop(plan, trainer.step, steps, flush_between)
     launches = plan.query(_lib.Q_KERNEL_LAUNCHES) - launches0
-    engine = plan.query(_lib.Q_ENGINE)
+    engine, fused = plan.query(_lib.Q_ENGINE), plan.query(_lib.Q_FUSED_KERNEL)
+    engine_name, fused_name, fused_passes = FUSED.get(fused, (ENGINES.get(engine), None, 0.0))
     interior = plan.spec.sets[0]
     local_points = interior.n_points
     # Dominant kernel, from the last timed step: the layer GEMM launches of the layer-wise engines
     # (an event pair around each), the interior set's one fused launch on the fused engines.
     lanes = plan.query(_lib.Q_LANES)
-    if engine in (0, 3):
+    if not fused:
         if lanes > 1:
             # Chunks overlap on two streams in the timed loop, so an event pair there spans more than its kernel:
             # time the GEMM launches in two more steps with every chunk on one stream (outside the timed loop).
@@ -404,9 +408,9 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
     else:
         set0_ns = plan.query(_lib.Q_SET0_NANOSECONDS)
         flops = w.flops_per_point(interior.streams) * local_points
-        kernel = {"name": "fused_mma_kernel" if engine == 2 else "fused_step_kernel", "launches_per_step": 1,
+        kernel = {"name": fused_name, "launches_per_step": 1,
                   "us_per_launch": set0_ns * 1e-3, "flops_per_launch": flops, "us_per_step": set0_ns * 1e-3,
-                  "bf16_rate_passes_per_flop": 3.0 if engine == 2 else 6.0 if dtype_name == "f32" else 0.0}
+                  "bf16_rate_passes_per_flop": fused_passes}
         achieved = flops / max(set0_ns, 1) * 1e-3
     allreduce_us = plan.query(_lib.Q_ALLREDUCE_NANOSECONDS) * 1e-3 if rig.world > 1 else 0.0
 
@@ -462,7 +466,7 @@ def measure(rig: Rig, name: str, total_points: int | None, steps: int, warmup: i
         peak_source = "torch.matmul float64 4096^3, best of 5, timed at start-up of this run"
     out = {
         "workload": w.name, "dtype": dtype_name, "interior_points": total_points_run, "ms_per_step": ms_per_step,
-        "points_per_s": total_points_run / (ms_per_step * 1e-3), "engine": ENGINES[engine], "streams": streams,
+        "points_per_s": total_points_run / (ms_per_step * 1e-3), "engine": engine_name, "streams": streams,
         "reference_streams": w.streams, "merged_second_order": interior.merge_weights is not None,
         "step_tflops": step_flops / (ms_per_step * 1e-3) / 1e12 / 1.0,
         "kernel": kernel, "kernel_tflops": achieved, "peak_tflops": peak, "peak_source": peak_source,

@@ -90,8 +90,8 @@ typedef enum qb200_query {
     QB200_Q_FLAT_DEVICE_PTR = 6,     /* device address of the flat [loss, gradients...] buffer */
     QB200_Q_SCRATCH_BYTES = 7,       /* bytes of saved-jet scratch the plan holds */
     QB200_Q_STEP_COUNT = 8,          /* optimizer updates applied so far */
-    QB200_Q_ENGINE = 9,              /* 0: layer-wise (FP pipe), 1: fused, float64 or widths up to 32, 2: fused, float32, widths above 32,
-                                        3: layer-wise with tcgen05 GEMMs */
+    QB200_Q_ENGINE = 9,              /* 0: layer-wise, 1: fused, float64 or widths up to 32, 2: fused, float32, widths above 32,
+                                        3: layer-wise with tcgen05 GEMMs; which kernel a fused plan runs: QB200_Q_FUSED_KERNEL */
     QB200_Q_SET0_NANOSECONDS = 10,   /* device time of the last execute's kernels for point set 0 (events) */
     QB200_Q_ALLREDUCE_NANOSECONDS = 11, /* device time of the last execute's gradient all-reduce, waits for peers included */
     QB200_Q_GEMM_NANOSECONDS = 12,   /* with QB200_OPT_KERNEL_TIMERS: summed device time of the last execute's layer GEMM launches
@@ -99,9 +99,11 @@ typedef enum qb200_query {
     QB200_Q_GEMM_LAUNCHES = 13,      /* ... how many launches that sum covers */
     QB200_Q_GEMM_FLOPS = 14,         /* ... and their 2*M*N*K in total */
     QB200_Q_LANES = 15,              /* streams over which the layer-wise engine spreads consecutive chunks (1 or 2) */
-    QB200_Q_GEMM_PIPE_FLOPS = 16     /* ... the tensor-pipe work of those launches in FLOPs at the bfloat16 rate: 2*M*N*K times 6 where the
+    QB200_Q_GEMM_PIPE_FLOPS = 16,    /* ... the tensor-pipe work of those launches in FLOPs at the bfloat16 rate: 2*M*N*K times 6 where the
                                         three products of an element are tf32 instructions (tf32 runs at half the bfloat16 rate), times 4
                                         where the two correction products are bfloat16 instructions; 0 for float64 and SIMT launches */
+    QB200_Q_FUSED_KERNEL = 17        /* kernel of a fused plan: 1 fused_step_kernel (FP32 pipe), 2 fused_mma_kernel (float32 in bfloat16 parts on the
+                                        tensor cores), 3 fused_dmma_kernel (FP64 MMA); 0 on the layer-wise engine */
 } qb200_query;
 
 /* Keys of qb200_plan_set_option. */

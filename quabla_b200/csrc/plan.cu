@@ -1839,6 +1839,7 @@ qb200_status Plan<T>::query(int key, int64_t* out) {
         case QB200_Q_SCRATCH_BYTES: *out = (int64_t)scratch_bytes_; return QB200_OK;
         case QB200_Q_STEP_COUNT: *out = steps_; return QB200_OK;
         case QB200_Q_ENGINE: *out = fused_ ? (fused_tensor_core_ && sizeof(T) == 4 && fused_width_ > 32 ? 2 : 1) : (tc_any_ ? 3 : 0); return QB200_OK;
+        case QB200_Q_FUSED_KERNEL: *out = !fused_ ? 0 : !fused_tensor_core_ ? 1 : sizeof(T) == 4 ? 2 : 3; return QB200_OK;
         case QB200_Q_ALLREDUCE_NANOSECONDS: {
             if (!ev_ar_valid_) {
                 *out = 0;  // no communicator attached, or no execute yet

@@ -30,7 +30,7 @@ def main() -> None:
     errors = [relative_error(outputs[0], expected_loss)]
     for got, expected in zip(outputs[1:], expected_grads):
         errors.append(relative_error(got.reshape(expected.shape), expected))
-    print(json.dumps({"engine": plan.query(_lib.Q_ENGINE), "launches": plan.query(_lib.Q_KERNEL_LAUNCHES),
+    print(json.dumps({"engine": plan.query(_lib.Q_ENGINE), "kernel": plan.query(_lib.Q_FUSED_KERNEL), "launches": plan.query(_lib.Q_KERNEL_LAUNCHES),
                       "max_error": float(np.max(errors)), "loss": float(outputs[0]),
                       "streams": compiled.spec.sets[0].streams}))
     plan.close()

@@ -31,6 +31,7 @@ def _run(name, points, **switches):
 def test_wide_float32_network_on_every_gemm_variant(cuda_device, switches):
     result = _run("heat3d", 640, **switches)
     assert result["engine"] == (0 if switches.get("QB200_TC") == "0" else 3)
+    assert result["kernel"] == 0
     assert result["max_error"] <= TOLERANCE[np.dtype(np.float32)]
 
 
@@ -69,12 +70,12 @@ def test_narrow_network_forced_onto_the_layerwise_engine(cuda_device, correction
 
 
 @pytest.mark.parametrize("name,points", [("poisson2d", 3000), ("beam", 2500)])
-@pytest.mark.parametrize("switches", [{}, {"QB200_FUSED_TILE": "32"}, {"QB200_FUSED": "simt"}],
-                         ids=["two CTAs per SM", "one CTA per SM", "simt"])
+@pytest.mark.parametrize("switches", [{}, {"QB200_FUSED": "simt"}], ids=["tensor cores", "simt"])
 def test_fused_engine_variants(cuda_device, name, points, switches):
     # Ragged point counts: the last tile of both tile sizes is partial.
     result = _run(name, points, **switches)
     assert result["engine"] == (1 if switches.get("QB200_FUSED") == "simt" else 2)
+    assert result["kernel"] == (1 if switches.get("QB200_FUSED") == "simt" else 2)
     assert result["max_error"] <= TOLERANCE[np.dtype(np.float32)]
 
 

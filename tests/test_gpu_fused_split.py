@@ -56,6 +56,7 @@ def _check(sizes, points, kind, activation="tanh", scale=1.0, dtype=np.float32):
     args = (params, p)
     compiled = CompiledLoss(loss, args, (0,), 0)
     assert compiled.plan.query(_lib.Q_ENGINE) in (1, 2)
+    assert compiled.plan.query(_lib.Q_FUSED_KERNEL) == (2 if np.dtype(dtype) == np.float32 else 3)
     spec = compiled.spec.unmerged or compiled.spec
     value, grads = contracted.value_and_grad(spec, compiled.named_inputs(args), threads=contracted.max_threads())
     compiled.bind(args)
