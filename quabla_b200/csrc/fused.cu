@@ -13,18 +13,18 @@ namespace qb {
 
 namespace {
 
-template <typename T, int W, int CODE, int ACT>
-FusedEntry<T> make_entry() {
-    typedef FusedGeom<T, W, CODE> G;
-    FusedEntry<T> e;
-    e.kernel = fused_step_kernel<T, W, CODE, ACT>;
+template <int CODE>
+FusedEntry<float> simt_entry() {
+    typedef FusedGeom<CODE> G;
+    FusedEntry<float> e;
+    e.kernel = fused_step_kernel<CODE>;
     e.streams = G::S;
     e.tile_points = G::TP;
     e.smem_bytes = G::SMEM_BASE_BYTES;
     e.scratch_per_layer = G::SCRATCH_PER_CTA;
     e.tensor_core = false;
     e.dw_bytes = 0;
-    e.width = W;
+    e.width = G::W;
     e.threads = FUSED_THREADS;
     e.ctas_per_sm = 1;
     return e;
@@ -42,10 +42,10 @@ bool want_simt() {
 // Signature codes: 0 = value only; 1 = {1}; 2 = {2}; 3 = {3}; 4 = {4}; 6 = {1,1};
 // 7 = {2,1}; 11 = {1,2}; 12 = {2,2}; SIG_MERGED + 6 / 31 = {1,1} / {1,1,1} plus the merged
 // second-order stream (2-D / 3-D Laplacian).
-#define QB_CASE(T, W, CODE)                       \
-    if (width == W && code == CODE) {             \
-        *out = make_entry<T, W, CODE, ACT_TANH>(); \
-        return true;                              \
+#define QB_CASE(CODE)               \
+    if (code == CODE) {             \
+        *out = simt_entry<CODE>();  \
+        return true;                \
     }
 
 template <typename T>
@@ -61,9 +61,8 @@ template <>
 bool fused_lookup<float>(int width, bool uniform, int layers, int code, int act, FusedEntry<float>* out) {
     if (act != ACT_TANH && act != ACT_SIN) return false;
     if (want_simt()) {
-        if (!uniform || act != ACT_TANH) return false;
-        QB_CASE(float, 64, 0) QB_CASE(float, 64, 1) QB_CASE(float, 64, 2) QB_CASE(float, 64, 4)
-        QB_CASE(float, 64, 7) QB_CASE(float, 64, 12) QB_CASE(float, 64, SIG_MERGED + 6)
+        if (width != 64 || !uniform || act != ACT_TANH) return false;
+        QB_CASE(0) QB_CASE(1) QB_CASE(2) QB_CASE(4) QB_CASE(7) QB_CASE(12) QB_CASE(SIG_MERGED + 6)
         return false;
     }
     return padded_lookup<float>(width, layers, code, act, out);

@@ -10,8 +10,10 @@
 // 1792-2972: one kernel per IR node; op/vjp.rs:176-209: a materialised
 // [B, in, out] product per weight gradient).
 //
-// Shapes: every hidden layer has the same width W, the input
-// width d0 <= 4, the output width 1.  A CTA of 256 threads owns a tile of TP
+// Shapes: float32 tanh networks whose hidden layers all have width 64, the input
+// width d0 <= 4, the output width 1 (QB200_FUSED=simt; by default the tensor-core
+// kernels, fused_mma_kernel.cuh and fused_dmma_kernel.cuh, run these and all
+// other narrow shapes).  A CTA of 256 threads owns a tile of TP
 // points; thread (tp, tn) holds, for 2 points x 4 units, ALL S streams in
 // registers, so the tanh-jet composition and its transpose are register-only.
 #pragma once
@@ -96,44 +98,25 @@ struct FusedArgs {
     int* error;                 // set to 1 when a bounded wait inside the kernel gave up
 };
 
-template <typename T> struct Pack2;
-template <> struct Pack2<float> { typedef float2 type; };
-template <> struct Pack2<double> { typedef double2 type; };
-
-template <typename T>
-__device__ __forceinline__ void ld2(const T* p, T& a, T& b) {
-    const typename Pack2<T>::type v = *reinterpret_cast<const typename Pack2<T>::type*>(p);
+__device__ __forceinline__ void ld2(const float* p, float& a, float& b) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
     a = v.x;
     b = v.y;
 }
-template <typename T>
-__device__ __forceinline__ void st2(T* p, T a, T b) {
-    typename Pack2<T>::type v;
-    v.x = a;
-    v.y = b;
-    *reinterpret_cast<typename Pack2<T>::type*>(p) = v;
-}
+__device__ __forceinline__ void st2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 __device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
     const float4 q = *reinterpret_cast<const float4*>(p);
     v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
 }
-__device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
-    const double2 a = *reinterpret_cast<const double2*>(p);
-    const double2 b = *reinterpret_cast<const double2*>(p + 2);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
 __device__ __forceinline__ void st4(float* p, const float (&v)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
-__device__ __forceinline__ void st4(double* p, const double (&v)[4]) {
-    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
-    *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
-}
 
 // Geometry shared by host (shared-memory size, scratch size) and device.
-template <typename T, int W, int CODE>
+template <int CODE>
 struct FusedGeom {
     typedef Sig<CODE> sig;
+    static constexpr int W = 64;
     static constexpr int S = sig::S;
     static constexpr int CG = W / 4;                  // column groups (4 units each)
     static constexpr int PG = FUSED_THREADS / CG;     // point groups (2 points each)
@@ -142,7 +125,7 @@ struct FusedGeom {
     static constexpr int ROWP = ROWS + 4;             // stride of the k-major activation buffer
     static constexpr int WP = W + 4;                  // stride of the row-major buffers
     static constexpr int MT = W / 16;                 // weight-gradient micro-tile per thread
-    // shared-memory regions, in elements of T
+    // shared-memory regions, in elements
     static constexpr int OFF_ACT = 0;                          // [W][ROWP]  k-major A operand
     static constexpr int OFF_HR = OFF_ACT + W * ROWP;          // [ROWS][WP] previous-layer jets, row-major
     static constexpr int OFF_ZR = OFF_HR + ROWS * WP;          // [ROWS][WP] pre-activation cotangents
@@ -152,28 +135,28 @@ struct FusedGeom {
     static constexpr int OFF_UH = OFF_U + ROWS;                // [S][TP]    their cotangents
     static constexpr int TOTAL = OFF_UH + ROWS;
     // plus 16 bytes per instruction of the residual program, staged after these regions
-    static constexpr size_t SMEM_BASE_BYTES = ((size_t)TOTAL * sizeof(T) + 15) / 16 * 16;
+    static constexpr size_t SMEM_BASE_BYTES = ((size_t)TOTAL * sizeof(float) + 15) / 16 * 16;
     static constexpr size_t SCRATCH_PER_CTA = (size_t)S * TP * W;  // elements per layer per buffer
 };
 
 // acc[s][i][j] = sum_k A[k][s*TP + 2*tp + i] * B[k][4*tn + j], k < K.
-template <typename T, int S, int TP, int ROWP, int WP>
-__device__ __forceinline__ void tile_gemm(const T* __restrict__ A, const T* __restrict__ B, int K, int tp, int tn,
-                                          T (&acc)[S][2][4]) {
+template <int S, int TP, int ROWP, int WP>
+__device__ __forceinline__ void tile_gemm(const float* __restrict__ A, const float* __restrict__ B, int K, int tp, int tn,
+                                          float (&acc)[S][2][4]) {
 #pragma unroll
     for (int s = 0; s < S; ++s)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[s][i][j] = T(0);
+            for (int j = 0; j < 4; ++j) acc[s][i][j] = 0.0f;
 #pragma unroll 4
     for (int k = 0; k < K; ++k) {
-        T b[4];
+        float b[4];
         ld4(B + k * WP + 4 * tn, b);
-        const T* arow = A + k * ROWP + 2 * tp;
+        const float* arow = A + k * ROWP + 2 * tp;
 #pragma unroll
         for (int s = 0; s < S; ++s) {
-            T a0, a1;
+            float a0, a1;
             ld2(arow + s * TP, a0, a1);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -267,65 +250,65 @@ __device__ __forceinline__ void jet_apply_transposed(const T (&z)[SG::S], T (&g)
     jet_apply_transposed_with<T, SG, MW>(d, z, g, mw);
 }
 
-template <typename T, int W, int CODE, int ACT>
-__global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<T> a) {
-    typedef FusedGeom<T, W, CODE> G;
+template <int CODE>
+__global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<float> a) {
+    typedef FusedGeom<CODE> G;
     typedef Sig<CODE> SG;
-    constexpr int S = G::S, TP = G::TP, CG = G::CG, PG = G::PG, ROWP = G::ROWP, WP = G::WP, ROWS = G::ROWS,
+    constexpr int W = G::W, S = G::S, TP = G::TP, CG = G::CG, PG = G::PG, ROWP = G::ROWP, WP = G::WP, ROWS = G::ROWS,
                   MT = G::MT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* smem = reinterpret_cast<T*>(smem_raw);
-    T* act = smem + G::OFF_ACT;
-    T* hr = smem + G::OFF_HR;
-    T* zr = smem + G::OFF_ZR;
-    T* wb = smem + G::OFF_WB;
-    T* red = smem + G::OFF_RED;
-    T* us = smem + G::OFF_U;
-    T* uh = smem + G::OFF_UH;
-    int4* code = reinterpret_cast<int4*>(smem_raw + (((size_t)G::TOTAL * sizeof(T) + 15) / 16) * 16);
+    float* smem = reinterpret_cast<float*>(smem_raw);
+    float* act = smem + G::OFF_ACT;
+    float* hr = smem + G::OFF_HR;
+    float* zr = smem + G::OFF_ZR;
+    float* wb = smem + G::OFF_WB;
+    float* red = smem + G::OFF_RED;
+    float* us = smem + G::OFF_U;
+    float* uh = smem + G::OFF_UH;
+    int4* code = reinterpret_cast<int4*>(smem_raw + (((size_t)G::TOTAL * sizeof(float) + 15) / 16) * 16);
 
     const int tid = threadIdx.x;
     const int tn = tid % CG, tp = tid / CG;
     const int L = a.L, d0 = a.d0;
     const bool backward = a.forward_only == 0;
-    T* my_grad = a.grad_cta + (size_t)blockIdx.x * a.P;
-    T* sz = a.scratch_z + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
-    T* sh = a.scratch_h + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
+    float* my_grad = a.grad_cta + (size_t)blockIdx.x * a.P;
+    float* sz = a.scratch_z + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
+    float* sh = a.scratch_h + (size_t)blockIdx.x * L * G::SCRATCH_PER_CTA;
 
     for (int i = tid; i < a.prog.n_instr; i += FUSED_THREADS) code[i] = a.prog.code[i];
     if (backward)
-        for (int i = tid; i < a.P; i += FUSED_THREADS) my_grad[i] = T(0);
+        for (int i = tid; i < a.P; i += FUSED_THREADS) my_grad[i] = 0.0f;
     double loss_sum = 0.0;  // threads < TP: one point each
-    const T seed = a.cotangent[0] * a.weight * a.extra;
+    const float seed = a.cotangent[0] * a.weight * a.extra;
     __syncthreads();
 
     const long long n_tiles = (a.n_points + TP - 1) / TP;
     for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const long long p0 = tile * TP;
-        T acc[S][2][4];
-        T x[2][4];  // the coordinates of this thread's two points
+        float acc[S][2][4];
+        float x[2][4];  // the coordinates of this thread's two points
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const long long p = min(p0 + 2 * tp + i, a.n_points - 1);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) x[i][k] = k < d0 ? a.table[p * a.ncols + k] : T(0);
+            for (int k = 0; k < 4; ++k) x[i][k] = k < d0 ? a.table[p * a.ncols + k] : 0.0f;
         }
 
         // ------------------------------ forward ------------------------------
         for (int l = 0; l < L; ++l) {
             if (l == 0) {
                 // First layer: K = d0 <= 4; the derivative streams see the direction vectors.
-                const T* w0 = a.params + a.w_off[0];
+                const float* w0 = a.params + a.w_off[0];
 #pragma unroll
                 for (int s = 0; s < S; ++s)
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) acc[s][i][j] = T(0);
+                        for (int j = 0; j < 4; ++j) acc[s][i][j] = 0.0f;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (k < d0) {
-                        T wrow[4];
+                        float wrow[4];
                         ld4(w0 + k * W + 4 * tn, wrow);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
@@ -334,7 +317,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
                         }
 #pragma unroll
                         for (int dj = 0; dj < SG::ndirs; ++dj) {
-                            const T v = a.dirs[dj * d0 + k];
+                            const float v = a.dirs[dj * d0 + k];
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
                                 acc[SG::base(dj)][0][j] += v * wrow[j];
@@ -344,14 +327,14 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
                     }
                 }
             } else {
-                const T* wl = a.params + a.w_off[l];
+                const float* wl = a.params + a.w_off[l];
                 for (int e = tid; e < W * W; e += FUSED_THREADS) wb[(e / W) * WP + (e % W)] = wl[e];
                 __syncthreads();  // weights and the previous epilogue's activations are in place
-                tile_gemm<T, S, TP, ROWP, WP>(act, wb, W, tp, tn, acc);
+                tile_gemm<S, TP, ROWP, WP>(act, wb, W, tp, tn, acc);
                 __syncthreads();  // every thread is done reading act and wb
             }
             if (a.b_off[l] >= 0) {
-                T bias[4];
+                float bias[4];
                 ld4(a.params + a.b_off[l] + 4 * tn, bias);
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
@@ -359,8 +342,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
                     for (int j = 0; j < 4; ++j) acc[0][i][j] += bias[j];
             }
             // Save the pre-activations, compose with tanh, save and stage the jets.
-            T* zl = sz + (size_t)l * G::SCRATCH_PER_CTA;
-            T* hl = sh + (size_t)l * G::SCRATCH_PER_CTA;
+            float* zl = sz + (size_t)l * G::SCRATCH_PER_CTA;
+            float* hl = sh + (size_t)l * G::SCRATCH_PER_CTA;
             if (backward) {
 #pragma unroll
                 for (int s = 0; s < S; ++s)
@@ -371,10 +354,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
             for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    T v[S];
+                    float v[S];
 #pragma unroll
                     for (int s = 0; s < S; ++s) v[s] = acc[s][i][j];
-                    jet_apply<T, SG, ACT>(v, a.merge_w);
+                    jet_apply<float, SG, ACT_TANH>(v, a.merge_w);
 #pragma unroll
                     for (int s = 0; s < S; ++s) acc[s][i][j] = v[s];
                 }
@@ -394,13 +377,13 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
         }
 
         // ------------------------- head and residual -------------------------
-        T wh[4];
+        float wh[4];
         ld4(a.params + a.w_off[L] + 4 * tn, wh);
 #pragma unroll
         for (int s = 0; s < S; ++s)
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                T dot = T(0);
+                float dot = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) dot += acc[s][i][j] * wh[j];
 #pragma unroll
@@ -413,14 +396,14 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
             const bool valid = p < a.n_points;
             const long long pc = valid ? p : a.n_points - 1;
             if (a.b_off[L] >= 0) us[tid] += a.params[a.b_off[L]];
-            T r[MAX_REGS];
-            run_program<T>(code, a.prog.n_instr, static_cast<const T*>(a.prog.consts), a.table + pc * a.ncols, us + tid,
+            float r[MAX_REGS];
+            run_program<float>(code, a.prog.n_instr, static_cast<const float*>(a.prog.consts), a.table + pc * a.ncols, us + tid,
                            TP, r);
             if (valid) loss_sum += (double)r[a.prog.value_reg];
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 const int reg = a.prog.grad_regs[s];
-                uh[s * TP + tid] = (valid && reg >= 0) ? seed * r[reg] : T(0);
+                uh[s * TP + tid] = (valid && reg >= 0) ? seed * r[reg] : 0.0f;
             }
         }
         if (!backward) {
@@ -432,10 +415,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
         // ------------------------------ backward ------------------------------
         // Head: dW = sum h * uhat, db = sum uhat(primal), G = uhat (x) w.
         {
-            T ug[S][2];
+            float ug[S][2];
 #pragma unroll
             for (int s = 0; s < S; ++s) ld2(uh + s * TP + 2 * tp, ug[s][0], ug[s][1]);
-            T pw[4] = {T(0), T(0), T(0), T(0)};
+            float pw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int s = 0; s < S; ++s)
 #pragma unroll
@@ -448,12 +431,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
             st4(red + tp * W + 4 * tn, pw);
             __syncthreads();
             if (tid < W) {
-                T total = T(0);
+                float total = 0.0f;
                 for (int g = 0; g < PG; ++g) total += red[g * W + tid];
                 my_grad[a.w_off[L] + tid] += total;
             }
             if (tid == 0 && a.b_off[L] >= 0) {
-                T total = T(0);
+                float total = 0.0f;
                 for (int p = 0; p < TP; ++p) total += uh[p];
                 my_grad[a.b_off[L]] += total;
             }
@@ -461,28 +444,28 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
         }
         for (int l = L - 1; l >= 0; --l) {
             // acc holds the cotangents of layer l's jets; turn them into cotangents of its pre-activations.
-            const T* zl = sz + (size_t)l * G::SCRATCH_PER_CTA;
+            const float* zl = sz + (size_t)l * G::SCRATCH_PER_CTA;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                T zs[S][4];
+                float zs[S][4];
 #pragma unroll
                 for (int s = 0; s < S; ++s) ld4(zl + ((size_t)s * TP + 2 * tp + i) * W + 4 * tn, zs[s]);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    T z[S], g[S];
+                    float z[S], g[S];
 #pragma unroll
                     for (int s = 0; s < S; ++s) {
                         z[s] = zs[s][j];
                         g[s] = acc[s][i][j];
                     }
-                    jet_apply_transposed<T, SG, ACT>(z, g, a.merge_w);
+                    jet_apply_transposed<float, SG, ACT_TANH>(z, g, a.merge_w);
 #pragma unroll
                     for (int s = 0; s < S; ++s) acc[s][i][j] = g[s];
                 }
             }
             // Bias gradient partials (primal stream) and, for the first layer, the weight gradient partials.
             {
-                T pb[4];
+                float pb[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) pb[j] = acc[0][0][j] + acc[0][1][j];
                 st4(red + tp * 5 * W + 4 * tn, pb);
@@ -491,12 +474,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (k < d0) {
-                        T pw[4];
+                        float pw[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) pw[j] = x[0][k] * acc[0][0][j] + x[1][k] * acc[0][1][j];
 #pragma unroll
                         for (int dj = 0; dj < SG::ndirs; ++dj) {
-                            const T v = a.dirs[dj * d0 + k];
+                            const float v = a.dirs[dj * d0 + k];
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
                                 pw[j] += v * (acc[SG::base(dj)][0][j] + acc[SG::base(dj)][1][j]);
@@ -507,7 +490,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
                 __syncthreads();
                 for (int e = tid; e < (1 + d0) * W; e += FUSED_THREADS) {
                     const int which = e / W, n = e % W;
-                    T total = T(0);
+                    float total = 0.0f;
                     for (int g = 0; g < PG; ++g) total += red[(g * 5 + which) * W + n];
                     if (which == 0) {
                         if (a.b_off[0] >= 0) my_grad[a.b_off[0] + n] += total;
@@ -529,33 +512,33 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
                 for (int i = 0; i < 2; ++i) st4(zr + (s * TP + 2 * tp + i) * WP + 4 * tn, acc[s][i]);
             }
             {
-                const T* hp = sh + (size_t)(l - 1) * G::SCRATCH_PER_CTA;
+                const float* hp = sh + (size_t)(l - 1) * G::SCRATCH_PER_CTA;
                 for (int e = tid; e < ROWS * CG; e += FUSED_THREADS) {
                     const int row = e / CG, c4 = e % CG;
-                    T v[4];
+                    float v[4];
                     ld4(hp + (size_t)row * W + 4 * c4, v);
                     st4(hr + row * WP + 4 * c4, v);
                 }
-                const T* wl = a.params + a.w_off[l];
+                const float* wl = a.params + a.w_off[l];
                 for (int e = tid; e < W * W; e += FUSED_THREADS) wb[(e % W) * WP + (e / W)] = wl[e];
             }
             __syncthreads();
             if (tid < W && a.b_off[l] >= 0) {
-                T total = T(0);
+                float total = 0.0f;
                 for (int g = 0; g < PG; ++g) total += red[g * 5 * W + tid];
                 my_grad[a.b_off[l] + tid] += total;
             }
             // Weight gradient of layer l: dW[k][n] += sum_rows hr[row][k] * zr[row][n].
             {
                 const int ty = tid / 16, tx = tid % 16;
-                T dw[MT][MT];
+                float dw[MT][MT];
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
 #pragma unroll
-                    for (int j = 0; j < MT; ++j) dw[i][j] = T(0);
+                    for (int j = 0; j < MT; ++j) dw[i][j] = 0.0f;
 #pragma unroll 4
                 for (int row = 0; row < ROWS; ++row) {
-                    T hv[MT], zv[MT];
+                    float hv[MT], zv[MT];
 #pragma unroll
                     for (int i = 0; i < MT; ++i) hv[i] = hr[row * WP + ty * MT + i];
 #pragma unroll
@@ -565,14 +548,14 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) fused_step_kernel(FusedArgs<
 #pragma unroll
                         for (int j = 0; j < MT; ++j) dw[i][j] += hv[i] * zv[j];
                 }
-                T* gw = my_grad + a.w_off[l];
+                float* gw = my_grad + a.w_off[l];
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
 #pragma unroll
                     for (int j = 0; j < MT; ++j) gw[(ty * MT + i) * W + tx * MT + j] += dw[i][j];
             }
             // Cotangents of layer l-1's jets: G = Zhat W^T.
-            tile_gemm<T, S, TP, ROWP, WP>(act, wb, W, tp, tn, acc);
+            tile_gemm<S, TP, ROWP, WP>(act, wb, W, tp, tn, acc);
             __syncthreads();
         }
     }
