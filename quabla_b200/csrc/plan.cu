@@ -588,10 +588,13 @@ qb200_status Plan<T>::init() {
         const char* env = getenv("QB200_LANES");
         const int asked = env != nullptr ? atoi(env) : 0;
         if (largest >= 16384 && (asked == 2 || (asked != 1 && sizeof(T) == 8))) n_lanes = 2;
-        // Plans that keep one lane for their largest set send the other sets down a second one: a boundary set is some
-        // fifty launches of a few microseconds each, which come on top of the interior's work on its stream and cost next to
-        // nothing beside it (Burgers gradients, 10,007 + 312 + 312 points: 2682 us on one lane, 1995 us on two).  Only
-        // where no set is cut into chunks by half the scratch budget.
+        // Plans that keep one lane for their largest set, of either dtype, send the other sets down a second one: a boundary
+        // set is some fifty launches of a few microseconds each, which come on top of the interior's work on its stream
+        // and cost next to nothing beside it.  One lane and two, in microseconds: float64 Burgers gradients, width
+        // 128, 10,007 + 312 + 312 points 2430 and 1764; float32 (tcgen05 GEMMs) the same 1173 and 868, with 1,000 interior
+        // points 763 and 485, with 65,536 2764 and 2376; 2-D Poisson, width 256, 2,003 points 382 and 261, 65,536 2904 and
+        // 2731, width 128, 262,144 3914 and 3858.  Two were ahead at all of 25 sizes: beside sets this short the clock of
+        // the float32 GEMMs does not matter.  Only where no set is cut into chunks by half the scratch budget.
         if (n_lanes == 1 && asked != 1 && desc_.sets.size() > 1) {
             by_set_ = true;
             for (size_t si = 0; si < desc_.sets.size(); ++si) {
@@ -1026,9 +1029,12 @@ bool Plan<T>::choose_fused() {
         if (!s.merge_w.empty()) code += SIG_MERGED;
         FusedEntry<T>& entry = fused_entries_[si];
         if (!fused_lookup<T>(width, uniform, hidden, code, desc_.activation, &entry)) return false;
-        // The layer-wise engine costs some nine launches per layer and point set, the fused one a launch per set: for
-        // every width and signature it is ahead from four layers (over all sets) or PADDED_MIN_POINTS points on.
-        // Below that only the widths 16, 32 and 64 that fill their kernels take it.
+        // A fused kernel is ahead of the layer-wise engine wherever there is one (one to three hidden layers of 8 to 64
+        // units, 64 to 1,500 points of one set, both dtypes: 17 to 51 us against 35 to 240 us a step; the layer-wise engine
+        // costs some nine launches per layer and point set).  Excepted are the smallest plans that ran layer by layer
+        // before these shapes had a fused kernel: fewer than four layers over all sets, fewer than PADDED_MIN_POINTS points,
+        // and a shape that was not one of the FP32/FP64-pipe kernels' (`fills`).  They keep that engine, and with it
+        // its results, to the bit; the cost is the difference above.
         const bool fills = uniform && (sizeof(T) == 4 ? width == 16 || width == 32 || width == 64
                                                       : (width == 16 || width == 32) && s.merge_w.empty());
         if (entry.tensor_core && !fills && hidden * (int)desc_.sets.size() < 4 && points < PADDED_MIN_POINTS) return false;

@@ -85,3 +85,32 @@ def test_time_of_the_first_set_on_either_lane(cuda_device, first, second):
     alone = sorted(times())[2]
     # Two lanes halve the time of a set cut into chunks at best.
     assert min(both) >= 0.4 * alone, (both, alone)
+
+
+@pytest.mark.parametrize("first,second,width", [(3001, 312, 128), (130, 3001, 256), (16500, 16500, 64 * 3)])
+def test_float32_sets_on_two_lanes(cuda_device, monkeypatch, first, second, width):
+    # tcgen05 GEMMs of two lanes at once, launched one by one and captured: repeatable, equal to one lane to the rounding
+    # of a float32 result (the lanes' sums are double), and as near to float64 as the parity gate asks.
+    loss, args = _two_sets(first, second, np.float32, width)
+    results = {}
+    for lanes in ("1", None):
+        if lanes is None:
+            monkeypatch.delenv("QB200_LANES")
+        else:
+            monkeypatch.setenv("QB200_LANES", lanes)
+        compiled = CompiledLoss(loss, args, (0,), 0)
+        assert compiled.plan.query(_lib.Q_LANES) == (1 if lanes else 2) and compiled.plan.query(_lib.Q_ENGINE) == 3
+        compiled.bind(args)
+        runs = []
+        for _ in range(4):
+            compiled.plan.execute()
+            runs.append([o.copy() for o in compiled.plan.outputs()])
+        assert all(a.tobytes() == b.tobytes() for later in runs[1:] for a, b in zip(runs[0], later))
+        results[lanes] = runs[0]
+    wide = ({k: v.astype(np.float64) for k, v in args[0].items()}, *(a.astype(np.float64) for a in args[1:]))
+    exact = CompiledLoss(loss, wide, (0,), 0)
+    exact.bind(wide)
+    exact.plan.execute()
+    for two, one, e in zip(results[None], results["1"], exact.plan.outputs()):
+        assert relative_error(two, one) <= 2.0 ** -23
+        assert relative_error(two, e) <= 1e-5
