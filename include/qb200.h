@@ -258,8 +258,8 @@ qb200_status qb200_plan_optimizer_step(qb200_plan* plan, const qb200_opt_config*
 /* qb200_plan_execute and qb200_plan_optimizer_step in one call: a training step. */
 qb200_status qb200_plan_train_step(qb200_plan* plan, const qb200_opt_config* config);
 
-/* Page-locked host memory for read-back buffers: private pages, of which a forked child has its own copy.  To be freed by
- * the process that allocated it. */
+/* Page-locked host memory for read-back buffers; shared with forked children.  To be freed by the process that allocated
+ * it. */
 qb200_status qb200_host_alloc(size_t nbytes, void** out);
 void qb200_host_free(void* host);
 

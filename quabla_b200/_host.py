@@ -1,10 +1,11 @@
-"""Page-locked read-back buffers for the arrays a plan returns.
+"""Page-locked landing buffers for what a plan reads back.
 
-A device-to-host copy into fresh pageable memory pays for the driver's bounce buffer and for a page fault per 4 KiB
-(1.3 MB of gradients: 0.57 ms); into a page-locked block it runs at link speed (0.03 ms).  Arrays handed out here are views of such
-a block; when the last one is gone the block goes back to the pool.  The pool is shared by all plans and threads and
-bounded: beyond `LIMIT` bytes in use the caller gets ordinary memory, and at most `IDLE_LIMIT` bytes stay page-locked
-without an owner.  A forked child has copies of the arrays, as of any other memory; its own arrays are ordinary ones.
+A device-to-host copy into fresh pageable memory pays for the driver's bounce buffer (1.3 MB of gradients: 0.57 ms); into
+a page-locked block it runs at link speed (0.03 ms).  A reader copies what it hands out from such an array into ordinary
+memory and drops it: page-locked memory is shared with forked children, and one array kept by a caller would keep the block.
+When the last array made from a block is gone the block goes back to the pool.  The pool is shared by all plans and
+threads and bounded: beyond `LIMIT` bytes in use the caller gets ordinary memory, and at most `IDLE_LIMIT` bytes stay
+page-locked without an owner.
 """
 
 from __future__ import annotations
@@ -49,13 +50,12 @@ class _Block:
         self.__array_interface__ = {"data": (address, False), "shape": (count,), "typestr": dtype.str, "version": 3}
 
     def __del__(self) -> None:
-        _give_back(self.address, self.size)
+        if _lock is not None and not _forked:  # else: the interpreter is going down, or the block is the parent's
+            _give_back(self.address, self.size)
 
 
 def _give_back(address: int, size: int) -> None:
     global _total, _idle_bytes
-    if _forked:
-        return
     with _lock:
         if _idle_bytes + size <= IDLE_LIMIT:
             _idle.setdefault(size, []).append(address)

@@ -18,7 +18,6 @@ from . import _host, _lib
 from ._symbolic import Program
 
 COTANGENT_NAME = "__quabla_loss_cotangent"
-SMALL_LEAF_BYTES = 16384  # copied out of a read-back buffer: about a microsecond
 
 
 @dataclass
@@ -156,11 +155,9 @@ class Plan:
         return found
 
     def _leaves(self, flat: np.ndarray, base: int = 0) -> list[np.ndarray]:
-        """One array per parameter from a flat buffer: views of it, small leaves copies (one bias kept for long does not
-        keep the whole buffer, which may be page-locked)."""
+        """One array per parameter, copied from a flat buffer into memory of its own."""
         item = self.dtype.itemsize
-        views = [np.ndarray(shape, self.dtype, flat, (base + first) * item) for shape, first in self._layout()]
-        return [v.copy() if v.nbytes <= SMALL_LEAF_BYTES else v for v in views]
+        return [np.ndarray(shape, self.dtype, flat, (base + first) * item).copy() for shape, first in self._layout()]
 
     def close(self) -> None:
         if getattr(self, "_handle", None) and self._owned:
@@ -221,12 +218,11 @@ class Plan:
         return out
 
     def outputs(self) -> list[np.ndarray]:
-        """The loss and every gradient, read in one transfer.  Large gradients are views of one buffer: keeping one keeps
-        the buffer (`.copy()` what is kept for long); the arrays share no elements."""
+        """The loss and every gradient, read in one transfer."""
         self._layout()
         flat = _host.empty(1 + self._flat_size, self.dtype)
         _lib.check(self._lib.qb200_plan_read_outputs(self._handle, flat.__array_interface__["data"][0], flat.nbytes))
-        return [np.array(flat[0])] + self._leaves(flat, 1)  # the loss on its own: it is often kept for long
+        return [np.array(flat[0])] + self._leaves(flat, 1)
 
     def read_state(self, moments: bool) -> list[list[np.ndarray]]:
         """[parameters] or [parameters, first moments, second moments], each in parameter order; one wait."""

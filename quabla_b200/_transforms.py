@@ -379,8 +379,7 @@ def jit(fun: Callable, *, device: str | None = None, precision: str | None = Non
 
 
 def value_and_grad(fun: Callable, argnums=0) -> Callable:
-    """`fun`'s value and its gradients, in the containers of the arguments.  On concrete arrays the gradients of one call
-    are new arrays; large ones share a buffer that lives as long as any of them (`.copy()` what is kept for long)."""
+    """`fun`'s value and its gradients, in the containers of the arguments."""
     return _ValueAndGrad(fun, argnums, "value_and_grad")
 
 

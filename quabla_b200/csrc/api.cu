@@ -5,7 +5,6 @@
 
 #include <chrono>
 #include <cmath>
-#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <mutex>
@@ -417,26 +416,15 @@ qb200_status qb200_plan_train_step(qb200_plan* plan, const qb200_opt_config* con
 qb200_status qb200_host_alloc(size_t nbytes, void** out) {
     if (out == nullptr || nbytes == 0) return fail(QB200_INVALID, "host_alloc needs a size and an output");
     *out = nullptr;
-    // Private pages, registered: cudaHostAlloc maps shared ones, which a forked child would see change under it.
-    constexpr size_t PAGE = 4096;
-    void* pages = nbytes <= SIZE_MAX - PAGE ? aligned_alloc(PAGE, (nbytes + PAGE - 1) / PAGE * PAGE) : nullptr;
-    if (pages == nullptr) return fail(QB200_CUDA_ERROR, "%zu bytes of host memory are not to be had", nbytes);
-    const cudaError_t e = cudaHostRegister(pages, (nbytes + PAGE - 1) / PAGE * PAGE, cudaHostRegisterPortable);
-    if (e == cudaSuccess) {
-        *out = pages;
-        return QB200_OK;
-    }
+    const cudaError_t e = cudaHostAlloc(out, nbytes, cudaHostAllocPortable);
+    if (e == cudaSuccess) return QB200_OK;
     cudaGetLastError();  // the caller goes on with ordinary memory: the next launch must not find this error
-    free(pages);
+    *out = nullptr;
     return fail(QB200_CUDA_ERROR, "page-locking %zu bytes failed: %s", nbytes, cudaGetErrorString(e));
 }
 
 void qb200_host_free(void* host) {
-    if (host == nullptr) return;
-    if (cudaHostUnregister(host) != cudaSuccess) {
-        cudaGetLastError();  // the runtime is gone (exit), and the registration with it
-    }
-    free(host);
+    if (host != nullptr) cudaFreeHost(host);
 }
 
 qb200_status qb200_plan_loss(qb200_plan* plan, void* host_scalar) {

@@ -417,8 +417,7 @@ class Trainer:
 
     @property
     def params(self) -> Any:
-        """The parameters as host arrays, read from the device at every access.  Large ones share a buffer that lives as
-        long as any of them."""
+        """The parameters as host arrays, read from the device at every access."""
         return self._params_tree(self._executor.parameters())
 
     def _params_tree(self, values: dict) -> Any:

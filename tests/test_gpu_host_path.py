@@ -175,14 +175,13 @@ def test_a_forked_child_has_arrays_of_its_own(cuda_device):
     plan.execute()
     grads = plan.outputs()[1:]
     kept = [g.copy() for g in grads]
-    large = max(range(len(grads)), key=lambda i: grads[i].nbytes)  # a view of the block, not a copy
-    address = grads[large].__array_interface__["data"][0]
+    large = max(range(len(grads)), key=lambda i: grads[i].nbytes)
     (go, went), (answer, told) = os.pipe(), os.pipe()
     child = os.fork()
     if child == 0:
         try:
             signal.alarm(60)
-            os.read(go, 1)  # the parent has overwritten its block by now
+            os.read(go, 1)  # the parent has read the next gradients by now
             same = all(g.tobytes() == k.tobytes() for g, k in zip(grads, kept))
             for g in grads:
                 g.fill(7.0)
@@ -195,7 +194,6 @@ def test_a_forked_child_has_arrays_of_its_own(cuda_device):
     plan.bind(compiled.spec.parameters[1][0], 2.0 * np.asarray(inputs[compiled.spec.parameters[1][0]]))
     plan.execute()
     later = plan.outputs()[1:]
-    assert later[large].__array_interface__["data"][0] == address
     os.write(went, b"g")
     said = os.read(answer, 1)
     os.waitpid(child, 0)

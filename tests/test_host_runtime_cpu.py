@@ -2,6 +2,7 @@
 
 import os
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -116,3 +117,27 @@ def test_read_back_falls_back_to_ordinary_memory(monkeypatch):
         a = _host.empty(1000, np.dtype(np.float64))
         assert a.flags.owndata and a.shape == (1000,)
     assert _host._total == total
+
+
+def test_blocks_that_outlive_the_modules_end_quietly():
+    # On a stand-in for the library's two calls; builtins and os are cleared after the package.
+    program = """
+import builtins, ctypes, os
+import numpy as np
+from quabla_b200 import _host, _lib
+
+class Memory:
+    held = {}
+    def qb200_host_alloc(self, nbytes, out):
+        block = ctypes.create_string_buffer(nbytes)
+        out._obj.value = ctypes.addressof(block)
+        self.held[out._obj.value] = block
+        return _lib.OK
+
+memory = Memory()
+_lib.load = lambda: memory
+builtins.keep = os.keep = [_host.empty(n, np.dtype(np.float64)) for n in (100, 100, 300000)]
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", program], cwd=root, capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0 and done.stderr == "", done.stderr
