@@ -69,7 +69,8 @@ def test_weighted_laplacian_on_every_engine(cuda_device, dtype, width, engine):
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 def test_three_dimensional_laplacian_with_unequal_weights(cuda_device, dtype):
-    # Width 48 has no fused kernel; 1001 points x 48 units is odd for 16-byte vectors in float64 only.
+    # Below 1,024 points three layers of width 48 stay on the layer-wise engine; 1001 points x 48 units is odd for 16-byte
+    # vectors in float64 only.
     def residual(f, q):
         h = qb.hessian(f)(q)
         return h[0, 0] + 2.0 * h[1, 1] + 0.5 * h[2, 2] + q[2]
